@@ -21,6 +21,7 @@
 #include <cstring>
 #include <deque>
 #include <functional>
+#include <limits>
 #include <map>
 #include <memory>
 #include <new>
@@ -2118,6 +2119,9 @@ private:
         o.nc_threshold = R(s.node_contact.restitution_speed_threshold);
         o.nc_static = R(s.node_contact.static_friction); o.nc_dynamic = R(s.node_contact.dynamic_friction);
         o.plate_half_thickness = R(s.plate_half_thickness);
+        o.dt_sq = o.dt * o.dt;
+        o.dt_sq_recip = o.dt_sq >= R(0x1p-90) && o.dt_sq < R(0x1p30) ? R(1) / o.dt_sq
+                                                                      : std::numeric_limits<R>::quiet_NaN();
         o.audit = s.audit_energy ? 1U : 0U;
         o.plane_count = s.plane_count;
         for (unsigned p = 0; p < kPlanes; ++p) {

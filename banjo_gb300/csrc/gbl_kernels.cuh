@@ -1441,33 +1441,98 @@ constexpr int kSolvePer = GBL_SOLVE_PER;
 __device__ __forceinline__ void waitPreviousGrid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allowNextGrid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// The projection of one live bond (LatticePhysics.hpp:1132-1168) from its
-// record, geometry, multiplier and plastic extension and its gathered nodes;
-// the multiplier is stored unless this is the last iteration. Returns whether
-// the nodes moved (a degenerate bond leaves them).
+// The projection of one live bond (LatticePhysics.hpp:1132-1168): its unit
+// direction and the multiplier's change, with the reference's expressions.
+// Returns whether the nodes move (a degenerate bond leaves them).
 template <class R, bool Direct, bool Plastic>
-__device__ __forceinline__ bool projectBond(const Dev<R> &L, const Settings<R> &S, std::uint32_t d,
-                                            const BondRec<R> &rec, const Q4<R> &g, R lambda, R plastic, bool last,
-                                            Q4<R> &qa, Q4<R> &qb) {
-    const std::uint32_t a = endA(rec), b = endB(rec);
-    const V3<R> ua = xyz(qa), ub = xyz(qb), edge{g.x, g.y, g.z};
-    const V3<R> delta = Direct ? (xyz(L.x0[b]) + ub) - (xyz(L.x0[a]) + ua) : edge + (ub - ua);
+__device__ __forceinline__ bool bondStep(V3<R> x0a, V3<R> x0b, V3<R> ua, V3<R> ub, V3<R> edge, R rsm, R original,
+                                         R compliance, R wa, R wb, R lambda, R plastic, R dt, V3<R> &dir, R &dl) {
+    const V3<R> delta = Direct ? (x0b + ub) - (x0a + ua) : edge + (ub - ua);
     const R cl = length(delta);
     if (!(cl > R(1.0e-12))) return false;
-    const R original = rec.rest;
     const R rest = Plastic ? original + plastic : original;
     R constraint;
     if (Direct) {
         constraint = cl - rest;
     } else {
         const V3<R> du = ub - ua;
-        const R num = rec.rsm + R(2) * dot(edge, du) + dot(du, du);
+        const R num = rsm + R(2) * dot(edge, du) + dot(du, du);
         constraint = (Plastic ? num - plastic * (rest + original) : num) / (cl + rest);
     }
-    const V3<R> dir = delta / cl;
+    dir = delta / cl;
+    const R alpha = compliance / (dt * dt);
+    dl = (-constraint - alpha * lambda) / (wa + wb + alpha);
+    return true;
+}
+// The float lane's step where an operand is outside the branch-free range.
+struct FloatStep {
+    V3<float> dir;
+    float dl;
+    bool moves;
+};
+template <bool Plastic>
+__device__ __noinline__ FloatStep floatStepAnywhere(V3<float> ua, V3<float> ub, V3<float> edge, float rsm,
+                                                    float original, float compliance, float wa, float wb, float lambda,
+                                                    float plastic, float dt) {
+    FloatStep s{};
+    s.moves = bondStep<float, false, Plastic>(V3<float>{}, V3<float>{}, ua, ub, edge, rsm, original, compliance, wa, wb,
+                                              lambda, plastic, dt, s.dir, s.dl);
+    return s;
+}
+// The float lane's step. The same values from the branch-free quotients: the
+// six divisions and the root of a bond took most of a round (a beam of 135
+// nodes swept in one CTA: 0.78 us a level with them, 0.40 without).
+template <bool Plastic>
+__device__ __forceinline__ FloatStep floatStep(const Settings<float> &S, V3<float> ua, V3<float> ub, V3<float> edge,
+                                               float rsm, float original, float compliance, float wa, float wb,
+                                               float lambda, float plastic) {
+    const V3<float> du = ub - ua;
+    const V3<float> delta = edge + du;
+    const float sq = dot(delta, delta);
+    const float cl = rootNearest(sq);
+    const float ycl = recipNearest(cl);
+    const float rest = Plastic ? original + plastic : original;
+    const float raw = rsm + 2.0F * dot(edge, du) + dot(du, du);
+    const float num = Plastic ? raw - plastic * (rest + original) : raw;
+    const float den = cl + rest;
+    const float alpha = quotient(compliance, S.dt_sq, S.dt_sq_recip);
+    const float w = wa + wb + alpha;
+    const float pull = -quotient(num, den, recipNearest(den)) - alpha * lambda;
+    FloatStep s;
+    s.dl = quotient(pull, w, recipNearest(w));
+    s.dir = {quotient(delta.x, cl, ycl), quotient(delta.y, cl, ycl), quotient(delta.z, cl, ycl)};
+    s.moves = true; // rootOk: the length is above 1e-12
+    const std::uint32_t least = min(min(min(dividendKey(delta.x), dividendKey(delta.y)),
+                                        min(dividendKey(delta.z), dividendKey(num))),
+                                    min(dividendKey(pull), dividendKey(compliance)));
+    // An infinite or NaN operand leaves a NaN or an infinity in s.dl or w.
+    if (!(rootOk(sq) && divisorOk(den) && divisorOk(w) && least >= kDividendLeast && fabsf(s.dl) < 0x1p100F))
+        s = floatStepAnywhere<Plastic>(ua, ub, edge, rsm, original, compliance, wa, wb, lambda, plastic, S.dt);
+    return s;
+}
+
+// One live bond from its record, geometry, multiplier and plastic extension
+// and its gathered nodes; the multiplier is stored unless this is the last
+// iteration. Returns whether the nodes moved.
+template <class R, bool Direct, bool Plastic>
+__device__ __forceinline__ bool projectBond(const Dev<R> &L, const Settings<R> &S, std::uint32_t d,
+                                            const BondRec<R> &rec, const Q4<R> &g, R lambda, R plastic, bool last,
+                                            Q4<R> &qa, Q4<R> &qb) {
+    const V3<R> ua = xyz(qa), ub = xyz(qb), edge{g.x, g.y, g.z};
     const R wa = qa.w, wb = qb.w;
-    const R alpha = g.w / (S.dt * S.dt);
-    const R dl = (-constraint - alpha * lambda) / (wa + wb + alpha);
+    V3<R> dir;
+    R dl;
+    if constexpr (std::is_same<R, float>::value && !Direct) {
+        const FloatStep s = floatStep<Plastic>(S, ua, ub, edge, rec.rsm, rec.rest, g.w, wa, wb, lambda, plastic);
+        if (!s.moves) return false;
+        dir = s.dir;
+        dl = s.dl;
+    } else {
+        const V3<R> x0a = Direct ? xyz(L.x0[endA(rec)]) : V3<R>{}, x0b = Direct ? xyz(L.x0[endB(rec)]) : V3<R>{};
+        if (!bondStep<R, Direct, Plastic>(x0a, x0b, ua, ub, edge, rec.rsm, rec.rest, g.w, wa, wb, lambda, plastic, S.dt,
+                                          dir, dl))
+            return false;
+    }
     if (!last) __stcs(L.lambda + d, lambda + dl);
     const V3<R> na = ua - (wa * dl) * dir;
     const V3<R> nb = ub + (wb * dl) * dir;
