@@ -1802,7 +1802,7 @@ public:
         float ms = 0;
         cudaEventElapsedTime(&ms, ev0_, ev1_);
         pullControl();
-        bool overflowed = false, wrenched = false, stage_timeout = false;
+        bool overflowed = false, wrenched = false;
         for (auto k : active_) {
             Ctl &c = ctl_host_[k];
             Resident<R> &l = *slots_[k];
@@ -1814,10 +1814,6 @@ public:
             if (c.error & kErrWrench) {
                 c.error = 0;
                 wrenched = true;
-            }
-            if (c.error & kErrStageWait) {
-                c.error = 0;
-                stage_timeout = true;
             }
             l.ext_remaining = c.loads_remaining;
             l.fillStatus(c);
@@ -1840,11 +1836,6 @@ public:
             check(cudaStreamSynchronize(stream_), "status");
             invalid("external wrench cannot be spread over its nodes at the current geometry (torque, resultant "
                     "or node force not representable)");
-        }
-        if (stage_timeout) {
-            pushControl();
-            check(cudaStreamSynchronize(stream_), "status");
-            runtime("the staged sweep's bulk copy into shared memory did not complete within its bounded wait");
         }
         const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count();
         for (auto k : active_) slots_[k]->status.wall_seconds += wall;
@@ -2001,36 +1992,31 @@ public:
         out.default_ms = best_ms;
         out.candidates = 1;
         if (many_) {
-            // The one-CTA sweep's CTA size and reach together, then the group size.
+            auto attempt = [&](const Shape &sh) {
+                const double ms = timeShape(sh);
+                ++out.candidates;
+                if (ms < best_ms) { best_ms = ms; best = sh; }
+            };
+            // Without the staged sweep: level launches for all, and the
+            // one-CTA sweep's CTA size and reach together; then the group size.
+            {
+                Shape sh = fallback;
+                sh.staged_max_nodes = 0;
+                attempt(sh);
+            }
             for (unsigned threads : {256U, 512U, 1024U})
                 for (std::uint32_t reach : {1U << 16, 1U << 17, 1U << 18, 1U << 19}) {
-                    Shape sh = best;
+                    Shape sh = fallback;
                     sh.sweep_threads = threads;
                     sh.whole_max_bonds = reach;
-                    if (sh.sweep_threads == fallback.sweep_threads && sh.whole_max_bonds == fallback.whole_max_bonds)
-                        continue;
-                    const double ms = timeShape(sh);
-                    ++out.candidates;
-                    if (ms < best_ms) { best_ms = ms; best = sh; }
+                    sh.staged_max_nodes = 0;
+                    attempt(sh);
                 }
             const Shape base = best;
             for (std::size_t mb : {16U, 32U, 96U, 192U}) {
                 Shape sh = base;
                 sh.group_bytes = mb << 20;
-                const double ms = timeShape(sh);
-                ++out.candidates;
-                if (ms < best_ms) { best_ms = ms; best = sh; }
-            }
-            // The shared-memory staged sweep for the small whole lattices.
-            if (!kDirect) {
-                const Shape kept = best;
-                for (std::uint32_t nodes : {kStagedMaxNodes / 2, kStagedMaxNodes}) {
-                    Shape sh = kept;
-                    sh.staged_max_nodes = nodes;
-                    const double ms = timeShape(sh);
-                    ++out.candidates;
-                    if (ms < best_ms) { best_ms = ms; best = sh; }
-                }
+                attempt(sh);
             }
         }
         positions(false);
@@ -2246,11 +2232,37 @@ private:
     // A launch's items: [first, first + count) of the work array; for a
     // single lattice, the same items as (base, end, per).
     struct Span { std::uint32_t first, count, base, end, per; };
-
     // A lattice of a batch swept by one CTA (kSweepLattice): small enough to
     // keep its nodes in L2 across its levels, with levels that fit the table.
     bool sweptWhole(const Resident<R> &l) const {
         return l.B > 0 && l.B <= shape_.whole_max_bonds && l.dev.level_count == l.levels.size();
+    }
+
+    // Whether the lattices sweep staged, one CTA each (kSweepStaged): when
+    // every one's widest level has a thread for each bond and its positions
+    // fit, and every CTA is resident at once. A level then costs 0.4 us (135
+    // nodes) to 1.0 us (1,024 bonds), where its launch costs 1.4 us or
+    // more. A batch with one larger lattice is level-launched whole: a
+    // launch covers every lattice of the batch, so the small ones ride along
+    // (sweep per substep, 128 lattices of 8 to 12 a side: 134 us staged,
+    // 228 level-launched; of 8 to 48: 1,459 us level-launched, 1,466 with the
+    // small ones staged beside them, 4,012 with those of up to 2^18 bonds in
+    // one CTA each; 1,000 of 8 to 12: 635 us level-launched, 870 staged).
+    bool stagedSweep() const {
+        if (kDirect || S_.iterations == 0 || active_.empty() || active_.size() > sms_) return false;
+        const std::uint32_t cap = std::min(shape_.staged_max_nodes, kStagedNodes);
+        for (auto k : active_) {
+            const Resident<R> &l = *slots_[k];
+            if (widestLevel(l) > kStagedThreads || l.N > cap || l.B == 0 || l.dev.level_count != l.levels.size() ||
+                l.levels.size() > kStagedLevels)
+                return false;
+        }
+        return true;
+    }
+    static std::uint32_t widestLevel(const Resident<R> &l) {
+        std::uint32_t widest = 0;
+        for (const auto &lv : l.levels) widest = std::max(widest, lv.end - lv.begin);
+        return widest;
     }
 
     // Work lists of every phase, one item per CTA, lattices in slot order.
@@ -2282,34 +2294,29 @@ private:
         each_ = span([](const Res &, U &b, U &e) { b = 0; e = 1; }, 1);
         slabs_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.sched.block_count; }, 1);
         buckets_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.nc_mem ? l.dev.nc_mask + 1U : 0U; }, kThreads);
-        // With many lattices, the small ones sweep in one CTA each (largest first);
-        // the level launches and the isolated-node launch cover the others.
-        auto leveled = [this](const Res &l) { return !many_ || !sweptWhole(l); };
+        // The lattices swept staged, or whole in one CTA each where the shape
+        // says so, largest first; the level launches and the isolated-node
+        // launch cover the rest.
+        const bool staged = stagedSweep();
+        auto leveled = [&](std::uint32_t k) { return !staged && !(many_ && sweptWhole(*slots_[k])); };
         {
-            // Those whose positions fit the staged sweep's shared memory take
-            // it when the shape asks for it.
-            std::vector<std::uint32_t> whole, staged;
-            staged_nodes_ = 0;
-            if (many_)
-                for (auto k : active_) {
+            std::vector<std::uint32_t> order;
+            for (auto k : active_)
+                if (!leveled(k)) order.push_back(k);
+            std::stable_sort(order.begin(), order.end(), [this](std::uint32_t x, std::uint32_t y) {
+                return slots_[x]->B > slots_[y]->B;
+            });
+            const U first = static_cast<U>(all.size());
+            for (auto k : order) all.push_back({k, 0, 1});
+            whole_ = Span{first, static_cast<U>(order.size()), 0, 1, 1};
+            staged_threads_ = 0;
+            staged_smem_ = 0;
+            if (staged)
+                for (auto k : order) {
                     const Res &l = *slots_[k];
-                    if (!sweptWhole(l)) continue;
-                    if (!kDirect && l.N <= shape_.staged_max_nodes) {
-                        staged.push_back(k);
-                        staged_nodes_ = std::max(staged_nodes_, l.N);
-                    } else {
-                        whole.push_back(k);
-                    }
+                    staged_threads_ = std::max(staged_threads_, std::max(64U, (widestLevel(l) + 31) / 32 * 32));
+                    staged_smem_ = std::max(staged_smem_, sizeof(Q4<float>) * l.N + 4 * (l.levels.size() + 1));
                 }
-            const auto larger = [this](std::uint32_t x, std::uint32_t y) { return slots_[x]->B > slots_[y]->B; };
-            std::stable_sort(whole.begin(), whole.end(), larger);
-            std::stable_sort(staged.begin(), staged.end(), larger);
-            U first = static_cast<U>(all.size());
-            for (auto k : whole) all.push_back({k, 0, 1});
-            whole_ = Span{first, static_cast<U>(whole.size()), 0, 1, 1};
-            first = static_cast<U>(all.size());
-            for (auto k : staged) all.push_back({k, 0, 1});
-            staged_ = Span{first, static_cast<U>(staged.size()), 0, 1, 1};
         }
         {
             const U first = static_cast<U>(all.size());
@@ -2336,7 +2343,7 @@ private:
             std::size_t bytes = 0;
             for (auto k : active_) {
                 const Res &l = *slots_[k];
-                if (!leveled(l)) continue;
+                if (!leveled(k)) continue;
                 const std::size_t need = static_cast<std::size_t>(l.N) * sizeof(Q4<R>);
                 if (!members.back().empty() && bytes + need > shape_.group_bytes) {
                     members.emplace_back();
@@ -2530,12 +2537,19 @@ private:
     template <bool M, class Mark> void enqueueSweep(Mark &&mark) {
         const Settings<R> &S = S_;
         cudaStream_t st = stream_;
-        const bool whole = M && (whole_.count || staged_.count);
+        // Whole sweeps: staged ones are the whole phase; others run beside the
+        // level launches.
+        if (staged_threads_) {
+            launchSweepStaged(whole_, st);
+            mark(5);
+            mark(7);
+            return;
+        }
+        const bool whole = M && whole_.count;
         if (whole) {
             check(cudaEventRecord(fork_, st), "event");
             check(cudaStreamWaitEvent(side_, fork_, 0), "stream wait");
-            if (whole_.count) launchSweepWhole(whole_, side_);
-            if (staged_.count) launchSweepStaged(staged_, side_);
+            launchSweepWhole(whole_, side_);
             check(cudaEventRecord(join_, side_), "event");
         }
         const unsigned I = S.iterations;
@@ -2598,49 +2612,35 @@ private:
         }
     }
 
-    // The whole sweeps of the lattices whose positions fit in shared memory
-    // (float lane): staged in by one bulk copy, swept in the SM, written back.
+    // One CTA per lattice (float lane).
     void launchSweepStaged(const Span &span, cudaStream_t st) {
         if constexpr (!kDirect) {
-            switch (shape_.sweep_threads) {
-            case 256: launchSweepStagedAs<256>(span, st); break;
-            case 1024: launchSweepStagedAs<1024>(span, st); break;
-            default: launchSweepStagedAs<512>(span, st); break;
+            const int key = (plastic_ ? 2 : 0) | (S_.plane_count ? 1 : 0);
+            const Grid<R> g = grid(span);
+            switch (key) {
+            case 0: kSweepStaged<false, false><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
+            case 1: kSweepStaged<false, true><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
+            case 2: kSweepStaged<true, false><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
+            default: kSweepStaged<true, true><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
             }
-        }
-    }
-    template <unsigned T> void launchSweepStagedAs(const Span &span, cudaStream_t st) {
-        const bool support = S_.plane_count != 0;
-        const int key = (plastic_ ? 2 : 0) | (support ? 1 : 0);
-        const Grid<R> g = grid(span);
-        const std::size_t smem = static_cast<std::size_t>(staged_nodes_) * sizeof(Q4<R>);
-        switch (key) {
-        case 0: kSweepLattice<R, kDirect, false, false, T, true><<<span.count, T, smem, st>>>(g, S_); break;
-        case 1: kSweepLattice<R, kDirect, false, true, T, true><<<span.count, T, smem, st>>>(g, S_); break;
-        case 2: kSweepLattice<R, kDirect, true, false, T, true><<<span.count, T, smem, st>>>(g, S_); break;
-        default: kSweepLattice<R, kDirect, true, true, T, true><<<span.count, T, smem, st>>>(g, S_); break;
         }
     }
     // The shared memory every staged instance may take: set once.
     void allowStagedSharedMemory() {
+        int device = 0, sms = 0;
+        check(cudaGetDevice(&device), "device");
+        check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device attribute");
+        sms_ = static_cast<unsigned>(sms);
         if constexpr (!kDirect) {
-            const int bytes = static_cast<int>(kStagedMaxNodes * sizeof(Q4<R>));
+            const int bytes = static_cast<int>(kStagedNodes * sizeof(Q4<float>) + 4 * (kStagedLevels + 1));
             auto allow = [&](auto kernel) {
                 check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
                       "staged sweep shared memory");
             };
-            allow(kSweepLattice<R, kDirect, false, false, 256, true>);
-            allow(kSweepLattice<R, kDirect, false, true, 256, true>);
-            allow(kSweepLattice<R, kDirect, true, false, 256, true>);
-            allow(kSweepLattice<R, kDirect, true, true, 256, true>);
-            allow(kSweepLattice<R, kDirect, false, false, 512, true>);
-            allow(kSweepLattice<R, kDirect, false, true, 512, true>);
-            allow(kSweepLattice<R, kDirect, true, false, 512, true>);
-            allow(kSweepLattice<R, kDirect, true, true, 512, true>);
-            allow(kSweepLattice<R, kDirect, false, false, 1024, true>);
-            allow(kSweepLattice<R, kDirect, false, true, 1024, true>);
-            allow(kSweepLattice<R, kDirect, true, false, 1024, true>);
-            allow(kSweepLattice<R, kDirect, true, true, 1024, true>);
+            allow(kSweepStaged<false, false>);
+            allow(kSweepStaged<false, true>);
+            allow(kSweepStaged<true, false>);
+            allow(kSweepStaged<true, true>);
         }
     }
 
@@ -2732,9 +2732,11 @@ private:
     unsigned *running_{}, *running_host_{};
     Dev<R> *table_{};
     Work *work_{};
-    Span nodes_{}, bonds_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, broken_{}, whole_{}, staged_{}, buckets_{},
+    Span nodes_{}, bonds_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, broken_{}, whole_{}, buckets_{},
         wrench_{};
-    std::uint32_t staged_nodes_{0}; // the staged sweep's shared memory, in nodes
+    unsigned staged_threads_{0}; // the staged sweep's CTA size (0: the lattices do not sweep staged)
+    std::size_t staged_smem_{0};
+    unsigned sms_{1};
     // Level-launched lattices, in groups swept one after another.
     struct Group {
         std::vector<Span> levels;
@@ -2750,9 +2752,9 @@ private:
     // workload; tune() times candidates on the lattices present.
     struct Shape {
         unsigned sweep_threads = kSweepThreads;
-        std::uint32_t whole_max_bonds = kMaxFusedBonds;
+        std::uint32_t whole_max_bonds = 0; // none: every shape that used it was slower than level launches
         std::size_t group_bytes = std::size_t(48) << 20;
-        std::uint32_t staged_max_nodes = 0; // whole sweeps staged in shared memory up to this many nodes
+        std::uint32_t staged_max_nodes = kStagedMaxNodes; // nodes of a lattice swept staged, at most (0: none)
     };
     Shape shape_;
     cudaStream_t own_stream_{}, stream_{}, side_{}, loads_{};
@@ -2923,19 +2925,11 @@ public:
 template <class R> class Server final : public ServerBase {
 public:
     static constexpr std::uint32_t kLargeBonds = 1U << 22;
-    static constexpr std::uint32_t kServedWholeBonds = 1U << 14;
     static constexpr unsigned kSmall = 0, kLarge = 1;
 
     Server(const gbl_step_settings &settings, std::uint64_t budget)
         : budget_(budget), contact_(settings.node_contact.mode != 0), t0_(clock()) {
         for (auto &lane : lanes_) lane.configure(settings);
-        // A server holds few lattices at a time: a lattice swept whole by one
-        // CTA takes that CTA's serial time per substep (about 3.5 ms for
-        // 2^18 bonds), where level launches spread it over the GPU. Only
-        // tiny lattices sweep whole here.
-        gbl_tuning shape{};
-        shape.whole_max_bonds = kServedWholeBonds;
-        for (auto &lane : lanes_) lane.setShape(shape);
     }
     ~Server() override {
         for (auto &kv : requests_)

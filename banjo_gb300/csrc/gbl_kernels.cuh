@@ -170,7 +170,6 @@ struct SourceSlot {
 
 constexpr unsigned kErrExternalOverflow = 1;
 constexpr unsigned kErrWrench = 2;
-constexpr unsigned kErrStageWait = 4; // a bounded wait for a bulk copy into shared memory ran out
 
 template <class R> struct Dev {
     std::uint32_t N, B, D, blocks, words_b, tiles_b;
@@ -1502,71 +1501,82 @@ __device__ __forceinline__ FloatStep floatStep(const Settings<float> &S, V3<floa
     s.dl = quotient(pull, w, recipNearest(w));
     s.dir = {quotient(delta.x, cl, ycl), quotient(delta.y, cl, ycl), quotient(delta.z, cl, ycl)};
     s.moves = true; // rootOk: the length is above 1e-12
-    const std::uint32_t least = min(min(min(dividendKey(delta.x), dividendKey(delta.y)),
-                                        min(dividendKey(delta.z), dividendKey(num))),
-                                    min(dividendKey(pull), dividendKey(compliance)));
+    const std::uint32_t least =
+        __vimin3_u32(__vimin3_u32(dividendKey(delta.x), dividendKey(delta.y), dividendKey(delta.z)), dividendKey(num),
+                     min(dividendKey(pull), dividendKey(compliance)));
     // An infinite or NaN operand leaves a NaN or an infinity in s.dl or w.
     if (!(rootOk(sq) && divisorOk(den) && divisorOk(w) && least >= kDividendLeast && fabsf(s.dl) < 0x1p100F))
         s = floatStepAnywhere<Plastic>(ua, ub, edge, rsm, original, compliance, wa, wb, lambda, plastic, S.dt);
     return s;
 }
 
-// One live bond from its record, geometry, multiplier and plastic extension
-// and its gathered nodes; the multiplier is stored unless this is the last
-// iteration. Returns whether the nodes moved.
-template <class R, bool Direct, bool Plastic>
-__device__ __forceinline__ bool projectBond(const Dev<R> &L, const Settings<R> &S, std::uint32_t d,
-                                            const BondRec<R> &rec, const Q4<R> &g, R lambda, R plastic, bool last,
-                                            Q4<R> &qa, Q4<R> &qb) {
-    const V3<R> ua = xyz(qa), ub = xyz(qb), edge{g.x, g.y, g.z};
-    const R wa = qa.w, wb = qb.w;
-    V3<R> dir;
-    R dl;
-    if constexpr (std::is_same<R, float>::value && !Direct) {
-        const FloatStep s = floatStep<Plastic>(S, ua, ub, edge, rec.rsm, rec.rest, g.w, wa, wb, lambda, plastic);
-        if (!s.moves) return false;
-        dir = s.dir;
-        dl = s.dl;
-    } else {
-        const V3<R> x0a = Direct ? xyz(L.x0[endA(rec)]) : V3<R>{}, x0b = Direct ? xyz(L.x0[endB(rec)]) : V3<R>{};
-        if (!bondStep<R, Direct, Plastic>(x0a, x0b, ua, ub, edge, rec.rsm, rec.rest, g.w, wa, wb, lambda, plastic, S.dt,
-                                          dir, dl))
-            return false;
-    }
-    if (!last) __stcs(L.lambda + d, lambda + dl);
-    const V3<R> na = ua - (wa * dl) * dir;
-    const V3<R> nb = ub + (wb * dl) * dir;
-    qa = Q4<R>{na.x, na.y, na.z, wa};
-    qb = Q4<R>{nb.x, nb.y, nb.z, wb};
-    return true;
-}
+// Where a sweep keeps its nodes' positions: the lattice's array in global
+// memory (through L2, which every SM shares), or a CTA's shared memory
+// (StagedNodes, below).
+template <class R> struct GlobalNodes {
+    Q4<R> *u;
+    __device__ __forceinline__ Q4<R> load(std::uint32_t i) const { return ldShared(u + i); }
+    __device__ __forceinline__ void store(std::uint32_t i, const Q4<R> &q) const { u[i] = q; }
+};
 
 // The support projection of a node after its last bond of the sweep.
-template <class R>
-__device__ __forceinline__ void supportLast(const Dev<R> &L, const Settings<R> &S, std::uint32_t i, bool have,
-                                            Q4<R> &q, bool &write) {
-    if (!have) q = L.u[i];
+template <class R, class Nodes>
+__device__ __forceinline__ void supportLast(const Dev<R> &L, const Settings<R> &S, const Nodes &nodes, std::uint32_t i,
+                                            bool have, Q4<R> &q, bool &write) {
+    if (!have) q = nodes.load(i);
     V3<R> u = xyz(q);
     if (supportProject(L, S, i, u)) {
         q = Q4<R>{u.x, u.y, u.z, q.w};
         write = true;
     }
 }
-// A bond's projection, then the support projection of the nodes whose last
-// bond of the sweep it is, then the write-back of what moved.
-template <class R, bool Direct, bool Plastic, bool Support>
-__device__ __forceinline__ void finishBond(const Dev<R> &L, const Settings<R> &S, std::uint32_t d,
-                                           const BondRec<R> &rec, bool live, const Q4<R> &g, R lambda, R plastic,
-                                           bool last, Q4<R> qa, Q4<R> qb) {
+// A bond from its record, geometry, multiplier and plastic extension: its nodes
+// gathered, the projection, then the support projection of the nodes whose
+// last bond of the sweep it is, then the write-back of what moved. The
+// multiplier is stored unless this is the last iteration. A degenerate bond
+// leaves its nodes; a broken or degenerate last bond still carries their
+// support projection.
+template <class R, bool Direct, bool Plastic, bool Support, class Nodes>
+__device__ __forceinline__ void solveBond(const Dev<R> &L, const Settings<R> &S, const Nodes &nodes, R *lambdas,
+                                          std::uint32_t d, const BondRec<R> &rec, const Q4<R> &g, R lambda, R plastic,
+                                          bool last) {
     const std::uint32_t a = endA(rec), b = endB(rec);
+    const bool live = !(rec.a & kDeadBit);
     bool write_a = false, write_b = false;
-    if (live) write_a = write_b = projectBond<R, Direct, Plastic>(L, S, d, rec, g, lambda, plastic, last, qa, qb);
-    if (Support) {
-        if (rec.a & kLastABit) supportLast(L, S, a, live, qa, write_a);
-        if (rec.b & kLastBBit) supportLast(L, S, b, live, qb, write_b);
+    Q4<R> qa{}, qb{};
+    if (live) {
+        qa = nodes.load(a);
+        qb = nodes.load(b);
+        const V3<R> ua = xyz(qa), ub = xyz(qb), edge{g.x, g.y, g.z};
+        const R wa = qa.w, wb = qb.w;
+        V3<R> dir;
+        R dl;
+        bool moves;
+        if constexpr (std::is_same<R, float>::value && !Direct) {
+            const FloatStep s = floatStep<Plastic>(S, ua, ub, edge, rec.rsm, rec.rest, g.w, wa, wb, lambda, plastic);
+            dir = s.dir;
+            dl = s.dl;
+            moves = s.moves;
+        } else {
+            const V3<R> x0a = Direct ? xyz(L.x0[a]) : V3<R>{}, x0b = Direct ? xyz(L.x0[b]) : V3<R>{};
+            moves = bondStep<R, Direct, Plastic>(x0a, x0b, ua, ub, edge, rec.rsm, rec.rest, g.w, wa, wb, lambda, plastic,
+                                                 S.dt, dir, dl);
+        }
+        if (moves) {
+            if (!last) __stcs(lambdas + d, lambda + dl);
+            const V3<R> na = ua - (wa * dl) * dir;
+            const V3<R> nb = ub + (wb * dl) * dir;
+            qa = Q4<R>{na.x, na.y, na.z, wa};
+            qb = Q4<R>{nb.x, nb.y, nb.z, wb};
+            write_a = write_b = true;
+        }
     }
-    if (write_a) L.u[a] = qa;
-    if (write_b) L.u[b] = qb;
+    if (Support && ((rec.a & kLastABit) || (rec.b & kLastBBit))) {
+        if (rec.a & kLastABit) supportLast(L, S, nodes, a, live, qa, write_a);
+        if (rec.b & kLastBBit) supportLast(L, S, nodes, b, live, qb, write_b);
+    }
+    if (write_a) nodes.store(a, qa);
+    if (write_b) nodes.store(b, qb);
 }
 
 template <class R, bool Many, bool Direct, bool First, bool Last, bool Plastic, bool Support>
@@ -1574,7 +1584,7 @@ __global__ void __launch_bounds__(kThreads, GBL_SOLVE_MIN_BLOCKS) kSolve(const G
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     BondRec<R> rec[kSolvePer];
-    Q4<R> geo[kSolvePer], qa[kSolvePer], qb[kSolvePer];
+    Q4<R> geo[kSolvePer];
     R lam[kSolvePer], pl[kSolvePer];
     std::uint32_t at[kSolvePer];
     // Everything that no kernel since the last end sample has written.
@@ -1592,21 +1602,11 @@ __global__ void __launch_bounds__(kThreads, GBL_SOLVE_MIN_BLOCKS) kSolve(const G
     waitPreviousGrid();
     allowNextGrid();
     if (stop) return;
-    bool live[kSolvePer], ok[kSolvePer];
-#pragma unroll
-    for (int k = 0; k < kSolvePer; ++k) {
-        ok[k] = at[k] < w.end && endsInBounds(rec[k], L.N, kSiteSolve);
-        live[k] = ok[k] && !(rec[k].a & kDeadBit);
-        if (live[k]) {
-            qa[k] = ldShared(L.u + endA(rec[k]));
-            qb[k] = ldShared(L.u + endB(rec[k]));
-        }
-    }
+    const GlobalNodes<R> nodes{L.u};
 #pragma unroll
     for (int k = 0; k < kSolvePer; ++k)
-        if (ok[k])
-            finishBond<R, Direct, Plastic, Support>(L, S, at[k], rec[k], live[k], geo[k], lam[k], pl[k], Last, qa[k],
-                                                    qb[k]);
+        if (at[k] < w.end && endsInBounds(rec[k], L.N, kSiteSolve))
+            solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, at[k], rec[k], geo[k], lam[k], pl[k], Last);
 }
 
 // The whole sweep of one lattice in one CTA: every iteration, every level in
@@ -1619,11 +1619,6 @@ __global__ void __launch_bounds__(kThreads, GBL_SOLVE_MIN_BLOCKS) kSolve(const G
 // autotuner picks; two CTAs per SM below 1024 threads.
 constexpr unsigned kSweepThreads = 512; // the default shape
 constexpr std::uint32_t kMaxFusedLevels = 1024;
-// A lattice's one-CTA sweep takes as long as its bonds over one CTA's rate, so
-// only lattices small enough to finish well within the batch's level launches
-// are swept whole (measured: a 48^3 trial alone in one CTA bounded the whole
-// batch's sweep). The default bound; the autotuner picks its own.
-constexpr std::uint32_t kMaxFusedBonds = 1U << 18;
 
 template <class R, bool Support>
 __device__ __forceinline__ void supportIsolatedInCta(const Dev<R> &L, const Settings<R> &S) {
@@ -1638,75 +1633,12 @@ __device__ __forceinline__ void supportIsolatedInCta(const Dev<R> &L, const Sett
     }
 }
 
-// Shared-memory staging of a small lattice's nodes for its one-CTA sweep: the
-// whole position array (one 16-byte record per node) comes in by one bulk
-// copy (the copy engine, cp.async.bulk, completing on an mbarrier), every
-// gather and write of the sweep then stays in the SM, and the array goes back
-// to global memory once at the end. The waits are bounded: a copy that has
-// not landed after kStageSpins polls marks the lattice's control block with
-// kErrStageWait (the host reports it), waits as long again for the copy to
-// drain, and the CTA leaves.
-constexpr std::uint32_t kStageSpins = 1U << 26;
-// Positions the staged sweep holds: 14,336 x 16 B = 224 KiB of dynamic shared
-// memory, with the descriptor and the barrier inside the 227 KiB a CTA may take.
-constexpr std::uint32_t kStagedMaxNodes = 14336;
-constexpr std::uint32_t kStageChunk = 32768; // bytes per bulk copy
-
-__device__ __forceinline__ std::uint32_t smemAddress(const void *p) {
-    return static_cast<std::uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ bool barrierDone(std::uint64_t *bar, std::uint32_t parity) {
-    std::uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done)
-                 : "r"(smemAddress(bar)), "r"(parity)
-                 : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ bool waitBarrier(std::uint64_t *bar, std::uint32_t parity) {
-    for (std::uint32_t spin = 0; spin < kStageSpins; ++spin)
-        if (barrierDone(bar, parity)) return true;
-    return false;
-}
-
-// The CTA's nodes [0, n) from global `src` into shared `dst` (n x 16 bytes,
-// both 16-byte aligned). Returns false, after the bounded drain, when the
-// copy did not land in time (every thread returns the same).
-template <class R>
-__device__ bool stageNodesIn(Q4<R> *dst, const Q4<R> *src, std::uint32_t n, std::uint64_t *bar, Ctl *ctl) {
-    const std::uint32_t bytes = n * static_cast<std::uint32_t>(sizeof(Q4<R>));
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smemAddress(bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smemAddress(bar)), "r"(bytes)
-                     : "memory");
-        for (std::uint32_t off = 0; off < bytes; off += kStageChunk) {
-            const std::uint32_t len = bytes - off < kStageChunk ? bytes - off : kStageChunk;
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-                             "r"(smemAddress(reinterpret_cast<unsigned char *>(dst) + off)),
-                         "l"(__cvta_generic_to_global(reinterpret_cast<const unsigned char *>(src) + off)), "r"(len),
-                         "r"(smemAddress(bar))
-                         : "memory");
-        }
-    }
-    __syncthreads(); // the barrier is initialised before anyone waits on it
-    const bool landed = waitBarrier(bar, 0);
-    if (__syncthreads_and(landed ? 1 : 0)) return true;
-    if (threadIdx.x == 0) atomicOr(&ctl->error, kErrStageWait);
-    (void)waitBarrier(bar, 0); // the copy still writes this CTA's shared memory: let it drain
-    __syncthreads();
-    return false;
-}
-
-template <class R, bool Direct, bool Plastic, bool Support, unsigned T, bool Staged = false>
+template <class R, bool Direct, bool Plastic, bool Support, unsigned T>
 __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 2) kSweepLattice(const Grid<R> launch, Settings<R> S) {
     // The lattice's descriptor, copied once into shared memory: its fields
     // are read throughout the sweep, and shared memory is never written by
     // the sweep's global stores, so the compiler may keep them as it likes.
     __shared__ __align__(16) unsigned char desc[sizeof(Dev<R>)];
-    __shared__ std::uint64_t stage_bar;
-    extern __shared__ __align__(128) unsigned char sweep_nodes[];
     {
         const Work w = item<true>(launch);
         const unsigned *src = reinterpret_cast<const unsigned *>(launch.table + w.lattice);
@@ -1714,20 +1646,9 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 2) kSweepLattice(const Grid
         for (unsigned k = threadIdx.x; k < sizeof(Dev<R>) / sizeof(unsigned); k += blockDim.x) dst[k] = src[k];
     }
     __syncthreads();
-    Q4<R> *const global_u = reinterpret_cast<const Dev<R> *>(desc)->u;
-    const std::uint32_t node_count = reinterpret_cast<const Dev<R> *>(desc)->N;
-    if (reinterpret_cast<const Dev<R> *>(desc)->ctl->stop) return;
-    if constexpr (Staged) {
-        // The sweep's node reads and writes go to the staged copy: the
-        // shared-memory descriptor's position pointer is swapped for it
-        // (generic loads and stores reach shared memory through it).
-        Q4<R> *nodes = reinterpret_cast<Q4<R> *>(sweep_nodes);
-        if (!stageNodesIn(nodes, global_u, node_count, &stage_bar, reinterpret_cast<const Dev<R> *>(desc)->ctl))
-            return;
-        if (threadIdx.x == 0) reinterpret_cast<Dev<R> *>(desc)->u = nodes;
-        __syncthreads();
-    }
     const Dev<R> &L = *reinterpret_cast<const Dev<R> *>(desc);
+    if (L.ctl->stop) return;
+    const GlobalNodes<R> nodes{L.u};
     const unsigned I = S.iterations;
     // One bond per thread per round; the rounds of the whole sweep in order
     // (iteration, level, base). The next round's streamed data (record,
@@ -1777,27 +1698,11 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 2) kSweepLattice(const Grid
         const std::uint32_t d = cur.base + threadIdx.x;
         if (d < end && endsInBounds(now.rec, L.N, kSiteSolve)) {
             if (self_next && cur.it != 0) now.lam = __ldcs(L.lambda + d);
-            const bool live = !(now.rec.a & kDeadBit);
-            Q4<R> qa{}, qb{};
-            if (live) {
-                if constexpr (Staged) {
-                    qa = L.u[endA(now.rec)];
-                    qb = L.u[endB(now.rec)];
-                } else {
-                    qa = ldShared(L.u + endA(now.rec));
-                    qb = ldShared(L.u + endB(now.rec));
-                }
-            }
-            finishBond<R, Direct, Plastic, Support>(L, S, d, now.rec, live, now.geo, now.lam, now.pl,
-                                                    cur.it + 1 == I, qa, qb);
+            solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, d, now.rec, now.geo, now.lam, now.pl,
+                                                   cur.it + 1 == I);
         }
         if (!more) {
             supportIsolatedInCta<R, Support>(L, S);
-            if constexpr (Staged) {
-                // The staged positions back to global memory.
-                __syncthreads();
-                for (std::uint32_t i = threadIdx.x; i < node_count; i += blockDim.x) global_u[i] = L.u[i];
-            }
             break;
         }
         if (nxt.lv != cur.lv || nxt.it != cur.it) {
@@ -1810,6 +1715,117 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 2) kSweepLattice(const Grid
         cur = nxt;
         now = next;
     }
+}
+
+// The whole sweep of a small lattice in one CTA (float lane), its positions in
+// shared memory for every iteration and level: one thread for every bond of
+// the widest level, a CTA barrier between levels, the next level's records
+// fetched while this one is solved (two buffers, used in turn: a register
+// that a load is still filling is never copied, which would wait for the
+// load). The arithmetic and the per-node order are those of the level launches.
+//
+// What bounds it: a level is one dependent chain (gather, solve, write,
+// barrier), and its warps share one SM's issue slots. Spreading a lattice over
+// a thread-block cluster was measured and is not kept: making a level's writes
+// visible across the cluster costs 0.43 us (the fence 330 cycles of it), as
+// much as the launch of a level saves.
+constexpr std::uint32_t kStagedMaxNodes = 14336; // the launch shape's largest value; capped at kStagedNodes
+constexpr std::uint32_t kStagedNodes = 14080;    // 220 KiB, the level table and the descriptor beside
+constexpr std::uint32_t kStagedLevels = 512;
+constexpr unsigned kStagedThreads = 1024;        // at most; 64 registers a thread
+
+struct StagedNodes {
+    Q4<float> *u; // shared memory
+    __device__ __forceinline__ Q4<float> load(std::uint32_t i) const { return u[i]; }
+    __device__ __forceinline__ void store(std::uint32_t i, const Q4<float> &q) const { u[i] = q; }
+};
+
+template <bool Plastic, bool Support>
+__global__ void __launch_bounds__(kStagedThreads, 1)
+kSweepStaged(const __grid_constant__ Grid<float> launch, const __grid_constant__ Settings<float> S) {
+    extern __shared__ __align__(16) unsigned char staged_smem[];
+    __shared__ SharedDesc<float> desc;
+    const unsigned T = blockDim.x, t = threadIdx.x;
+    // The lattice's descriptor in shared memory, read from there as needed:
+    // one lattice's comes from the launch's own parameters.
+    {
+        const unsigned *src = reinterpret_cast<const unsigned *>(
+            launch.list ? launch.table + launch.list[blockIdx.x].lattice : &launch.one);
+        unsigned *dst = reinterpret_cast<unsigned *>(desc.bytes);
+        for (unsigned k = t; k < sizeof(Dev<float>) / sizeof(unsigned); k += T) dst[k] = src[k];
+        __syncthreads();
+    }
+    const Dev<float> &L = *reinterpret_cast<const Dev<float> *>(desc.bytes);
+    if (L.ctl->stop) return;
+    const std::uint32_t N = L.N, levels = L.level_count, I = S.iterations;
+    Q4<float> *own = reinterpret_cast<Q4<float> *>(staged_smem);
+    std::uint32_t *begin = reinterpret_cast<std::uint32_t *>(staged_smem + sizeof(Q4<float>) * N);
+    Q4<float> *const u = L.u;
+#pragma unroll 4
+    for (std::uint32_t k = t; k < N; k += T) own[k] = ldShared(u + k);
+    for (std::uint32_t k = t; k <= levels; k += T) begin[k] = L.level_begin[k];
+    const StagedNodes nodes{own};
+    const BondRec<float> *const recs = L.rec;
+    const Q4<float> *const geos = L.geo;
+    float *const lambdas = L.lambda;
+    __syncthreads();
+
+    // A bond is one thread's for the whole sweep, which writes its multiplier
+    // an iteration before reading it; with a single level that is the step
+    // before, so it is then loaded after the write.
+    const bool late_lambda = levels == 1;
+    struct Streamed {
+        BondRec<float> rec;
+        Q4<float> geo;
+        float lam, pl;
+        std::uint32_t d; // the bond, or kNoBond
+    };
+    auto fetch = [&](std::uint32_t it, std::uint32_t lv, Streamed &x) {
+        const std::uint32_t d = begin[lv] + t;
+        const bool has = it < I && d < begin[lv + 1];
+        x.d = has ? d : kNoBond;
+        if (has) {
+            x.rec = ldStream(recs + d);
+            x.geo = ldStream(geos + d);
+            x.lam = (it == 0 || late_lambda) ? 0.0F : __ldcs(lambdas + d);
+            x.pl = Plastic ? L.plastic[d].x : 0.0F;
+        }
+    };
+    std::uint32_t it = 0, lv = 0;
+    // One level; false after the last one of the sweep.
+    auto level = [&](Streamed &now, Streamed &next) {
+        const bool last = it + 1 == I;
+        std::uint32_t next_it = it, next_lv = lv + 1;
+        if (next_lv == levels) {
+            next_lv = 0;
+            ++next_it;
+        }
+        fetch(next_it, next_lv, next);
+        if (now.d != kNoBond && endsInBounds(now.rec, N, kSiteSolve)) {
+            if (late_lambda && it != 0) now.lam = __ldcs(lambdas + now.d);
+            solveBond<float, false, Plastic, Support>(L, S, nodes, lambdas, now.d, now.rec, now.geo, now.lam, now.pl, last);
+        }
+        if (Support && next_it != it) {
+            // Nodes without bonds, each iteration by the same thread; no
+            // bond's solve touches them.
+            for (std::uint32_t k = t; k < L.isolated_count; k += T) {
+                const std::uint32_t i = L.isolated[k];
+                if (!inBounds(i, N, kSiteIsolated)) continue;
+                const Q4<float> uq = nodes.load(i);
+                V3<float> p = xyz(uq);
+                if (supportProject(L, S, i, p)) nodes.store(i, Q4<float>{p.x, p.y, p.z, uq.w});
+            }
+        }
+        __syncthreads();
+        it = next_it;
+        lv = next_lv;
+        return it < I;
+    };
+    Streamed x0{}, x1{};
+    fetch(0, 0, x0);
+    while (level(x0, x1) && level(x1, x0)) {
+    }
+    for (std::uint32_t k = t; k < N; k += T) u[k] = own[k];
 }
 
 // Radial pair damping of one level (LatticePhysics.hpp:1170-1184).
