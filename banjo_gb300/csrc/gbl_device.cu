@@ -2465,7 +2465,7 @@ private:
         check(cudaEventRecord(load_join_, loads_), "event");
         if (S.sphere_enabled && slabs_.count) {
             kCandidates<R, M><<<slabs_.count, 1024, 0, st>>>(grid(slabs_));
-            kMarkHalo<R, M><<<slabs_.count, 1024, 0, st>>>(grid(slabs_));
+            kMarkHalo<R, M><<<dim3(slabs_.count, kHaloParts), 1024, 0, st>>>(grid(slabs_));
         }
         mark(3);
         if (side_restart) {
