@@ -2676,10 +2676,7 @@ private:
                                                                                         plate, yield);
         }
         mark(1);
-        if (bonds_.count)
-            kRestartBondsAll<R, M, kDirect><<<bonds_.count, kThreads, 0, st>>>(grid(bonds_), after_kick);
-        if (nodes_.count)
-            kRestartBondsDirty<R, M, kDirect><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), after_kick);
+        if (bonds_.count) kRestartBonds<R, M, kDirect><<<bonds_.count, kThreads, 0, st>>>(grid(bonds_), after_kick);
         mark(2);
     }
 

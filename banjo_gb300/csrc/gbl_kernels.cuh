@@ -587,33 +587,32 @@ __device__ __forceinline__ void startSample(const Dev<R> &L, std::uint32_t j) {
     L.prev[j] = p;
 }
 
-// Every live bond, after an upload: items cover the bond storage range.
+// Every live bond after an upload, or the live bonds at each dirty node after a
+// failure round: items cover the bond storage range, and the lattice's threads
+// share the (slot, dirty node) pairs, consecutive threads on consecutive dirty
+// nodes. A bond with both ends dirty is sampled twice to the same values. (One
+// thread per dirty node walking its slots was a chain of 18 or 32 samples: 39
+// us a substep in the 32x8x8 beam, now 8; 100 in the 128x32x32 bar, now 11.)
 template <class R, bool Many, bool Direct>
-__global__ void __launch_bounds__(kThreads) kRestartBondsAll(const Grid<R> launch, int after_kick) {
+__global__ void __launch_bounds__(kThreads) kRestartBonds(const Grid<R> launch, int after_kick) {
     const Work w = item<Many>(launch);
     Dev<R> L = descriptor<R, Many>(launch, w);
     if (after_kick) L.u = L.up;
-    if (L.ctl->stop || !L.ctl->full_restart) return;
+    if (L.ctl->stop) return;
     const std::uint32_t d = w.begin + threadIdx.x;
-    if (d < w.end) startSample<R, Direct>(L, d);
-}
-
-// The live bonds at each dirty node, after a failure round: items cover the
-// node index range (one thread per dirty-list entry, over its neighbour
-// slots). A bond with both ends dirty is sampled twice to the same values.
-template <class R, bool Many, bool Direct>
-__global__ void __launch_bounds__(kThreads) kRestartBondsDirty(const Grid<R> launch, int after_kick) {
-    const Work w = item<Many>(launch);
-    Dev<R> L = descriptor<R, Many>(launch, w);
-    if (after_kick) L.u = L.up;
-    if (L.ctl->stop || L.ctl->full_restart) return;
-    const std::uint32_t t = w.begin + threadIdx.x;
-    if (t >= w.end || t >= L.ctl->dirty_count) return;
-    const std::uint32_t node = L.dirty_list[t];
-    if (!inBounds(node, L.N, kSiteDirty)) return;
-    for (std::uint32_t k = 0; k < L.D; ++k) {
-        const std::uint32_t d = L.nbr_bond[static_cast<std::size_t>(k) * L.N + node];
-        if (d != kNoBond && inBounds(d, L.B, kSiteDirtyBond)) startSample<R, Direct>(L, d);
+    if (d >= w.end) return;
+    if (L.ctl->full_restart) {
+        startSample<R, Direct>(L, d);
+        return;
+    }
+    const std::uint32_t dirty = L.ctl->dirty_count;
+    const std::uint64_t pairs = static_cast<std::uint64_t>(dirty) * L.D;
+    for (std::uint64_t q = d; q < pairs; q += L.B) {
+        const std::uint32_t k = static_cast<std::uint32_t>(q / dirty);
+        const std::uint32_t node = L.dirty_list[q - static_cast<std::uint64_t>(k) * dirty];
+        if (!inBounds(node, L.N, kSiteDirty)) continue;
+        const std::uint32_t bond = L.nbr_bond[static_cast<std::size_t>(k) * L.N + node];
+        if (bond != kNoBond && inBounds(bond, L.B, kSiteDirtyBond)) startSample<R, Direct>(L, bond);
     }
 }
 
