@@ -802,11 +802,12 @@ template <class R> struct Resident {
         a.reserve(d.engaged, kPlanes * static_cast<std::size_t>(N));
         a.reserve(d.candidate, N); a.reserve(d.cand_bits, (N + 31) / 32 + 1);
         a.reserve(d.lambda, B);
-        a.reserve(d.ev_bits, d.words_b + 1); a.reserve(d.ev_tile, d.tiles_b + 1); a.reserve(d.ev_list, B + 1);
-        a.reserve(d.ev_removed, B); a.reserve(d.ev_packed, B + 1); a.reserve(d.ev_prefix, B + 1);
+        const std::size_t words = static_cast<std::size_t>(d.tiles_b) * kTileWords;
+        a.reserve(d.ev_bits, words); a.reserve(d.ev_tile, d.tiles_b + 1);
+        a.reserve(d.ev_removed, B);
         a.reserve(d.ev_ends, B);
-        a.reserve(d.dmg_bits, d.words_b + 1); a.reserve(d.dmg_tile, d.tiles_b + 1);
-        a.reserve(d.dmg_list, B + 1); a.reserve(d.ev_damage, B); a.reserve(d.dmg_value, B + 1);
+        a.reserve(d.dmg_bits, words); a.reserve(d.dmg_tile, d.tiles_b + 1);
+        a.reserve(d.ev_damage, B); a.reserve(d.dmg_value, B + 1);
         a.reserve(d.tile_plastic, d.tiles_b + 1); a.reserve(d.tile_removed, d.tiles_b + 1);
         const std::size_t scan_blocks = d.tiles_b / kScanBlock + 1;
         a.reserve(d.blk_ev, scan_blocks); a.reserve(d.blk_dmg, scan_blocks);
@@ -823,7 +824,6 @@ template <class R> struct Resident {
     static std::size_t footprint(std::uint32_t N, std::uint32_t B, std::uint32_t D, std::uint32_t blocks) {
         Arena a;
         Dev<R> d{};
-        d.words_b = (B + 31) / 32;
         d.tiles_b = (B + kThreads - 1) / kThreads;
         reserve(a, d, N, B, D, blocks, N);
         return a.bytes() + static_cast<std::size_t>(N) * (sizeof(Q4<R>) + 16 * sizeof(double) + sizeof(std::uint32_t));
@@ -843,7 +843,6 @@ template <class R> struct Resident {
         Dev<R> &d = dev;
         d = Dev<R>{};
         d.N = N; d.B = B; d.D = D; d.blocks = sched.block_count;
-        d.words_b = (B + 31) / 32;
         d.tiles_b = (B + kThreads - 1) / kThreads;
         filled_ = reserve(arena, d, N, B, D, sched.block_count, isolated.size());
         mass.resize(N);
@@ -1000,7 +999,7 @@ template <class R> struct Resident {
         }
         if (B) {
             const unsigned grid = reorderGrid(B);
-            std::uint32_t *sched2dev_dev = dev.ev_list; // scratch of the cleared part, cleared below
+            std::uint32_t *sched2dev_dev = dev.ffb; // scratch of the cleared part, cleared below
             kInvertOrder<<<grid, kThreads, 0, stream>>>(sched2dev_dev, dev.dev2sched, B);
             const std::size_t P = static_cast<std::size_t>(dev.D) * N;
             if (P) kSlotsToStorage<<<reorderGrid(P), kThreads, 0, stream>>>(dev.nbr_bond, sched2dev_dev, P);
@@ -2289,7 +2288,10 @@ private:
         using U = std::uint32_t;
         nodes_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.N; }, kThreads);
         bonds_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.B; }, kThreads);
-        tiles_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.dev.tiles_b; }, kThreads / 32);
+        tiles_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.dev.tiles_b; }, kCountTiles);
+        static_assert(kCountTiles == kEmitTiles * (kEmitThreads / 32), "one item of tiles for both launches");
+        several_blocks_ = false;
+        for (auto k : active_) several_blocks_ = several_blocks_ || slots_[k]->dev.tiles_b >= kScanBlock;
         blocks_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.dev.tiles_b / kScanBlock + 1; }, 1);
         each_ = span([](const Res &, U &b, U &e) { b = 0; e = 1; }, 1);
         slabs_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.sched.block_count; }, 1);
@@ -2317,15 +2319,6 @@ private:
                     staged_threads_ = std::max(staged_threads_, std::max(64U, (widestLevel(l) + 31) / 32 * 32));
                     staged_smem_ = std::max(staged_smem_, sizeof(Q4<float>) * l.N + 4 * (l.levels.size() + 1));
                 }
-        }
-        {
-            const U first = static_cast<U>(all.size());
-            for (auto k : active_) {
-                const U parts = std::max(1U, std::min(608U, slots_[k]->B / 65536U));
-                for (U q = 0; q < parts; ++q) all.push_back({k, q, parts});
-            }
-            const U count = static_cast<U>(all.size()) - first;
-            broken_ = Span{first, count, 0, count, 1};
         }
         {
             // One item per (lattice, wrench slot): the batch's spreads in one launch.
@@ -2515,10 +2508,9 @@ private:
         if (contact) contactPhase<M>(st, mark);
         endPhase<M>(st, split ? 2 : 0, mark);
         if (tiles_.count) kTileCounts<R, M><<<tiles_.count, kThreads, 0, st>>>(grid(tiles_));
-        kBlockScan<R, M><<<blocks_.count, kScanBlock, 0, st>>>(grid(blocks_), plastic_ ? 1 : 0);
-        kTopScan<R, M><<<each_.count, kScanBlock, 0, st>>>(grid(each_));
-        if (tiles_.count) kEmitEvents<R, M><<<tiles_.count, kThreads, 0, st>>>(grid(tiles_));
-        kLedgerBroken<R, M><<<broken_.count, kThreads, 0, st>>>(grid(broken_));
+        kEventScan<R, M><<<blocks_.count, kScanBlock, 0, st>>>(grid(blocks_), plastic_ ? 1 : 0);
+        if (several_blocks_) kTopScan<R, M><<<each_.count, kScanBlock, 0, st>>>(grid(each_));
+        if (tiles_.count) kEmitEvents<R, M><<<tiles_.count, kEmitThreads, 0, st>>>(grid(tiles_));
         mark(12);
         check(cudaStreamWaitEvent(st, load_join_, 0), "stream wait");
         kLedger<R, M><<<each_.count, 32, 0, st>>>(grid(each_), S);
@@ -2729,11 +2721,12 @@ private:
     unsigned *running_{}, *running_host_{};
     Dev<R> *table_{};
     Work *work_{};
-    Span nodes_{}, bonds_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, broken_{}, whole_{}, buckets_{},
+    Span nodes_{}, bonds_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, whole_{}, buckets_{},
         wrench_{};
     unsigned staged_threads_{0}; // the staged sweep's CTA size (0: the lattices do not sweep staged)
     std::size_t staged_smem_{0};
     unsigned sms_{1};
+    bool several_blocks_{false}; // a lattice has more than one scan block of tiles
     // Level-launched lattices, in groups swept one after another.
     struct Group {
         std::vector<Span> levels;

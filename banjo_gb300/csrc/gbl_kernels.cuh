@@ -172,7 +172,7 @@ constexpr unsigned kErrExternalOverflow = 1;
 constexpr unsigned kErrWrench = 2;
 
 template <class R> struct Dev {
-    std::uint32_t N, B, D, blocks, words_b, tiles_b;
+    std::uint32_t N, B, D, blocks, tiles_b;
     Q4<R> *u, *v, *x0, *up, *strain;
     R *rinv, *unm, *approach;
     std::uint8_t *dirty, *engaged, *candidate;
@@ -185,20 +185,20 @@ template <class R> struct Dev {
     Q2<R> *thr2, *plastic;
     R *lambda;
     std::uint8_t *mode;
-    // Substep ledger scratch. ev_*: broken bonds (bit per bond, per-tile count
-    // then offset, ordered list, removed energy by bond and packed in list
-    // order, in-tile inclusive prefix); dmg_*: bonds whose damage passed the
-    // run maximum (the candidates of the damage-record scan); tile_*: per
-    // end-sample tile FP64 partials and their prefix.
-    std::uint32_t *ev_bits, *ev_tile, *ev_list;
-    double *ev_removed, *ev_packed, *ev_prefix;
+    // Substep ledger scratch. ev_*: broken bonds (bit per bond, whole tiles of
+    // words; per-tile offset; removed energy by bond); dmg_*: bonds whose
+    // damage passed the run maximum (the candidates of the damage-record
+    // scan, their values in bond order); tile_*: per end-sample tile plastic
+    // work, per tile the prefix of the removed energy.
+    std::uint32_t *ev_bits, *ev_tile;
+    double *ev_removed;
     uint2 *ev_ends;               // the two nodes of a broken bond, by schedule index
     std::uint32_t *dev2sched;     // bond storage order (level-major) -> schedule index
     std::uint32_t *isolated;      // nodes without bonds (their support projection has no sweep to ride on)
     std::uint32_t isolated_count;
     std::uint32_t *level_begin;   // sweep level boundaries in storage order (level_count + 1), when level_count fits
     std::uint32_t level_count;
-    std::uint32_t *dmg_bits, *dmg_tile, *dmg_list;
+    std::uint32_t *dmg_bits, *dmg_tile;
     float *ev_damage, *dmg_value;
     double *tile_plastic, *tile_removed;
     std::uint32_t *blk_ev, *blk_dmg;   // per scan block of tiles: totals, then offsets
@@ -257,12 +257,6 @@ template <bool Many, class R> __device__ __forceinline__ Work item(const Grid<R>
     if (Many) return g.list[blockIdx.x];
     const std::uint32_t b = g.base + blockIdx.x * g.per;
     return Work{0U, b, b + g.per < g.end ? b + g.per : g.end};
-}
-
-// Items of a launch split into parts: {lattice, part, parts}.
-template <bool Many, class R> __device__ __forceinline__ Work part(const Grid<R> &g) {
-    if (Many) return g.list[blockIdx.x];
-    return Work{0U, blockIdx.x, gridDim.x};
 }
 
 template <class R, bool Many> __device__ __forceinline__ Dev<R> descriptor(const Grid<R> &g, const Work &w) {
@@ -1918,7 +1912,7 @@ __global__ void __launch_bounds__(kThreads) kSupportVelocity(const Grid<R> launc
 // depends on the bond order only, never on thread timing: plastic work is
 // summed per tile by a fixed shuffle tree and the tiles in index order; broken
 // bonds and damage-record candidates are flagged one bit per bond and listed
-// in bond order by kTileCounts/kBlockScan/kTopScan/kEmitEvents.
+// in bond order by kTileCounts/kEventScan/kTopScan/kEmitEvents.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned floatBits(float x) { return __float_as_uint(x); }
 
@@ -2069,26 +2063,18 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
 // The substep ledger's ordered lists and FP64 sums, fully parallel and in a
 // fixed order. A "tile" is 256 bonds of schedule order (8 bit words); a scan
 // block is kScanBlock tiles. Every sum below is formed in an order fixed by the
-// bond order alone: sequential inside a 32-bond word, a Hillis-Steele scan
-// across the words of a tile, across the tiles of a block, across the blocks.
+// bond order alone: sequential inside a 32-bond word, a tree over the words of
+// a tile, shuffle scans across the tiles of a block (warps, then their
+// totals), the same across the blocks.
+//
+// These are small launches whose time is their own latency: barriers (a scan
+// through shared memory took twenty of them per value, two now) and, where
+// bonds break, the loads of their records, which therefore go word by word or
+// bond by bond in parallel (one thread summing a whole tile's made the scan of
+// 128 shattering trials, end sample included, 1.17 ms long against 0.62).
 // ---------------------------------------------------------------------------
 constexpr unsigned kScanBlock = 1024;
-
-// Hillis-Steele inclusive scan of one double per thread across a 1024-thread
-// CTA (a fixed order); `buf` is 1024 doubles of shared memory.
-__device__ __forceinline__ double blockInclusiveScan(double x, double *buf) {
-    buf[threadIdx.x] = x;
-    __syncthreads();
-    for (unsigned o = 1; o < blockDim.x; o <<= 1) {
-        const double y = threadIdx.x >= o ? buf[threadIdx.x - o] : 0.0;
-        __syncthreads();
-        if (threadIdx.x >= o) buf[threadIdx.x] += y;
-        __syncthreads();
-    }
-    const double r = buf[threadIdx.x];
-    __syncthreads();
-    return r;
-}
+constexpr unsigned kTileWords = kThreads / 32;
 
 __device__ __forceinline__ unsigned blockExclusiveScanU(unsigned x, unsigned *buf, unsigned &total) {
     buf[threadIdx.x] = x;
@@ -2105,238 +2091,254 @@ __device__ __forceinline__ unsigned blockExclusiveScanU(unsigned x, unsigned *bu
     return inclusive - x;
 }
 
-// Removed energy of a tile's broken bonds: per word, in bit order; across the
-// tile's words by an inclusive shuffle scan. Returns this lane's inclusive sum
-// (lane 7, or the last word of the tile, holds the tile's total).
-__device__ __forceinline__ double tileRemovedScan(double own) {
+// Inclusive scan over a warp in a fixed order.
+template <class T> __device__ __forceinline__ T warpInclusive(T x) {
     const unsigned lane = threadIdx.x & 31;
-    double inclusive = own;
     for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(0xffffffffU, inclusive, o);
-        if (lane >= static_cast<unsigned>(o)) inclusive += y;
+        const T y = __shfl_up_sync(0xffffffffU, x, o);
+        if (lane >= static_cast<unsigned>(o)) x += y;
     }
-    return inclusive;
+    return x;
 }
 
-// One warp per tile: broken-bond and damage-candidate counts and the tile's
-// removed energy.
+// What one thread of a 1024-thread CTA contributes to the ledger's scans, and
+// what comes back: its exclusive prefixes, and the CTA's totals.
+struct LedgerScan {
+    unsigned broken, damaged;
+    double removed, work; // work: total only
+};
+__device__ __forceinline__ LedgerScan ledgerScan(const LedgerScan &in, LedgerScan &total) {
+    __shared__ unsigned wb[32], wd[32];
+    __shared__ double wr[32], ww[32];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    const unsigned ib = warpInclusive(in.broken), id = warpInclusive(in.damaged);
+    const double ir = warpInclusive(in.removed), work = warpSumFixed(in.work);
+    if (lane == 31) {
+        wb[warp] = ib;
+        wd[warp] = id;
+        wr[warp] = ir;
+    }
+    if (lane == 0) ww[warp] = work;
+    __syncthreads();
+    // Every warp scans the 32 totals itself: no second trip through memory.
+    const unsigned tb = warpInclusive(wb[lane]), td = warpInclusive(wd[lane]);
+    const double tr = warpInclusive(wr[lane]), tw = warpSumFixed(ww[lane]);
+    total = {__shfl_sync(0xffffffffU, tb, 31), __shfl_sync(0xffffffffU, td, 31), __shfl_sync(0xffffffffU, tr, 31),
+             __shfl_sync(0xffffffffU, tw, 0)};
+    const int before = static_cast<int>(warp) - 1;
+    const unsigned sb = __shfl_sync(0xffffffffU, tb, before < 0 ? 0 : before);
+    const unsigned sd = __shfl_sync(0xffffffffU, td, before < 0 ? 0 : before);
+    const double sr = __shfl_sync(0xffffffffU, tr, before < 0 ? 0 : before);
+    const double er = __shfl_up_sync(0xffffffffU, ir, 1);
+    LedgerScan out;
+    out.broken = (before < 0 ? 0U : sb) + ib - in.broken;
+    out.damaged = (before < 0 ? 0U : sd) + id - in.damaged;
+    out.removed = (before < 0 ? 0.0 : sr) + (lane == 0 ? 0.0 : er);
+    out.work = 0.0;
+    __syncthreads(); // the totals may be overwritten by a next round
+    return out;
+}
+
+// A word's removed energy, in bond order.
+__device__ __forceinline__ double wordRemoved(const double *removed, std::uint32_t word, unsigned bits) {
+    double sum = 0.0;
+    for (; bits; bits &= bits - 1) sum += removed[word * 32 + static_cast<unsigned>(__ffs(bits) - 1)];
+    return sum;
+}
+
+// The substep's totals, once every block's prefix is known.
+__device__ __forceinline__ void ledgerTotals(Ctl &c, const LedgerScan &total) {
+    c.event_count = total.broken;
+    c.dmg_count = total.damaged;
+    c.removed_substep = total.removed;
+    c.plastic_substep = total.work;
+    c.energy_gain = 0;
+    c.dirty_count = 0; // the restart of this substep has consumed the list
+}
+
+// Eight lanes per tile, one per word: broken-bond and damage-candidate counts
+// and the tile's removed energy.
+constexpr unsigned kCountTiles = kThreads / kTileWords; // tiles per CTA
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kTileCounts(const Grid<R> launch) {
     const Work w = item<Many>(launch);
-    const Dev<R> L = descriptor<R, Many>(launch, w);
+    __shared__ SharedDesc<R> desc;
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     if (L.ctl->stop) return;
-    const unsigned tile = w.begin + threadIdx.x / 32; // items: up to 8 tiles of one lattice
-    const unsigned lane = threadIdx.x & 31;
-    if (tile >= w.end) return;
-    constexpr unsigned kWords = kThreads / 32;
-    const unsigned wd = tile * kWords + lane;
-    const bool word = lane < kWords && wd < L.words_b;
-    const unsigned bits = word ? L.ev_bits[wd] : 0U;
-    const unsigned dbits = word ? L.dmg_bits[wd] : 0U;
-    double own = 0.0;
-    for (unsigned m = bits; m; m &= m - 1) own += L.ev_removed[wd * 32 + static_cast<unsigned>(__ffs(m) - 1)];
-    unsigned nb = __popc(bits), nd = __popc(dbits);
-    for (int o = 16; o > 0; o >>= 1) {
-        nb += __shfl_down_sync(0xffffffffU, nb, o);
-        nd += __shfl_down_sync(0xffffffffU, nd, o);
+    const unsigned tile = w.begin + threadIdx.x / kTileWords; // items: up to kCountTiles tiles of one lattice
+    const bool in = tile < w.end;
+    const std::uint32_t wd = tile * kTileWords + threadIdx.x % kTileWords;
+    const unsigned bits = in ? L.ev_bits[wd] : 0U;
+    unsigned broken = __popc(bits), damaged = in ? __popc(L.dmg_bits[wd]) : 0U;
+    double removed = bits ? wordRemoved(L.ev_removed, wd, bits) : 0.0;
+    for (int o = 1; o < static_cast<int>(kTileWords); o <<= 1) {
+        broken += __shfl_xor_sync(0xffffffffU, broken, o);
+        damaged += __shfl_xor_sync(0xffffffffU, damaged, o);
+        removed += __shfl_xor_sync(0xffffffffU, removed, o);
     }
-    const double total = __shfl_sync(0xffffffffU, tileRemovedScan(own), 31);
-    if (lane == 0) {
-        L.ev_tile[tile] = nb;
-        L.dmg_tile[tile] = nd;
-        L.tile_removed[tile] = total;
+    if (in && threadIdx.x % kTileWords == 0) {
+        L.ev_tile[tile] = broken;
+        L.dmg_tile[tile] = damaged;
+        L.tile_removed[tile] = removed;
     }
 }
 
-// One CTA per scan block: exclusive offsets of the tiles inside the block (in
-// place) and the block's totals; the plastic work of the end-sample tiles of
-// the same index range is reduced by a fixed tree.
+// One CTA per scan block, a thread per tile: the tiles' exclusive offsets
+// inside the block, and the block's totals with its plastic work. A lattice
+// of one block (up to 262,143 bonds) is done; kTopScan follows for the others.
 template <class R, bool Many>
-__global__ void __launch_bounds__(kScanBlock) kBlockScan(const Grid<R> launch, int plastic) {
+__global__ void __launch_bounds__(kScanBlock) kEventScan(const Grid<R> launch, int plastic) {
     const Work w = item<Many>(launch);
-    const Dev<R> L = descriptor<R, Many>(launch, w);
-    __shared__ double dbuf[kScanBlock];
-    __shared__ unsigned ubuf[kScanBlock];
-    if (L.ctl->stop) return;
+    __shared__ SharedDesc<R> desc;
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
+    Ctl &c = *L.ctl;
+    if (c.stop) return;
     const unsigned blk = w.begin; // one item per (lattice, scan block)
     const unsigned t = blk * kScanBlock + threadIdx.x;
     const bool in = t < L.tiles_b;
-    unsigned tb = 0, td = 0;
-    const unsigned ob = blockExclusiveScanU(in ? L.ev_tile[t] : 0U, ubuf, tb);
-    const unsigned od = blockExclusiveScanU(in ? L.dmg_tile[t] : 0U, ubuf, td);
-    // The inclusive scan leaves dbuf holding every thread's inclusive sum.
-    (void)blockInclusiveScan(in ? L.tile_removed[t] : 0.0, dbuf);
-    const double exclusive = threadIdx.x ? dbuf[threadIdx.x - 1] : 0.0;
-    const double removed_total = dbuf[kScanBlock - 1];
-    __syncthreads();
+    LedgerScan own{0U, 0U, 0.0, plastic && in ? L.tile_plastic[t] : 0.0};
     if (in) {
-        L.ev_tile[t] = ob;
-        L.dmg_tile[t] = od;
-        L.tile_removed[t] = exclusive;
+        own.broken = L.ev_tile[t];
+        own.damaged = L.dmg_tile[t];
+        own.removed = L.tile_removed[t];
     }
-    double block_work = 0.0;
-    if (plastic) {
-        dbuf[threadIdx.x] = in ? L.tile_plastic[t] : 0.0;
-        __syncthreads();
-        for (unsigned s = kScanBlock / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) dbuf[threadIdx.x] += dbuf[threadIdx.x + s];
-            __syncthreads();
-        }
-        block_work = dbuf[0];
+    LedgerScan total{};
+    const LedgerScan before = ledgerScan(own, total);
+    // Only a tile with events is looked at again.
+    if (in && (own.broken || own.damaged)) {
+        L.ev_tile[t] = before.broken;
+        L.dmg_tile[t] = before.damaged;
+        L.tile_removed[t] = before.removed;
     }
     if (threadIdx.x == 0) {
-        L.blk_ev[blk] = tb;
-        L.blk_dmg[blk] = td;
-        L.blk_removed[blk] = removed_total;
-        L.blk_plastic[blk] = block_work;
+        const bool alone = L.tiles_b < kScanBlock;
+        L.blk_ev[blk] = alone ? 0U : total.broken;
+        L.blk_dmg[blk] = alone ? 0U : total.damaged;
+        L.blk_removed[blk] = alone ? 0.0 : total.removed;
+        L.blk_plastic[blk] = total.work;
+        if (alone) ledgerTotals(c, total);
     }
 }
 
-// One CTA: exclusive offsets of the blocks (rounds of 1024 blocks with a
-// carry), and the substep's totals.
+// One CTA per lattice of several blocks: their exclusive offsets (rounds of
+// 1024 blocks with a carry), and the substep's totals.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kScanBlock) kTopScan(const Grid<R> launch) {
     const Work w = item<Many>(launch);
-    const Dev<R> L = descriptor<R, Many>(launch, w);
+    __shared__ SharedDesc<R> desc;
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     const unsigned blocks = L.tiles_b / kScanBlock + 1; // one item per lattice
-    __shared__ double dbuf[kScanBlock];
-    __shared__ unsigned ubuf[kScanBlock];
-    __shared__ double plastic_carry;
     Ctl &c = *L.ctl;
-    if (c.stop) return;
-    unsigned carry_b = 0, carry_d = 0;
-    double carry_r = 0.0;
-    if (threadIdx.x == 0) plastic_carry = 0.0;
+    if (c.stop || blocks == 1) return;
+    LedgerScan carry{0U, 0U, 0.0, 0.0};
     for (unsigned base = 0; base < blocks; base += kScanBlock) {
         const unsigned k = base + threadIdx.x;
         const bool in = k < blocks;
-        unsigned tb = 0, td = 0;
-        const unsigned ob = blockExclusiveScanU(in ? L.blk_ev[k] : 0U, ubuf, tb);
-        const unsigned od = blockExclusiveScanU(in ? L.blk_dmg[k] : 0U, ubuf, td);
-        (void)blockInclusiveScan(in ? L.blk_removed[k] : 0.0, dbuf);
-        const double before = threadIdx.x ? dbuf[threadIdx.x - 1] : 0.0;
-        const double round_total = dbuf[kScanBlock - 1];
-        __syncthreads();
-        dbuf[threadIdx.x] = in ? L.blk_plastic[k] : 0.0;
-        __syncthreads();
-        for (unsigned s = kScanBlock / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) dbuf[threadIdx.x] += dbuf[threadIdx.x + s];
-            __syncthreads();
-        }
+        LedgerScan own{0U, 0U, 0.0, 0.0}, total{};
+        if (in) own = {L.blk_ev[k], L.blk_dmg[k], L.blk_removed[k], L.blk_plastic[k]};
+        const LedgerScan before = ledgerScan(own, total);
         if (in) {
-            L.blk_ev[k] = carry_b + ob;
-            L.blk_dmg[k] = carry_d + od;
-            L.blk_removed[k] = carry_r + before;
+            L.blk_ev[k] = carry.broken + before.broken;
+            L.blk_dmg[k] = carry.damaged + before.damaged;
+            L.blk_removed[k] = carry.removed + before.removed;
         }
-        if (threadIdx.x == 0) plastic_carry += dbuf[0];
-        carry_b += tb;
-        carry_d += td;
-        carry_r += round_total;
-        __syncthreads();
+        carry.broken += total.broken;
+        carry.damaged += total.damaged;
+        carry.removed += total.removed;
+        carry.work += total.work;
     }
-    if (threadIdx.x == 0) {
-        c.event_count = carry_b;
-        c.dmg_count = carry_d;
-        c.removed_substep = carry_r;
-        c.plastic_substep = plastic_carry;
-        c.energy_gain = 0;
-        c.dirty_count = 0; // the restart of this substep has consumed the list
-    }
+    if (threadIdx.x == 0) ledgerTotals(c, carry);
 }
 
-// One warp per tile: the tile's broken bonds in bond order with their removed
-// energy and their prefix of the substep's removed energy (block offset, tile
-// offset, in-tile inclusive scan: the same orders as the counts), and its
-// damage candidates in order. The bit words are cleared for the next substep.
+// One warp per kEmitTiles tiles, the tiles with events one after another, in
+// bond order. Broken bonds: the energy-gain test of each against the running
+// removed energy it would see (CpuLatticeBackend.cpp:469-474; its prefix is
+// block offset, tile offset and in-tile scan, the orders of the counts), the
+// first-failure list, and the dirty marks and list of the next substep's
+// restart (CpuLatticeBackend.cpp:476-477). Damage candidates: their values in
+// order. The bit words are cleared for the next substep. A tile's bonds are
+// listed in shared memory by the lane of their word, then taken one per lane,
+// so that their records' loads and the dirty marks' atomics overlap.
+constexpr unsigned kEmitTiles = 8;
+constexpr unsigned kEmitThreads = 128;
 template <class R, bool Many>
-__global__ void __launch_bounds__(kThreads) kEmitEvents(const Grid<R> launch) {
+__global__ void __launch_bounds__(kEmitThreads) kEmitEvents(const Grid<R> launch) {
     const Work w = item<Many>(launch);
-    const Dev<R> L = descriptor<R, Many>(launch, w);
-    const Ctl &c = *L.ctl;
-    if (c.stop || (c.event_count == 0 && c.dmg_count == 0)) return;
-    const unsigned tile = w.begin + threadIdx.x / 32;
-    const unsigned lane = threadIdx.x & 31;
-    if (tile >= w.end) return;
-    constexpr unsigned kWords = kThreads / 32;
-    const unsigned wd = tile * kWords + lane;
-    const bool word = lane < kWords && wd < L.words_b;
-    const unsigned blk = tile / kScanBlock;
-    unsigned bits = word ? L.ev_bits[wd] : 0U;
-    if (__any_sync(0xffffffffU, bits != 0)) {
-        double own = 0.0;
-        for (unsigned m = bits; m; m &= m - 1) own += L.ev_removed[wd * 32 + static_cast<unsigned>(__ffs(m) - 1)];
-        const double inclusive = tileRemovedScan(own);
-        const double exclusive = __shfl_up_sync(0xffffffffU, inclusive, 1);
-        unsigned n = __popc(bits), x = n;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffU, x, o);
-            if (lane >= static_cast<unsigned>(o)) x += y;
-        }
-        unsigned at = L.blk_ev[blk] + L.ev_tile[tile] + x - n;
-        const double offset = L.blk_removed[blk] + L.tile_removed[tile];
-        double run = lane == 0 ? 0.0 : exclusive;
-        for (; bits; bits &= bits - 1) {
-            const unsigned j = wd * 32 + static_cast<unsigned>(__ffs(bits) - 1);
-            const double e = L.ev_removed[j];
-            run += e;
-            L.ev_list[at] = j;
-            L.ev_packed[at] = e;
-            L.ev_prefix[at] = offset + run;
-            ++at;
-        }
-        if (word) L.ev_bits[wd] = 0; // the end sample sets bits with atomicOr
-    }
-    unsigned dbits = word ? L.dmg_bits[wd] : 0U;
-    if (__any_sync(0xffffffffU, dbits != 0)) {
-        unsigned n = __popc(dbits), x = n;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffU, x, o);
-            if (lane >= static_cast<unsigned>(o)) x += y;
-        }
-        unsigned at = L.blk_dmg[blk] + L.dmg_tile[tile] + x - n;
-        for (; dbits; dbits &= dbits - 1) {
-            const unsigned j = wd * 32 + static_cast<unsigned>(__ffs(dbits) - 1);
-            L.dmg_list[at] = j;
-            L.dmg_value[at] = L.ev_damage[j];
-            ++at;
-        }
-        if (word) L.dmg_bits[wd] = 0;
-    }
-}
-
-// Parallel over this substep's broken bonds, in list order: the energy-gain
-// test of each bond against the running removed energy it would see
-// (CpuLatticeBackend.cpp:469-474), the first-failure list, and the dirty
-// marks and list of the next substep's restart (CpuLatticeBackend.cpp:476-477).
-template <class R, bool Many>
-__global__ void __launch_bounds__(kThreads) kLedgerBroken(const Grid<R> launch) {
-    const Work w = part<Many>(launch);
-    const Dev<R> L = descriptor<R, Many>(launch, w);
+    __shared__ SharedDesc<R> desc;
+    __shared__ std::uint16_t lists[kEmitThreads / 32][kThreads];
+    __shared__ double energies[kEmitThreads / 32][kThreads];
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     Ctl &c = *L.ctl;
-    if (c.stop) return;
-    const unsigned n = c.event_count;
+    if (c.stop || (c.event_count == 0 && c.dmg_count == 0)) return;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    std::uint16_t *list = lists[warp];  // a tile's broken bonds in order, then its damage candidates
+    double *energy = energies[warp];    // the removed energy of each, then its in-tile inclusive prefix
     const bool first_round = c.broken_bonds == 0;
     const double prior = c.removed_energy;
     const double fraction = c.energy_flat_fraction;
-    // Items: part `begin` of `end` parts of this lattice's event list.
-    for (unsigned e = w.begin * blockDim.x + threadIdx.x; e < n; e += w.end * blockDim.x) {
-        const std::uint32_t j = L.ev_list[e];
-        if (!inBounds(j, L.B, kSiteEvent)) continue;
-        const double running = prior + L.ev_prefix[e];
-        const double removed = L.ev_packed[e];
-        if (removed > fraction * (running < 1.0e-12 ? 1.0e-12 : running)) atomicOr(&c.energy_gain, 1U);
-        if (first_round) L.ffb[e] = j;
-        const uint2 e2 = L.ev_ends[j];
-        const std::uint32_t ends[2] = {e2.x, e2.y};
-        for (int q = 0; q < 2; ++q) {
-            const std::uint32_t node = ends[q];
-            if (!inBounds(node, L.N, kSiteEventEnd)) continue;
-            unsigned *word = reinterpret_cast<unsigned *>(L.dirty + (node & ~3U));
-            const unsigned bit = 1U << (8 * (node & 3U));
-            if (!(atomicOr(word, bit) & bit)) {
-                const unsigned at = atomicAdd(&c.dirty_count, 1U);
-                if (inBounds(at, L.N, kSiteDirty)) L.dirty_list[at] = node;
+    const unsigned first = w.begin + warp * kEmitTiles; // items: up to kEmitTiles tiles per warp of one lattice
+    for (unsigned tile = first; tile < first + kEmitTiles && tile < w.end; ++tile) {
+        const unsigned wd = tile * kTileWords + lane;
+        const unsigned blk = tile / kScanBlock;
+        const unsigned bits = lane < kTileWords ? L.ev_bits[wd] : 0U;
+        const unsigned dbits = lane < kTileWords ? L.dmg_bits[wd] : 0U;
+        // The set bits of the lanes' words into `list`, in order.
+        auto enlist = [&](unsigned set, unsigned from) {
+            for (; set; set &= set - 1)
+                list[from++] = static_cast<std::uint16_t>(lane * 32 + static_cast<unsigned>(__ffs(set) - 1));
+        };
+        if (__any_sync(0xffffffffU, bits != 0)) {
+            const unsigned n = __popc(bits), upto = warpInclusive(n);
+            const unsigned count = __shfl_sync(0xffffffffU, upto, 31);
+            enlist(bits, upto - n);
+            if (bits) L.ev_bits[wd] = 0; // the end sample sets bits with atomicOr
+            __syncwarp();
+            for (unsigned e = lane; e < count; e += 32) energy[e] = L.ev_removed[tile * kThreads + list[e]];
+            __syncwarp();
+            double own = 0.0;
+            for (unsigned e = upto - n; e < upto; ++e) own += energy[e];
+            double run = __shfl_up_sync(0xffffffffU, warpInclusive(own), 1);
+            if (lane == 0) run = 0.0;
+            __syncwarp();
+            for (unsigned e = upto - n; e < upto; ++e) {
+                run += energy[e];
+                energy[e] = run;
             }
+            __syncwarp();
+            const unsigned at = L.blk_ev[blk] + L.ev_tile[tile];
+            const double offset = L.blk_removed[blk] + L.tile_removed[tile];
+            bool gain = false;
+            for (unsigned e = lane; e < count; e += 32) {
+                const std::uint32_t j = tile * kThreads + list[e];
+                if (!inBounds(j, L.B, kSiteEvent)) continue;
+                const double removed = L.ev_removed[j], running = prior + (offset + energy[e]);
+                gain = gain || removed > fraction * (running < 1.0e-12 ? 1.0e-12 : running);
+                if (first_round) L.ffb[at + e] = j;
+                const uint2 e2 = L.ev_ends[j];
+                const std::uint32_t ends[2] = {e2.x, e2.y};
+                for (int q = 0; q < 2; ++q) {
+                    const std::uint32_t node = ends[q];
+                    if (!inBounds(node, L.N, kSiteEventEnd)) continue;
+                    unsigned *word = reinterpret_cast<unsigned *>(L.dirty + (node & ~3U));
+                    const unsigned bit = 1U << (8 * (node & 3U));
+                    if (!(atomicOr(word, bit) & bit)) {
+                        const unsigned slot = atomicAdd(&c.dirty_count, 1U);
+                        if (inBounds(slot, L.N, kSiteDirty)) L.dirty_list[slot] = node;
+                    }
+                }
+            }
+            if (__any_sync(0xffffffffU, gain) && lane == 0) atomicOr(&c.energy_gain, 1U);
+            __syncwarp();
+        }
+        if (__any_sync(0xffffffffU, dbits != 0)) {
+            const unsigned n = __popc(dbits), upto = warpInclusive(n);
+            const unsigned count = __shfl_sync(0xffffffffU, upto, 31);
+            enlist(dbits, upto - n);
+            if (dbits) L.dmg_bits[wd] = 0;
+            __syncwarp();
+            const unsigned at = L.blk_dmg[blk] + L.dmg_tile[tile];
+            for (unsigned e = lane; e < count; e += 32) L.dmg_value[at + e] = L.ev_damage[tile * kThreads + list[e]];
+            __syncwarp();
         }
     }
 }
