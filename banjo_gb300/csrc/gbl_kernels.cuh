@@ -2507,18 +2507,40 @@ __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> laun
 }
 
 // ---------------------------------------------------------------------------
-// The serial tail of a substep, one thread: the substep's FP64 sums into the
-// run totals, the damage-record scan over its (few) candidates in bond order,
+// The serial tail of a substep, one warp: the damage-record scan over its
+// candidates in bond order; then one thread: the substep's FP64 sums into the
+// run totals,
 // the sphere drift and support contact, the failure-round bookkeeping and the
 // exit rules (CpuLatticeBackend.cpp:279-298, 441-488), after the load ledger.
 // ---------------------------------------------------------------------------
 template <class R, bool Many>
-__global__ void kLedger(const Grid<R> launch, Settings<R> S) {
+__global__ void __launch_bounds__(32) kLedger(const Grid<R> launch, Settings<R> S) {
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
-    if (threadIdx.x != 0) return;
     Ctl &c = *L.ctl;
     if (c.stop) return;
+    // The damage record over its candidates in bond order: the warp looks for
+    // the next one above the record as it stands, 32 at a time (a candidate
+    // rarely is: the record only grows). One thread reading them one after
+    // another took 162 us of a substep of 128 shattering trials.
+    double record = c.max_damage;
+    bool gained = false;
+    if (!c.error) {
+        const unsigned n = c.dmg_count;
+        for (unsigned base = 0; base < n; base += 32) {
+            const unsigned e = base + threadIdx.x;
+            const double dmg = e < n ? static_cast<double>(L.dmg_value[e]) : -1.0;
+            for (unsigned from = 0; from < 32;) {
+                const unsigned above = __ballot_sync(0xffffffffU, threadIdx.x >= from && dmg > record + 1.0e-6);
+                if (!above) break;
+                const unsigned at = static_cast<unsigned>(__ffs(above) - 1);
+                record = __shfl_sync(0xffffffffU, dmg, static_cast<int>(at));
+                gained = true;
+                from = at + 1;
+            }
+        }
+    }
+    if (threadIdx.x != 0) return;
     if (c.error) {
         c.stop = 1;
         atomicSub(L.running, 1U);
@@ -2528,12 +2550,9 @@ __global__ void kLedger(const Grid<R> launch, Settings<R> S) {
     if (c.ext_count && c.loads_remaining > 0) c.loads_remaining -= 1; // the substep's load, folded by kLoadLedger
     c.full_restart = 0;
     c.plastic_work += c.plastic_substep;
-    for (unsigned e = 0; e < c.dmg_count; ++e) {
-        const float dmg = L.dmg_value[e];
-        if (static_cast<double>(dmg) > c.max_damage + 1.0e-6) {
-            c.max_damage = dmg;
-            c.last_damage_gain_step = step;
-        }
+    if (gained) {
+        c.max_damage = record;
+        c.last_damage_gain_step = step;
     }
     const unsigned broken = c.event_count;
     c.projections += (c.live_bonds - c.broken_bonds) * S.iterations;
