@@ -2441,24 +2441,28 @@ private:
         const bool side_restart = S.sphere_enabled != 0;
         if (!side_restart) restartPhase<M>(st, 0, mark);
         if (M) {
-            if (wrench_.count) kWrenchMany<R><<<wrench_.count, kWrenchThreads, 0, st>>>(grid(wrench_));
+            if (wrench_.count) next(kWrenchMany<R>, wrench_.count, kWrenchThreads, 0, st, grid(wrench_));
         } else {
             for (auto k : active_) {
                 const Resident<R> &l = *slots_[k];
                 if (l.wrench_cap)
-                    kWrench<R><<<l.wrench_cap, kWrenchThreads, 0, st>>>(l.dev, l.dev.wrench, l.dev.ext_nodes, nullptr,
-                                                                       1);
+                    next(kWrench<R>, l.wrench_cap, kWrenchThreads, 0, st, l.dev, l.dev.wrench, l.dev.ext_nodes, nullptr, 1);
             }
         }
-        if (nodes_.count) kKick<R, M><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), S);
-        // The load ledger, on its own stream until the serial tail.
-        check(cudaEventRecord(load_fork_, st), "event");
-        check(cudaStreamWaitEvent(loads_, load_fork_, 0), "stream wait");
-        kLoadLedger<R, M><<<dim3(each_.count, kLedgerFolds), kLedgerThreads, 0, loads_>>>(grid(each_), S);
-        check(cudaEventRecord(load_join_, loads_), "event");
+        if (nodes_.count) next(kKick<R, M>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
+        // The load ledger, on its own stream until the serial tail, when any
+        // lattice has had a load (the graph is rebuilt at its first one).
+        bool loads = false;
+        for (auto k : active_) loads = loads || slots_[k]->ext_force;
+        if (loads) {
+            check(cudaEventRecord(load_fork_, st), "event");
+            check(cudaStreamWaitEvent(loads_, load_fork_, 0), "stream wait");
+            next(kLoadLedger<R, M>, dim3(each_.count, kLedgerFolds), kLedgerThreads, 0, loads_, grid(each_), S);
+            check(cudaEventRecord(load_join_, loads_), "event");
+        }
         if (S.sphere_enabled && slabs_.count) {
-            kCandidates<R, M><<<slabs_.count, 1024, 0, st>>>(grid(slabs_));
-            kMarkHalo<R, M><<<dim3(slabs_.count, kHaloParts), 1024, 0, st>>>(grid(slabs_));
+            next(kCandidates<R, M>, slabs_.count, 1024, 0, st, grid(slabs_));
+            next(kMarkHalo<R, M>, dim3(slabs_.count, kHaloParts), 1024, 0, st, grid(slabs_));
         }
         mark(3);
         if (side_restart) {
@@ -2467,22 +2471,21 @@ private:
             restartPhase<M>(side_, 1);
             check(cudaEventRecord(join_, side_), "event");
             if (S.audit) audit<M>(st, kAuditMark);
-            kSpherePass<R, M><<<each_.count, kSphereThreads, sphere_buffers_ * kSphereSlab, st>>>(grid(each_), S, 1,
-                                                                                               sphere_buffers_);
+            next(kSpherePass<R, M>, each_.count, kSphereThreads, sphere_buffers_ * kSphereSlab, st, grid(each_), S, 1, sphere_buffers_);
             if (S.audit) audit<M>(st, kAuditStriker);
             check(cudaStreamWaitEvent(st, join_, 0), "stream wait");
         }
         mark(4);
         enqueueSweep<M>(mark);
         if (nodes_.count)
-            kVelocity<R, M><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), S, S.damping_fraction <= R(0) ? 1 : 0);
+            next(kVelocity<R, M>, nodes_.count, kThreads, 0, st, grid(nodes_), S, S.damping_fraction <= R(0) ? 1 : 0);
         mark(8);
         if (S.damping_fraction > R(0)) {
             if (S.audit) audit<M>(st, kAuditMark);
             for (const Span &lv : damp_)
-                if (lv.count) kDamp<R, M, kDirect><<<lv.count, kThreads, 0, st>>>(grid(lv), S.damping_fraction);
+                if (lv.count) next(kDamp<R, M, kDirect>, lv.count, kThreads, 0, st, grid(lv), S.damping_fraction);
             if (S.audit) audit<M>(st, kAuditDamping);
-            if (nodes_.count) kSupportVelocity<R, M><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), S);
+            if (nodes_.count) next(kSupportVelocity<R, M>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
             mark(9);
         }
         // With a sphere, the strain and end sample outside the contact halo
@@ -2499,21 +2502,20 @@ private:
         }
         if (S.sphere_enabled) {
             if (S.audit) audit<M>(st, kAuditMark);
-            kSpherePass<R, M><<<each_.count, kSphereThreads, sphere_buffers_ * kSphereSlab, st>>>(grid(each_), S, 2,
-                                                                                               sphere_buffers_);
+            next(kSpherePass<R, M>, each_.count, kSphereThreads, sphere_buffers_ * kSphereSlab, st, grid(each_), S, 2, sphere_buffers_);
             if (S.audit) audit<M>(st, kAuditStriker);
         }
         mark(10);
         if (split) check(cudaStreamWaitEvent(st, join_, 0), "stream wait");
         if (contact) contactPhase<M>(st, mark);
         endPhase<M>(st, split ? 2 : 0, mark);
-        if (tiles_.count) kTileCounts<R, M><<<tiles_.count, kThreads, 0, st>>>(grid(tiles_));
-        kEventScan<R, M><<<blocks_.count, kScanBlock, 0, st>>>(grid(blocks_), plastic_ ? 1 : 0);
-        if (several_blocks_) kTopScan<R, M><<<each_.count, kScanBlock, 0, st>>>(grid(each_));
-        if (tiles_.count) kEmitEvents<R, M><<<tiles_.count, kEmitThreads, 0, st>>>(grid(tiles_));
+        if (tiles_.count) next(kTileCounts<R, M>, tiles_.count, kThreads, 0, st, grid(tiles_));
+        next(kEventScan<R, M>, blocks_.count, kScanBlock, 0, st, grid(blocks_), plastic_ ? 1 : 0);
+        if (several_blocks_) next(kTopScan<R, M>, each_.count, kScanBlock, 0, st, grid(each_));
+        if (tiles_.count) next(kEmitEvents<R, M>, tiles_.count, kEmitThreads, 0, st, grid(tiles_));
         mark(12);
-        check(cudaStreamWaitEvent(st, load_join_, 0), "stream wait");
-        kLedger<R, M><<<each_.count, 32, 0, st>>>(grid(each_), S);
+        if (loads) check(cudaStreamWaitEvent(st, load_join_, 0), "stream wait");
+        next(kLedger<R, M>, each_.count, 32, 0, st, grid(each_), S);
         mark(13);
         check(cudaGetLastError(), "kernel launch");
     }
@@ -2521,7 +2523,7 @@ private:
     // The energy audit (CpuLatticeBackend.cpp:388-422): every lattice's
     // kinetic energy folded in node order, before a phase or after it.
     template <bool M> void audit(cudaStream_t st, int mode) {
-        kKineticFold<R, M><<<each_.count, kFoldThreads, 0, st>>>(grid(each_), mode);
+        next(kKineticFold<R, M>, each_.count, kFoldThreads, 0, st, grid(each_), mode);
     }
 
     // The projection sweep: the small lattices of a batch sweep whole, one
@@ -2551,13 +2553,29 @@ private:
                 for (const Span &lv : g.levels) launchSolve<M>(lv, first, last, g.levels.size() >= 2);
                 mark(5);
                 if (S.plane_count && g.isolated.count)
-                    kSupportIsolated<R, M><<<g.isolated.count, kThreads, 0, st>>>(grid(g.isolated), S);
+                    next(kSupportIsolated<R, M>, g.isolated.count, kThreads, 0, st, grid(g.isolated), S);
                 mark(7);
             }
         if (whole) {
             check(cudaStreamWaitEvent(st, join_, 0), "stream wait");
             mark(5);
         }
+    }
+
+    // A launch of the substep's chain (startAfterPrevious).
+    template <class... P, class... A>
+    void next(void (*kernel)(P...), dim3 blocks, unsigned threads, std::size_t smem, cudaStream_t st, A &&...args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = blocks;
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        check(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...), "kernel launch");
     }
 
     // A launch that may start while the previous kernel of the stream still
@@ -2597,10 +2615,10 @@ private:
         const int key = (plastic_ ? 2 : 0) | (support ? 1 : 0);
         const Grid<R> g = grid(span);
         switch (key) {
-        case 0: kSweepLattice<R, kDirect, false, false, T><<<span.count, T, 0, st>>>(g, S_); break;
-        case 1: kSweepLattice<R, kDirect, false, true, T><<<span.count, T, 0, st>>>(g, S_); break;
-        case 2: kSweepLattice<R, kDirect, true, false, T><<<span.count, T, 0, st>>>(g, S_); break;
-        default: kSweepLattice<R, kDirect, true, true, T><<<span.count, T, 0, st>>>(g, S_); break;
+        case 0: next(kSweepLattice<R, kDirect, false, false, T>, span.count, T, 0, st, g, S_); break;
+        case 1: next(kSweepLattice<R, kDirect, false, true, T>, span.count, T, 0, st, g, S_); break;
+        case 2: next(kSweepLattice<R, kDirect, true, false, T>, span.count, T, 0, st, g, S_); break;
+        default: next(kSweepLattice<R, kDirect, true, true, T>, span.count, T, 0, st, g, S_); break;
         }
     }
 
@@ -2610,10 +2628,10 @@ private:
             const int key = (plastic_ ? 2 : 0) | (S_.plane_count ? 1 : 0);
             const Grid<R> g = grid(span);
             switch (key) {
-            case 0: kSweepStaged<false, false><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
-            case 1: kSweepStaged<false, true><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
-            case 2: kSweepStaged<true, false><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
-            default: kSweepStaged<true, true><<<span.count, staged_threads_, staged_smem_, st>>>(g, S_); break;
+            case 0: next(kSweepStaged<false, false>, span.count, staged_threads_, staged_smem_, st, g, S_); break;
+            case 1: next(kSweepStaged<false, true>, span.count, staged_threads_, staged_smem_, st, g, S_); break;
+            case 2: next(kSweepStaged<true, false>, span.count, staged_threads_, staged_smem_, st, g, S_); break;
+            default: next(kSweepStaged<true, true>, span.count, staged_threads_, staged_smem_, st, g, S_); break;
             }
         }
     }
@@ -2640,17 +2658,17 @@ private:
     // kernel of it returns at once when no rebuild is due), the narrow phase.
     template <bool M, class Mark> void contactPhase(cudaStream_t st, Mark &&mark) {
         const Settings<R> &S = S_;
-        if (nodes_.count) kContactStale<R, M><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), S);
-        if (buckets_.count) kContactClear<R, M><<<buckets_.count, kThreads, 0, st>>>(grid(buckets_));
-        if (nodes_.count) kContactCells<R, M><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), S);
-        if (buckets_.count) kContactBuckets<R, M><<<buckets_.count, kThreads, 0, st>>>(grid(buckets_));
-        if (nodes_.count) kContactScatter<R, M><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_));
-        if (buckets_.count) kContactSort<R, M><<<buckets_.count, kThreads, 0, st>>>(grid(buckets_));
-        if (nodes_.count) kContactGather<R, M, false><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), S);
-        kContactTiles<R, M><<<each_.count, kContactScanThreads, 0, st>>>(grid(each_));
-        if (nodes_.count) kContactGather<R, M, true><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), S);
+        if (nodes_.count) next(kContactStale<R, M>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
+        if (buckets_.count) next(kContactClear<R, M>, buckets_.count, kThreads, 0, st, grid(buckets_));
+        if (nodes_.count) next(kContactCells<R, M>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
+        if (buckets_.count) next(kContactBuckets<R, M>, buckets_.count, kThreads, 0, st, grid(buckets_));
+        if (nodes_.count) next(kContactScatter<R, M>, nodes_.count, kThreads, 0, st, grid(nodes_));
+        if (buckets_.count) next(kContactSort<R, M>, buckets_.count, kThreads, 0, st, grid(buckets_));
+        if (nodes_.count) next(kContactGather<R, M, false>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
+        next(kContactTiles<R, M>, each_.count, kContactScanThreads, 0, st, grid(each_));
+        if (nodes_.count) next(kContactGather<R, M, true>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
         mark(14);
-        kContactNarrow<R, M><<<each_.count, 32, 0, st>>>(grid(each_), S);
+        next(kContactNarrow<R, M>, each_.count, 32, 0, st, grid(each_), S);
         mark(15);
     }
 
@@ -2661,14 +2679,12 @@ private:
         if (nodes_.count) {
             const R plate = S_.plate_half_thickness, yield = S_.yield_stretch;
             if (plate > R(0))
-                kRestartStrain<R, M, kDirect, true><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), after_kick, plate,
-                                                                                       yield);
+                next(kRestartStrain<R, M, kDirect, true>, nodes_.count, kThreads, 0, st, grid(nodes_), after_kick, plate, yield);
             else
-                kRestartStrain<R, M, kDirect, false><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), after_kick,
-                                                                                        plate, yield);
+                next(kRestartStrain<R, M, kDirect, false>, nodes_.count, kThreads, 0, st, grid(nodes_), after_kick, plate, yield);
         }
         mark(1);
-        if (bonds_.count) kRestartBonds<R, M, kDirect><<<bonds_.count, kThreads, 0, st>>>(grid(bonds_), after_kick);
+        if (bonds_.count) next(kRestartBonds<R, M, kDirect>, bonds_.count, kThreads, 0, st, grid(bonds_), after_kick);
         mark(2);
     }
 
@@ -2679,14 +2695,14 @@ private:
         if (nodes_.count) {
             const R plate = S_.plate_half_thickness, yield = S_.yield_stretch;
             if (plate > R(0))
-                kStrainAll<R, M, kDirect, true><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), part, plate, yield);
+                next(kStrainAll<R, M, kDirect, true>, nodes_.count, kThreads, 0, st, grid(nodes_), part, plate, yield);
             else
-                kStrainAll<R, M, kDirect, false><<<nodes_.count, kThreads, 0, st>>>(grid(nodes_), part, plate, yield);
+                next(kStrainAll<R, M, kDirect, false>, nodes_.count, kThreads, 0, st, grid(nodes_), part, plate, yield);
         }
         mark(11);
         if (bonds_.count) {
-            if (plastic_) kEndSample<R, M, kDirect, true><<<bonds_.count, kThreads, 0, st>>>(grid(bonds_), S_, part);
-            else kEndSample<R, M, kDirect, false><<<bonds_.count, kThreads, 0, st>>>(grid(bonds_), S_, part);
+            if (plastic_) next(kEndSample<R, M, kDirect, true>, bonds_.count, kThreads, 0, st, grid(bonds_), S_, part);
+            else next(kEndSample<R, M, kDirect, false>, bonds_.count, kThreads, 0, st, grid(bonds_), S_, part);
         }
     }
 

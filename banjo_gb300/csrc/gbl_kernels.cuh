@@ -234,6 +234,19 @@ template <class R> struct Dev {
 
 constexpr int kThreads = 256;
 
+// Programmatic dependent launch (sm_90+): the kernels of a substep are launched
+// while the one before still runs, so that launch latency and CTA start-up
+// (1 to 1.5 us, most of what the small ones take) overlap it. Each waits for
+// the previous grid to finish, its writes visible, before it touches anything
+// an earlier kernel writes, and lets the next one launch only after its own
+// wait: at most two overlap, and all before the previous one is complete.
+__device__ __forceinline__ void waitPreviousGrid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allowNextGrid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void startAfterPrevious() {
+    waitPreviousGrid();
+    allowNextGrid();
+}
+
 // One CTA's share of a launch: a range of one lattice's nodes, bonds, tiles or
 // scan blocks (what the range indexes is the kernel's).
 struct Work {
@@ -488,6 +501,7 @@ template <class R> __device__ __forceinline__ std::uint32_t substepStamp(const D
 
 template <class R, bool Many, bool Direct, bool Plate>
 __global__ void __launch_bounds__(kThreads) kStrainAll(const Grid<R> launch, int part, R plate, R yield) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
@@ -510,6 +524,7 @@ __global__ void __launch_bounds__(kThreads) kStrainAll(const Grid<R> launch, int
 // it (beside the first contact pass) from u_prev, where the kick copied them.
 template <class R, bool Many, bool Direct, bool Plate>
 __global__ void __launch_bounds__(kThreads) kRestartStrain(const Grid<R> launch, int after_kick, R plate, R yield) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     Dev<R> L = descriptor<R, Many>(launch, w);
     if (after_kick) L.u = L.up; // the kick kept the substep's starting positions there
@@ -589,6 +604,7 @@ __device__ __forceinline__ void startSample(const Dev<R> &L, std::uint32_t j) {
 // us a substep in the 32x8x8 beam, now 8; 100 in the 128x32x32 bar, now 11.)
 template <class R, bool Many, bool Direct>
 __global__ void __launch_bounds__(kThreads) kRestartBonds(const Grid<R> launch, int after_kick) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     Dev<R> L = descriptor<R, Many>(launch, w);
     if (after_kick) L.u = L.up;
@@ -627,6 +643,7 @@ __device__ __forceinline__ bool sphereCandidate(const Settings<R> &S, const Sphe
 
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kKick(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
@@ -883,12 +900,14 @@ __device__ __forceinline__ void wrenchSpread(const Dev<R> &L, const WrenchDev *w
 template <class R>
 __global__ void __launch_bounds__(kWrenchThreads)
 kWrench(const Dev<R> L, const WrenchDev *ws, const std::uint32_t *lists, unsigned *verdict, int apply) {
+    startAfterPrevious();
     wrenchSpread(L, ws, lists, verdict, apply, blockIdx.x);
 }
 
 // A batch's wrenches in one launch: one CTA per (lattice, wrench) item.
 template <class R>
 __global__ void __launch_bounds__(kWrenchThreads) kWrenchMany(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = launch.list[blockIdx.x];
     const Dev<R> &L = launch.table[w.lattice];
     wrenchSpread(L, L.wrench, L.ext_nodes, nullptr, 1, w.begin);
@@ -898,6 +917,7 @@ __global__ void __launch_bounds__(kWrenchThreads) kWrenchMany(const Grid<R> laun
 // one CTA per slab scans its bit words in node order.
 template <class R, bool Many>
 __global__ void __launch_bounds__(1024) kCandidates(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop) return;
@@ -966,6 +986,7 @@ __global__ void __launch_bounds__(1024) kCandidates(const Grid<R> launch) {
 constexpr unsigned kHaloParts = 9;
 template <class R, bool Many>
 __global__ void __launch_bounds__(1024) kMarkHalo(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop) return;
@@ -1137,6 +1158,7 @@ constexpr unsigned kSphereThreads = 256;
 template <class R, bool Many>
 __global__ void __launch_bounds__(kSphereThreads) kSpherePass(const Grid<R> launch, Settings<R> S, int pass,
                                                               unsigned buffers) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     extern __shared__ __align__(16) unsigned char sphere_smem[];
@@ -1429,16 +1451,10 @@ __device__ __forceinline__ bool supportProject(const Dev<R> &L, const Settings<R
 #endif
 constexpr int kSolvePer = GBL_SOLVE_PER;
 
-// Programmatic dependent launch (sm_90+): a sweep level is launched while the
-// previous one still runs; its CTAs load what no earlier kernel of the substep
-// writes (records, geometry, multipliers, plastic extension, the stop flag),
-// then wait for the previous grid to finish and its writes to be visible
-// before they touch the nodes. A level lets the next one launch only after its
-// own wait, so at most two levels overlap and everything before the previous
-// level is complete when a level starts.
-__device__ __forceinline__ void waitPreviousGrid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void allowNextGrid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
+// A sweep level (programmatic dependent launch, startAfterPrevious) loads what
+// no earlier kernel of the substep writes -- records, geometry, multipliers,
+// plastic extension, the stop flag -- before it waits for the previous grid;
+// at most two levels overlap.
 // The projection of one live bond (LatticePhysics.hpp:1132-1168): its unit
 // direction and the multiplier's change, with the reference's expressions.
 // Returns whether the nodes move (a degenerate bond leaves them).
@@ -1634,6 +1650,7 @@ __device__ __forceinline__ void supportIsolatedInCta(const Dev<R> &L, const Sett
 
 template <class R, bool Direct, bool Plastic, bool Support, unsigned T>
 __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 2) kSweepLattice(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     // The lattice's descriptor, copied once into shared memory: its fields
     // are read throughout the sweep, and shared memory is never written by
     // the sweep's global stores, so the compiler may keep them as it likes.
@@ -1754,6 +1771,7 @@ kSweepStaged(const __grid_constant__ Grid<float> launch, const __grid_constant__
         for (unsigned k = t; k < sizeof(Dev<float>) / sizeof(unsigned); k += T) dst[k] = src[k];
         __syncthreads();
     }
+    startAfterPrevious();
     const Dev<float> &L = *reinterpret_cast<const Dev<float> *>(desc.bytes);
     if (L.ctl->stop) return;
     const std::uint32_t N = L.N, levels = L.level_count, I = S.iterations;
@@ -1830,6 +1848,7 @@ kSweepStaged(const __grid_constant__ Grid<float> launch, const __grid_constant__
 // Radial pair damping of one level (LatticePhysics.hpp:1170-1184).
 template <class R, bool Many, bool Direct>
 __global__ void __launch_bounds__(kThreads) kDamp(const Grid<R> launch, R fraction) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop) return;
@@ -1857,6 +1876,7 @@ __global__ void __launch_bounds__(kThreads) kDamp(const Grid<R> launch, R fracti
 // nodes), after a sweep (LatticePhysics.hpp:1255-1261).
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kSupportIsolated(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop) return;
@@ -1875,6 +1895,7 @@ __global__ void __launch_bounds__(kThreads) kSupportIsolated(const Grid<R> launc
 // non-candidates when no damping sweep follows (LatticePhysics.hpp:1725-1730).
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kVelocity(const Grid<R> launch, Settings<R> S, int respond) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
@@ -1892,6 +1913,7 @@ __global__ void __launch_bounds__(kThreads) kVelocity(const Grid<R> launch, Sett
 // Support response of non-candidates after the damping sweep (CpuLatticeBackend.cpp:414-415).
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kSupportVelocity(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop) return;
@@ -1924,6 +1946,7 @@ __device__ __forceinline__ double warpSumFixed(double x) {
 
 template <class R, bool Many, bool Direct, bool Plastic>
 __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Settings<R> S, int part) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
@@ -2161,6 +2184,7 @@ __device__ __forceinline__ void ledgerTotals(Ctl &c, const LedgerScan &total) {
 constexpr unsigned kCountTiles = kThreads / kTileWords; // tiles per CTA
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kTileCounts(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
@@ -2188,6 +2212,7 @@ __global__ void __launch_bounds__(kThreads) kTileCounts(const Grid<R> launch) {
 // of one block (up to 262,143 bonds) is done; kTopScan follows for the others.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kScanBlock) kEventScan(const Grid<R> launch, int plastic) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
@@ -2224,6 +2249,7 @@ __global__ void __launch_bounds__(kScanBlock) kEventScan(const Grid<R> launch, i
 // 1024 blocks with a carry), and the substep's totals.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kScanBlock) kTopScan(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
@@ -2263,6 +2289,7 @@ constexpr unsigned kEmitTiles = 8;
 constexpr unsigned kEmitThreads = 128;
 template <class R, bool Many>
 __global__ void __launch_bounds__(kEmitThreads) kEmitEvents(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     __shared__ SharedDesc<R> desc;
     __shared__ std::uint16_t lists[kEmitThreads / 32][kThreads];
@@ -2358,6 +2385,7 @@ constexpr int kAuditMark = 0, kAuditStriker = 1, kAuditDamping = 2;
 
 template <class R, bool Many>
 __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launch, int mode) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     Ctl &c = *L.ctl;
@@ -2426,6 +2454,7 @@ __device__ __forceinline__ void addLoadComponent(LoadLedger &g, int q, double x)
 // on thirteen lanes of one warp).
 template <class R, bool Many>
 __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     Ctl &c = *L.ctl;
@@ -2509,12 +2538,13 @@ __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> laun
 // ---------------------------------------------------------------------------
 // The serial tail of a substep, one warp: the damage-record scan over its
 // candidates in bond order; then one thread: the substep's FP64 sums into the
-// run totals,
-// the sphere drift and support contact, the failure-round bookkeeping and the
-// exit rules (CpuLatticeBackend.cpp:279-298, 441-488), after the load ledger.
+// run totals, the sphere drift and support contact, the failure-round
+// bookkeeping and the exit rules (CpuLatticeBackend.cpp:279-298, 441-488),
+// after the load ledger.
 // ---------------------------------------------------------------------------
 template <class R, bool Many>
 __global__ void __launch_bounds__(32) kLedger(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     Ctl &c = *L.ctl;
@@ -2619,6 +2649,7 @@ template <class R> __device__ __forceinline__ R contactCutoff(const Settings<R> 
 // the list was built asks for a rebuild.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kContactStale(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     Ctl &c = *L.ctl;
@@ -2634,6 +2665,7 @@ __global__ void __launch_bounds__(kThreads) kContactStale(const Grid<R> launch, 
 // Rebuild, step 0 (bucket items): clear the bucket counts.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kContactClear(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     Ctl &c = *L.ctl;
@@ -2648,6 +2680,7 @@ __global__ void __launch_bounds__(kThreads) kContactClear(const Grid<R> launch) 
 // bucket counts of the movable nodes.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kContactCells(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop || !L.ctl->nc_rebuild) return;
@@ -2669,6 +2702,7 @@ __global__ void __launch_bounds__(kThreads) kContactCells(const Grid<R> launch, 
 // moves whole buckets. The count becomes the scatter cursor.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kContactBuckets(const Grid<R> launch) {
+    startAfterPrevious();
     __shared__ unsigned buf[kThreads];
     __shared__ unsigned base;
     const Work w = item<Many>(launch);
@@ -2690,6 +2724,7 @@ __global__ void __launch_bounds__(kThreads) kContactBuckets(const Grid<R> launch
 // Rebuild, step 3 (node items): the movable nodes into their buckets.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kContactScatter(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop || !L.ctl->nc_rebuild) return;
@@ -2703,6 +2738,7 @@ __global__ void __launch_bounds__(kThreads) kContactScatter(const Grid<R> launch
 // hold half a node on average; an insertion sort in place).
 template <class R, bool Many>
 __global__ void __launch_bounds__(kThreads) kContactSort(const Grid<R> launch) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     if (L.ctl->stop || !L.ctl->nc_rebuild) return;
@@ -2723,6 +2759,7 @@ __global__ void __launch_bounds__(kThreads) kContactSort(const Grid<R> launch) {
 // that did not fit. Write pass: the pairs at the owner's place in the list.
 template <class R, bool Many, bool Write>
 __global__ void __launch_bounds__(kThreads) kContactGather(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     __shared__ unsigned buf[kThreads];
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
@@ -2795,6 +2832,7 @@ __global__ void __launch_bounds__(kThreads) kContactGather(const Grid<R> launch,
 // and the list's length (nodeContactActiveList).
 template <class R, bool Many>
 __global__ void __launch_bounds__(kContactScanThreads) kContactTiles(const Grid<R> launch) {
+    startAfterPrevious();
     __shared__ unsigned buf[kContactScanThreads];
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
@@ -2823,6 +2861,7 @@ __global__ void __launch_bounds__(kContactScanThreads) kContactTiles(const Grid<
 // their tests and overlaps are counted as they are.
 template <class R, bool Many>
 __global__ void __launch_bounds__(32) kContactNarrow(const Grid<R> launch, Settings<R> S) {
+    startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
     Ctl &c = *L.ctl;
