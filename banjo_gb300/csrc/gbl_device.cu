@@ -582,6 +582,13 @@ template <class R> struct Resident {
         for (auto b : contactParts(n)) total += b;
         return total;
     }
+    // The sphere contact's candidate records (with a sphere in the settings).
+    static std::size_t sphereBytes(std::uint32_t blocks) {
+        return static_cast<std::size_t>(blocks) * kCandidatesPerBlock * sizeof(Staged<R>);
+    }
+    void ensureSphere() {
+        if (!dev.cand_stage) check(cudaMalloc(&dev.cand_stage, sphereBytes(sched.block_count)), "device allocation");
+    }
     void ensureContact() {
         if (nc_mem) return;
         const auto parts = contactParts(N);
@@ -613,6 +620,7 @@ template <class R> struct Resident {
         }
         if (flowed_dev_) cudaFree(flowed_dev_);
         if (nc_mem) cudaFree(nc_mem);
+        if (dev.cand_stage) cudaFree(dev.cand_stage);
         if (ext_force) cudaFree(ext_force);
         if (ext_req) cudaFree(ext_req);
         if (ext_contrib) cudaFree(ext_contrib);
@@ -1527,13 +1535,11 @@ template <class R> struct Resident {
 // work lists and the captured substep graph are rebuilt when the set changes.
 template <class R> class Engine {
     static constexpr bool kDirect = std::is_same<R, double>::value;
-    static constexpr unsigned kSphereSlab = sphereSlabBytes<R>();
+    static constexpr unsigned kSphereBytes = 2 * kSphereChunkBytes<R>;
 
 public:
     Engine() {
-        // Two staging buffers for the contact pass where the device's shared
-        // memory per block holds them, else one.
-        int device = 0, optin = 0;
+        int device = 0;
         check(cudaGetDevice(&device), "device");
         // Lattices are allocated from the device's pool, stream-ordered. Up to
         // 16 GiB that lattices free stays in the pool for the next upload or
@@ -1548,9 +1554,7 @@ public:
             std::uint64_t keep = std::uint64_t(16) << 30;
             check(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "memory pool");
         }
-        check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device), "device attribute");
-        sphere_buffers_ = 2U * kSphereSlab + 1024U <= static_cast<unsigned>(optin) ? 2U : 1U;
-        const int smem = static_cast<int>(sphere_buffers_ * kSphereSlab);
+        const int smem = static_cast<int>(kSphereBytes);
         check(cudaFuncSetAttribute(kSpherePass<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
               "contact pass shared memory");
         check(cudaFuncSetAttribute(kSpherePass<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
@@ -1651,6 +1655,7 @@ public:
                 dropGraph();
             }
             if (S_.nc_mode != 0) slots_[k]->ensureContact();
+            if (S_.sphere_enabled) slots_[k]->ensureSphere();
             initControl(k, step_limit);
             pushDescriptor(k);
             check(cudaStreamSynchronize(stream_), "admit");
@@ -1679,6 +1684,8 @@ public:
         for (auto k : active_) plastic_ = plastic_ || slots_[k]->plastic_state;
         if (S_.nc_mode != 0)
             for (auto k : active_) slots_[k]->ensureContact();
+        if (S_.sphere_enabled)
+            for (auto k : active_) slots_[k]->ensureSphere();
         growControl(slots_.size());
         for (auto k : active_) initControl(k, 0);
         for (auto k : active_) pushDescriptor(k);
@@ -1694,9 +1701,10 @@ public:
         S_ = convertSettings(set);
         plastic_ = S_.yield_stretch > R(0);
         for (auto k : active_) plastic_ = plastic_ || slots_[k]->plastic_state;
-        if (S_.nc_mode != 0) {
+        if (S_.nc_mode != 0 || S_.sphere_enabled) {
             for (auto k : active_) {
-                slots_[k]->ensureContact();
+                if (S_.nc_mode != 0) slots_[k]->ensureContact();
+                if (S_.sphere_enabled) slots_[k]->ensureSphere();
                 pushDescriptor(k);
             }
             check(cudaStreamSynchronize(stream_), "descriptors");
@@ -2466,12 +2474,13 @@ private:
         }
         mark(3);
         if (side_restart) {
+            if (S.audit) audit<M>(st, kAuditMark);
+            sphereStage<M>(st, 1);
             check(cudaEventRecord(fork_, st), "event");
+            spherePass<M>(st, 1);
             check(cudaStreamWaitEvent(side_, fork_, 0), "stream wait");
             restartPhase<M>(side_, 1);
             check(cudaEventRecord(join_, side_), "event");
-            if (S.audit) audit<M>(st, kAuditMark);
-            next(kSpherePass<R, M>, each_.count, kSphereThreads, sphere_buffers_ * kSphereSlab, st, grid(each_), S, 1, sphere_buffers_);
             if (S.audit) audit<M>(st, kAuditStriker);
             check(cudaStreamWaitEvent(st, join_, 0), "stream wait");
         }
@@ -2494,15 +2503,16 @@ private:
         // pass, so with it on the end phase waits for it whole.
         const bool contact = S.nc_mode != 0;
         const bool split = S.sphere_enabled != 0 && !contact;
-        if (split) {
-            check(cudaEventRecord(fork_, st), "event");
-            check(cudaStreamWaitEvent(side_, fork_, 0), "stream wait");
-            endPhase<M>(side_, 1);
-            check(cudaEventRecord(join_, side_), "event");
-        }
         if (S.sphere_enabled) {
             if (S.audit) audit<M>(st, kAuditMark);
-            next(kSpherePass<R, M>, each_.count, kSphereThreads, sphere_buffers_ * kSphereSlab, st, grid(each_), S, 2, sphere_buffers_);
+            sphereStage<M>(st, 2);
+            if (split) check(cudaEventRecord(fork_, st), "event");
+            spherePass<M>(st, 2);
+            if (split) {
+                check(cudaStreamWaitEvent(side_, fork_, 0), "stream wait");
+                endPhase<M>(side_, 1);
+                check(cudaEventRecord(join_, side_), "event");
+            }
             if (S.audit) audit<M>(st, kAuditStriker);
         }
         mark(10);
@@ -2518,6 +2528,17 @@ private:
         next(kLedger<R, M>, each_.count, 32, 0, st, grid(each_), S);
         mark(13);
         check(cudaGetLastError(), "kernel launch");
+    }
+
+    // A contact pass: the candidates' records, then the chain. The chain's CTA
+    // needs an SM to itself, so it is launched while the stage runs (its
+    // launch overlaps it) and the second stream's kernels only once the stage
+    // is done: they would fill every SM first.
+    template <bool M> void sphereStage(cudaStream_t st, int pass) {
+        if (slabs_.count) next(kSphereStage<R, M>, dim3(slabs_.count, kStageParts), kStageThreads, 0, st, grid(slabs_), S_, pass);
+    }
+    template <bool M> void spherePass(cudaStream_t st, int pass) {
+        next(kSpherePass<R, M>, each_.count, kSphereThreads<R>, kSphereBytes, st, grid(each_), S_, pass);
     }
 
     // The energy audit (CpuLatticeBackend.cpp:388-422): every lattice's
@@ -2574,7 +2595,7 @@ private:
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = st == side_ ? 0 : 1; // the second stream's wait for the whole of what it forks from
         check(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...), "kernel launch");
     }
 
@@ -2729,7 +2750,6 @@ private:
     std::mutex place_mutex_;
     Settings<R> S_{};
     bool plastic_{false}, ready_{false}, many_{false}, dirty_{true};
-    unsigned sphere_buffers_{1};
     std::uint32_t one_{0};
     Ctl *ctl_{};
     std::size_t cap_{0}, work_cap_{0};
@@ -2934,7 +2954,8 @@ public:
     static constexpr unsigned kSmall = 0, kLarge = 1;
 
     Server(const gbl_step_settings &settings, std::uint64_t budget)
-        : budget_(budget), contact_(settings.node_contact.mode != 0), t0_(clock()) {
+        : budget_(budget), contact_(settings.node_contact.mode != 0), sphere_(settings.sphere_enabled != 0),
+          t0_(clock()) {
         for (auto &lane : lanes_) lane.configure(settings);
     }
     ~Server() override {
@@ -2951,7 +2972,8 @@ public:
             invalid("lattice schedule does not match the lattice");
         const std::uint64_t bytes =
             Resident<R>::footprint(st.node_count, st.bond_count, st.max_degree, sv.block_count) +
-            (contact_ ? Resident<R>::contactBytes(st.node_count) : 0);
+            (contact_ ? Resident<R>::contactBytes(st.node_count) : 0) +
+            (sphere_ ? Resident<R>::sphereBytes(sv.block_count) : 0);
         if (bytes > budget_) invalid("request exceeds the device memory budget on its own");
         Request q;
         q.submitted = clock() - t0_;
@@ -3208,6 +3230,7 @@ private:
     std::atomic<std::uint32_t> large_bonds_{kLargeBonds};
     std::uint64_t budget_, used_{0}, last_ticket_{0};
     bool contact_; // node-to-node contact on: every request also holds its pair-list scratch
+    bool sphere_;  // a sphere: every request also holds its candidates' records
     std::uint64_t queued_{0}, running_{0}, done_{0}, substeps_run_{0};
     double device_seconds_{0}, admit_seconds_{0}, retire_seconds_{0}, run_seconds_{0};
     double t0_;

@@ -171,6 +171,7 @@ struct SourceSlot {
 constexpr unsigned kErrExternalOverflow = 1;
 constexpr unsigned kErrWrench = 2;
 
+template <class R> struct Staged;
 template <class R> struct Dev {
     std::uint32_t N, B, D, blocks, tiles_b;
     Q4<R> *u, *v, *x0, *up, *strain;
@@ -204,6 +205,7 @@ template <class R> struct Dev {
     std::uint32_t *blk_ev, *blk_dmg;   // per scan block of tiles: totals, then offsets
     double *blk_removed, *blk_plastic;
     std::uint32_t *node_block_begin, *cand_list, *cand_count, *dirty_list, *ffb;
+    Staged<R> *cand_stage; // the listed candidates' records, slab by slab (allocated when the settings have a sphere)
     // Contact halo of the substep (stamped with the substep's number + 1): the
     // listed sphere candidates and their neighbours, and the end-sample tiles
     // holding a bond at one of them. Everything outside it is final before the
@@ -1015,15 +1017,14 @@ __global__ void __launch_bounds__(1024) kMarkHalo(const Grid<R> launch) {
 // Sphere contact (LatticePhysics.hpp:1322-1428): candidates in slab, then node
 // order, one contact at a time -- every contact moves the sphere the next one
 // sees, so that chain is serial by definition. It runs on one warp of one
-// CTA per lattice; everything that does not depend on the sphere's changing
-// state is computed by the whole CTA around it.
+// CTA per lattice (kSpherePass); everything that does not depend on the
+// sphere's changing state is done before it, on every SM (kSphereStage).
 //
-// A candidate's node data are staged in shared memory. In pass 1 the sphere
-// centre cannot move (only pass 2 corrects positions), so the offset r, its
-// length and unit normal, the gap, the inverse masses and the effective
-// inverse mass along the normal are computed in parallel before the chain,
-// with the reference's expressions; the chain then starts at the relative
-// velocity. In pass 2 the parallel part is the node's position and masses.
+// A candidate's record: in pass 1 the sphere centre cannot move (only pass 2
+// corrects positions), so the offset r, its length and unit normal, the gap,
+// the inverse masses and the effective inverse mass along the normal are the
+// stage's, with the reference's expressions, and the chain starts at the
+// relative velocity. In pass 2 they are the node's position and masses.
 // ---------------------------------------------------------------------------
 template <class R> struct Staged {
     V3<R> p;       // position x0 + u (pass 2), or r = p - centre (pass 1)
@@ -1035,120 +1036,214 @@ template <class R> struct Staged {
     Q4<R> u, v;    // u (w: inv_mass), v (w: mass)
 };
 
-// What one hit adds to the contact ledger's FP64 sums, in backend precision:
-// the chain writes it to a log in shared memory and goes on, and the fold
-// lanes widen and add it in log order (LatticePhysics.hpp:1354-1381), so the
-// FP64 adds stay off the serial chain.
+// What one hit leaves: its candidate (for the write-back) and what it adds to
+// the contact ledger's FP64 sums, in backend precision. The chain writes it to
+// a log in shared memory and goes on, and the fold lanes widen and add it in
+// log order (LatticePhysics.hpp:1354-1381), so the FP64 adds stay off the
+// serial chain.
 template <class R> struct ContactLog {
     R normal_imp[3], friction_imp[3];
-    R lost;            // the node's kinetic energy before minus after
-    unsigned friction; // friction_imp applies
+    R lost;         // the node's kinetic energy before minus after
+    unsigned flags; // kLogFriction: friction_imp applies; kLogImpulse: the sums do; candidate << 8
 };
+constexpr unsigned kLogFriction = 1, kLogImpulse = 2;
 
-// Bytes of shared memory per staging buffer of the contact pass: a slab's
-// staged candidates and the log of its hits.
-template <class R> constexpr unsigned sphereSlabBytes() {
-    return kCandidatesPerBlock * static_cast<unsigned>(sizeof(Staged<R>) + sizeof(ContactLog<R>));
-}
+// Candidates a staging buffer of the contact pass holds, and its bytes: the
+// records of a chunk of a slab's candidates and the log of its hits. Two
+// buffers fit the shared memory a CTA may take.
+template <class R> constexpr unsigned kSphereChunk = sizeof(R) == 4 ? kCandidatesPerBlock : 480;
+template <class R>
+constexpr unsigned kSphereChunkBytes = kSphereChunk<R> * static_cast<unsigned>(sizeof(Staged<R>) + sizeof(ContactLog<R>));
 
 template <class R>
-__device__ __forceinline__ void contactApply(V3<R> imp, V3<R> r, R inm, R ism, R iin, V3<R> &nv, Sphere<R> &sp) {
+__device__ __forceinline__ void contactApply(V3<R> imp, V3<R> r, R inm, R ism, R iin, V3<R> &nv, V3<R> &sv, V3<R> &sw) {
     nv = nv + inm * imp;
-    sp.velocity = sp.velocity - ism * imp;
+    sv = sv - ism * imp;
     const V3<R> ti = -cross(r, imp);
-    sp.angular = sp.angular + iin * ti;
+    sw = sw + iin * ti;
 }
 
-// A candidate against the current sphere state: 0 outside the contact gate
-// (LatticePhysics.hpp:1338-1342; nothing happens), 1 a graze (past the gate,
-// but no normal impulse and no position correction: it only raises the
-// penetration record), 2 a hit (it changes the node and the sphere). The
-// normal relative velocity and the normal impulse come back for the hit.
-template <class R>
-__device__ __forceinline__ int contactProbe(const Settings<R> &S, const Sphere<R> &sp, V3<R> nv, V3<R> r,
-                                            V3<R> normal, R gap, R eff_n, bool correct, R &vn, R &ni) {
-    const V3<R> rel = nv - sp.velocity - cross(sp.angular, r);
-    vn = dot(rel, normal);
-    if (gap > maxR(S.c_margin, -vn * S.dt)) return 0;
+// A candidate's geometry against the sphere's centre.
+template <class R> struct ContactGeometry {
+    V3<R> r, normal;
+    R gap, eff_n; // |r| - (sphere radius + node contact radius); effective inverse mass along the normal
+};
+template <class R, class M>
+__device__ __forceinline__ ContactGeometry<R> contactGeometry(M &m, V3<R> r, R cr, R inm, R ism, R iin) {
+    ContactGeometry<R> g;
+    g.r = r;
+    const R sq = dot(r, r), distance = m.root(sq);
+    g.normal = distance > R(1.0e-12) ? m.div(r, distance) : mk<R>(1, 0, 0); // normalized(r)
+    const V3<R> rn = cross(r, g.normal);
+    g.eff_n = inm + ism + iin * dot(rn, rn);
+    g.gap = distance - cr;
+    return g;
+}
+
+// A candidate against the current sphere state, carried through as if it were
+// the next contact (LatticePhysics.hpp:1338-1386): 0 outside the contact gate
+// (nothing happens), 1 a graze (past the gate, but no normal impulse and no
+// position correction: it only raises the penetration record), 2 a hit, with
+// the node's and the sphere's velocities after it.
+template <class R> struct ContactTry {
+    int kind;
+    bool impulse;       // a normal impulse (else only a position correction)
+    V3<R> nv, sv, sw;   // the node's velocity, the sphere's velocities
+    ContactLog<R> log;
+};
+template <class R, class M>
+__device__ __forceinline__ ContactTry<R> contactTry(M &m, const Settings<R> &S, const Sphere<R> &sp, V3<R> nv,
+                                                    const ContactGeometry<R> &g, R mass, R inm, R before, R ism, R iin,
+                                                    bool correct) {
+    ContactTry<R> o;
+    const V3<R> rel = nv - sp.velocity - cross(sp.angular, g.r);
+    const R vn = dot(rel, g.normal);
+    const bool outside = g.gap > maxR(S.c_margin, -vn * S.dt);
     const R restitution = -vn > S.c_threshold ? S.c_restitution : R(0);
-    const R desired = gap > S.c_margin ? -gap / S.dt : -restitution * minR(vn, R(0));
-    ni = maxR(R(0), (desired - vn) / eff_n);
-    return (ni > R(0) || (correct && gap < -S.c_margin)) ? 2 : 1;
-}
-
-// The contact of one staged candidate past the gate, from its normal
-// relative velocity and normal impulse on (LatticePhysics.hpp:1343-1386).
-// `max_pen` and `max_corr` shadow acc.max_penetration and acc.max_correction
-// in R: the ledger only ever holds a widened R, so the comparisons are the
-// reference's. A hit's ledger sums go to `log`; it returns whether it hit.
-template <class R>
-__device__ __forceinline__ bool contactChain(const Settings<R> &S, Sphere<R> &sp, Staged<R> &c, V3<R> r, V3<R> normal,
-                                             R gap, R ni, R ism, R iin, bool correct, ContactAcc &acc, R &max_pen,
-                                             R &max_corr, ContactLog<R> &log) {
-    V3<R> nv = xyz(c.v);
-    if (-gap > max_pen) {
-        max_pen = -gap;
-        acc.max_penetration = static_cast<double>(-gap);
-    }
-    const R inm = c.inm;
-    const R mass = c.v.w;
-    const bool hit = ni > R(0);
-    if (hit) {
-        const V3<R> imp = ni * normal;
-        contactApply(imp, r, inm, ism, iin, nv, sp);
-        log.normal_imp[0] = imp.x;
-        log.normal_imp[1] = imp.y;
-        log.normal_imp[2] = imp.z;
-        log.friction = 0;
-        const V3<R> after = nv - sp.velocity - cross(sp.angular, r);
-        const V3<R> tangent = after - dot(after, normal) * normal;
-        const R ts = length(tangent);
+    const R desired = g.gap > S.c_margin ? m.div(-g.gap, S.dt) : -restitution * minR(vn, R(0));
+    const R ni = maxR(R(0), m.div(desired - vn, g.eff_n));
+    o.impulse = ni > R(0);
+    o.kind = outside ? 0 : (o.impulse || (correct && g.gap < -S.c_margin)) ? 2 : 1;
+    o.nv = nv;
+    o.sv = sp.velocity;
+    o.sw = sp.angular;
+    const V3<R> imp = ni * g.normal;
+    if (!(o.kind == 2 && o.impulse)) return o;
+    contactApply(imp, g.r, inm, ism, iin, o.nv, o.sv, o.sw);
+    o.log.normal_imp[0] = imp.x;
+    o.log.normal_imp[1] = imp.y;
+    o.log.normal_imp[2] = imp.z;
+    o.log.flags = kLogImpulse;
+    const V3<R> after = o.nv - o.sv - cross(o.sw, g.r);
+    const V3<R> tangent = after - dot(after, g.normal) * g.normal;
+    // A tangential speed of at most 1e-12 takes no friction; a square below
+    // 2^-80 is under it whatever its root's rounding.
+    const R sq = dot(tangent, tangent);
+    if (!(sq < R(0x1p-80))) {
+        const R ts = m.root(sq);
         if (ts > R(1.0e-12)) {
-            const V3<R> d = tangent / ts;
-            const V3<R> rd = cross(r, d);
-            const R stick = ts / (inm + ism + iin * dot(rd, rd));
+            const V3<R> d = m.div(tangent, ts);
+            const V3<R> rd = cross(g.r, d);
+            const R stick = m.div(ts, inm + ism + iin * dot(rd, rd));
             const R fi = stick <= S.c_static * ni ? stick : minR(stick, S.c_dynamic * ni);
             const V3<R> fimp = -fi * d;
-            contactApply(fimp, r, inm, ism, iin, nv, sp);
-            log.friction_imp[0] = fimp.x;
-            log.friction_imp[1] = fimp.y;
-            log.friction_imp[2] = fimp.z;
-            log.friction = 1;
-        }
-        c.v = Q4<R>{nv.x, nv.y, nv.z, mass};
-        log.lost = c.before - R(0.5) * mass * dot(nv, nv);
-        ++acc.impulse_contacts;
-    }
-    if (correct && gap < -S.c_margin) {
-        const R corr = minR(-gap - S.c_margin, R(0.2) * maxR(S.c_node_radius, sp.radius * R(0.01)));
-        const R sum = inm + ism;
-        const V3<R> ns = (corr * inm / sum) * normal;
-        const V3<R> ss = -((corr * ism / sum) * normal);
-        const V3<R> un = xyz(c.u) + ns;
-        c.u = Q4<R>{un.x, un.y, un.z, c.u.w};
-        sp.center = sp.center + ss;
-        if (corr > max_corr) {
-            max_corr = corr;
-            acc.max_correction = static_cast<double>(corr);
+            contactApply(fimp, g.r, inm, ism, iin, o.nv, o.sv, o.sw);
+            o.log.friction_imp[0] = fimp.x;
+            o.log.friction_imp[1] = fimp.y;
+            o.log.friction_imp[2] = fimp.z;
+            o.log.flags = kLogImpulse | kLogFriction;
         }
     }
-    return hit;
+    o.log.lost = before - R(0.5) * mass * dot(o.nv, o.nv);
+    return o;
 }
 
-constexpr unsigned kSphereThreads = 256;
-// Staging buffers of the contact pass: with two, the chain of one slab runs on
-// warp 0 while warp 1 folds the ledger log of the slab before it and the other
-// warps write back the slab before it from the other buffer and then stage
-// the slab after it into that buffer (a thread writes back and stages the
-// same buffer slots, so no barrier is needed between); with one (when two do
-// not fit the device's shared memory), one slab at a time.
+// The position correction of a deep hit (second pass): the node's new
+// displacement and the sphere centre's.
+template <class R>
+__device__ __forceinline__ R contactCorrect(const Settings<R> &S, const Sphere<R> &sp, const ContactGeometry<R> &g, R inm,
+                                            R ism, Q4<R> &u, V3<R> &center) {
+    const R corr = minR(-g.gap - S.c_margin, R(0.2) * maxR(S.c_node_radius, sp.radius * R(0.01)));
+    const R sum = inm + ism;
+    const V3<R> ns = (corr * inm / sum) * g.normal;
+    const V3<R> ss = -((corr * ism / sum) * g.normal);
+    const V3<R> un = xyz(u) + ns;
+    u = Q4<R>{un.x, un.y, un.z, u.w};
+    center = sp.center + ss;
+    return corr;
+}
 
-// The chain runs on warp 0, with every lane holding the same sphere state and
-// ledgers. Only a candidate that passes the contact gate changes anything, so
-// the lanes test the next 32 candidates against the current state at once; the
-// first that passes is applied (by every lane, identically) and the scan
-// resumes after it. The candidates skipped were tested against exactly the
-// state the serial order shows them, so the result is the serial chain's.
+// A candidate's node arrays after the pass: pass 1 predicts its position and
+// keeps its approach speeds, pass 2 gives it the support planes' response.
+template <class R>
+__device__ __forceinline__ void contactSettle(const Dev<R> &L, const Settings<R> &S, int pass, std::uint32_t i,
+                                              const Q4<R> &uq, const Q4<R> &vq) {
+    if (pass == 1) {
+        for (std::uint32_t p = 0; p < S.plane_count; ++p) L.approach[p * L.N + i] = dot(xyz(vq), S.planes[p].normal);
+        const V3<R> un = xyz(uq) + S.dt * xyz(vq);
+        L.u[i] = Q4<R>{un.x, un.y, un.z, uq.w};
+        L.v[i] = vq;
+    } else {
+        V3<R> vel = xyz(vq);
+        for (std::uint32_t p = 0; p < S.plane_count; ++p)
+            if (L.engaged[p * L.N + i]) vel = supportVelocity(S.planes[p], vel, L.approach[p * L.N + i]);
+        L.u[i] = uq;
+        L.v[i] = Q4<R>{vel.x, vel.y, vel.z, vq.w};
+    }
+}
+
+// The candidates of one slab, one CTA of the parts along y: their records, and
+// their node arrays as the pass leaves them if the chain does not touch them
+// (it rewrites the nodes it hits). The chain's CTA then only copies records,
+// where it used to gather and divide for them: in the double lane, whose
+// divisions one SM is slow at, a pass of 75 hits took 962 us, now 817.
+constexpr unsigned kStageThreads = 128;
+constexpr unsigned kStageParts = kCandidatesPerBlock / kStageThreads;
+template <class R, bool Many>
+__global__ void __launch_bounds__(kStageThreads) kSphereStage(const Grid<R> launch, Settings<R> S, int pass) {
+    startAfterPrevious();
+    const Work w = item<Many>(launch);
+    __shared__ SharedDesc<R> desc;
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
+    if (L.ctl->stop) return;
+    const std::uint32_t b = w.begin;
+    const std::uint32_t k = blockIdx.y * kStageThreads + threadIdx.x;
+    if (k >= L.cand_count[b]) return;
+    const std::uint32_t i = L.cand_list[b * kCandidatesPerBlock + k];
+    Staged<R> &out = L.cand_stage[b * kCandidatesPerBlock + k];
+    if (!inBounds(i, L.N, kSiteCandidate)) {
+        out = Staged<R>{}; // no mass: the chain passes it by
+        return;
+    }
+    const Sphere<R> sp = *L.sphere;
+    const R ism = R(1) / sp.mass, iin = R(1) / sp.inertia, cr = sp.radius + S.c_node_radius;
+    Staged<R> c;
+    c.u = L.u[i];
+    c.v = L.v[i];
+    const R mass = c.v.w;
+    const V3<R> p = xyz(L.x0[i]) + xyz(c.u);
+    c.inm = R(1) / mass;
+    c.before = R(0.5) * mass * dot(xyz(c.v), xyz(c.v));
+    if (pass == 1) {
+        const V3<R> r = p - sp.center;
+        const R distance = length(r);
+        const V3<R> normal = normalized(r);
+        const V3<R> rn = cross(r, normal);
+        c.p = r;
+        c.normal = normal;
+        c.gap = distance - cr;
+        c.eff_n = c.inm + ism + iin * dot(rn, rn);
+    } else {
+        c.p = p;
+        c.normal = V3<R>{};
+        c.gap = c.eff_n = R(0);
+    }
+    out = c;
+    contactSettle(L, S, pass, i, c.u, c.v);
+}
+
+// The CTA takes nearly all of an SM's registers, so no other kernel's CTAs come
+// to share the SM the chain runs on (with 256 threads the kernels beside it
+// did: 1,460 against 966 us).
+template <class R> constexpr unsigned kSphereThreads = sizeof(R) == 4 ? 512 : 320;
+// Two staging buffers: the chain of one chunk of candidates runs on warp 0 while
+// warp 1 folds the ledger log of the chunk before it and the other warps
+// write back that chunk's hits and then copy the next chunk's records into the
+// same buffer (after a barrier of their own and the fold's).
+
+// The chain runs on warp 0, with every lane holding the same sphere state.
+// Only a candidate that passes the contact gate changes anything. The lanes
+// hold the next 32 candidates in registers and each carries its own through
+// against the current state as if it were the next contact; the first lane
+// that hits has done the serial chain's next step, its sphere state goes to
+// every lane, and the lanes after it try again. The candidates before it were
+// tested against exactly the state the serial order shows them, so the result
+// is the serial chain's; the records (deepest penetration, largest
+// correction) are maxima, which any order forms alike. What a hit costs is its
+// own dependent arithmetic -- three divisions and a root, without branches in
+// the float lane -- a ballot and six shuffles. Both passes of a substep, with
+// what runs beside them: impact 256x128x128 (2,700 hits) 1,500 us, 1,902
+// before; 128x64x64 471 us, 572 before.
 // Slabs are disjoint sets of nodes: staging one slab's candidates, running
 // another's chain and writing back a third's touch different nodes.
 //
@@ -1156,248 +1251,193 @@ constexpr unsigned kSphereThreads = 256;
 // independent serial folds; lanes 0-3 of warp 1 run one each over the hit
 // logs, slab after slab, in the order the chain wrote them.
 template <class R, bool Many>
-__global__ void __launch_bounds__(kSphereThreads) kSpherePass(const Grid<R> launch, Settings<R> S, int pass,
-                                                              unsigned buffers) {
+__global__ void __launch_bounds__(kSphereThreads<R>) kSpherePass(const Grid<R> launch, Settings<R> S, int pass) {
     startAfterPrevious();
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
+    constexpr unsigned kChunk = kSphereChunk<R>;
     extern __shared__ __align__(16) unsigned char sphere_smem[];
     Staged<R> *stage_base = reinterpret_cast<Staged<R> *>(sphere_smem);
-    ContactLog<R> *log_base =
-        reinterpret_cast<ContactLog<R> *>(sphere_smem + buffers * kCandidatesPerBlock * sizeof(Staged<R>));
-    __shared__ Sphere<R> start;
+    ContactLog<R> *log_base = reinterpret_cast<ContactLog<R> *>(sphere_smem + 2 * kChunk * sizeof(Staged<R>));
     __shared__ unsigned log_count[2];
     __shared__ double folded[4];
     if (L.ctl->stop) return;
     const unsigned lane = threadIdx.x & 31U;
     const bool chain = threadIdx.x < 32;
     const bool fold = threadIdx.x >= 32 && threadIdx.x < 36;
-    Sphere<R> sp{};
+    Sphere<R> sp = *L.sphere;
+    const R ism = R(1) / sp.mass; // constant over the pass, as is the inertia
+    const R iin = R(1) / sp.inertia;
+    const R cr = sp.radius + S.c_node_radius;
     ContactAcc acc{};
     V3<R> c0{};
     R e0 = R(0), max_pen = R(0), max_corr = R(0);
     double sum = 0.0; // the fold lane's ledger sum
     if (chain) {
-        sp = *L.sphere;
         if (pass == 1) sp.velocity = sp.velocity + S.dt * S.gravity; // the kicked sphere becomes the state
         acc = L.ctl->contact;
         max_pen = R(acc.max_penetration);
         max_corr = R(acc.max_correction);
         c0 = sp.center;
         e0 = R(0.5) * sp.mass * dot(sp.velocity, sp.velocity) + R(0.5) * sp.inertia * dot(sp.angular, sp.angular);
-        if (threadIdx.x == 0) start = sp;
     } else if (fold) {
         const ContactAcc &a = L.ctl->contact;
         sum = lane == 0 ? a.impulse_x : lane == 1 ? a.impulse_y : lane == 2 ? a.impulse_z : a.dissipated;
     }
-    __syncthreads();
-    // Constant over the pass: the sphere's mass and inertia never change.
-    const R ism = R(1) / start.mass;
-    const R iin = R(1) / start.inertia;
-    const R cr = start.radius + S.c_node_radius;
 
-    // A slab's candidates into a buffer, by threads [t0, t0 + nt).
-    auto stageSlab = [&](std::uint32_t b, Staged<R> *st, unsigned t0, unsigned nt) {
-        const std::uint32_t n = L.cand_count[b];
-        const std::uint32_t *list = L.cand_list + b * kCandidatesPerBlock;
-        for (std::uint32_t k = threadIdx.x - t0; k < n; k += nt) {
-            const std::uint32_t i = list[k];
-            Staged<R> c;
-            if (!inBounds(i, L.N, kSiteCandidate)) {
-                c = Staged<R>{}; // no mass: the chain passes it by
-                st[k] = c;
-                continue;
-            }
-            c.u = L.u[i];
-            c.v = L.v[i];
-            const R mass = c.v.w;
-            const V3<R> p = xyz(L.x0[i]) + xyz(c.u);
-            c.inm = R(1) / mass;
-            c.before = R(0.5) * mass * dot(xyz(c.v), xyz(c.v));
-            if (pass == 1) {
-                const V3<R> r = p - start.center;
-                const R distance = length(r);
-                const V3<R> normal = normalized(r);
-                const V3<R> rn = cross(r, normal);
-                c.p = r;
-                c.normal = normal;
-                c.gap = distance - cr;
-                c.eff_n = c.inm + ism + iin * dot(rn, rn);
-            } else {
-                c.p = p;
-            }
-            st[k] = c;
+    // A chunk: candidates [off, off + count) of slab b (b == L.blocks: none).
+    struct Chunk {
+        std::uint32_t b, off, count;
+    };
+    auto chunkAt = [&](std::uint32_t b, std::uint32_t off) {
+        for (; b < L.blocks; ++b, off = 0) {
+            const std::uint32_t n = L.cand_count[b];
+            if (off < n) return Chunk{b, off, n - off < kChunk ? n - off : kChunk};
+        }
+        return Chunk{b, 0U, 0U};
+    };
+    // Its records into a buffer, 16 bytes at a time, by threads [t0, t0 + nt).
+    auto copyIn = [&](const Chunk &c, Staged<R> *st, unsigned t0, unsigned nt) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(L.cand_stage + c.b * kCandidatesPerBlock + c.off);
+        uint4 *dst = reinterpret_cast<uint4 *>(st);
+        const std::uint32_t words = c.count * static_cast<std::uint32_t>(sizeof(Staged<R>) / sizeof(uint4));
+#pragma unroll 8
+        for (std::uint32_t k = threadIdx.x - t0; k < words; k += nt) dst[k] = __ldcg(src + k);
+    };
+    // Its hits back to the node arrays, by threads [t0, t0 + nt).
+    auto writeBack = [&](const Chunk &c, const Staged<R> *st, const ContactLog<R> *lg, unsigned hits, unsigned t0,
+                         unsigned nt) {
+        for (unsigned e = threadIdx.x - t0; e < hits; e += nt) {
+            const std::uint32_t k = lg[e].flags >> 8;
+            const std::uint32_t i = L.cand_list[c.b * kCandidatesPerBlock + c.off + k];
+            if (inBounds(i, L.N, kSiteCandidate)) contactSettle(L, S, pass, i, st[k].u, st[k].v);
         }
     };
-    // A slab's candidates back to the node arrays, by threads [t0, t0 + nt).
-    auto writeBack = [&](std::uint32_t b, const Staged<R> *st, unsigned t0, unsigned nt) {
-        const std::uint32_t n = L.cand_count[b];
-        const std::uint32_t *list = L.cand_list + b * kCandidatesPerBlock;
-        for (std::uint32_t k = threadIdx.x - t0; k < n; k += nt) {
-            const std::uint32_t i = list[k];
-            if (!inBounds(i, L.N, kSiteCandidate)) continue;
-            const Q4<R> vq = st[k].v;
-            const Q4<R> uq = st[k].u;
-            if (pass == 1) {
-                for (std::uint32_t p = 0; p < S.plane_count; ++p)
-                    L.approach[p * L.N + i] = dot(xyz(vq), S.planes[p].normal);
-                const V3<R> un = xyz(uq) + S.dt * xyz(vq);
-                L.u[i] = Q4<R>{un.x, un.y, un.z, uq.w};
-                L.v[i] = vq;
-            } else {
-                V3<R> vel = xyz(vq);
-                for (std::uint32_t p = 0; p < S.plane_count; ++p)
-                    if (L.engaged[p * L.N + i]) vel = supportVelocity(S.planes[p], vel, L.approach[p * L.N + i]);
-                L.u[i] = uq;
-                L.v[i] = Q4<R>{vel.x, vel.y, vel.z, vq.w};
-            }
-        }
-    };
-    // A slab's hit log into the fold lanes' sums (lane q: sum q).
+    // Its hit log into the fold lanes' sums (lane q: sum q).
     auto foldLog = [&](const ContactLog<R> *lg, unsigned n) {
-        if (lane < 3) {
-            for (unsigned e = 0; e < n; ++e) {
+        for (unsigned e = 0; e < n; ++e) {
+            const unsigned flags = lg[e].flags;
+            if (!(flags & kLogImpulse)) continue;
+            if (lane < 3) {
                 sum += static_cast<double>(lg[e].normal_imp[lane]);
-                if (lg[e].friction) sum += static_cast<double>(lg[e].friction_imp[lane]);
+                if (flags & kLogFriction) sum += static_cast<double>(lg[e].friction_imp[lane]);
+            } else {
+                sum += static_cast<double>(lg[e].lost);
             }
-        } else {
-            for (unsigned e = 0; e < n; ++e) sum += static_cast<double>(lg[e].lost);
         }
     };
-    // The serial chain over a staged slab, on warp 0; its hits go to `lg`.
+    // The serial chain over a chunk, on warp 0; its hits go to `lg`.
     auto runChain = [&](std::uint32_t n, Staged<R> *st, ContactLog<R> *lg, unsigned &logged) {
-        std::uint32_t k0 = 0;
-        unsigned hits = 0;
-        while (k0 < n) {
+        unsigned hits = 0, impulses = 0;
+        for (std::uint32_t k0 = 0; k0 < n; k0 += 32) {
             const std::uint32_t k = k0 + lane;
-            // hit: the contact changes the sphere or the node (an impulse, or
-            // a position correction in pass 2). graze: it passes the gate but
-            // only raises the penetration record, a maximum that any order
-            // forms alike.
-            bool hit = false, graze = false;
-            R pen = R(0);
-            V3<R> r{}, normal{};
-            R gap = R(0), eff_n = R(0), vn = R(0), ni = R(0);
-            if (k < n) {
-                const Staged<R> &c = st[k];
-                if (c.v.w > R(0)) {
-                    if (pass == 1) {
-                        r = c.p;
-                        normal = c.normal;
-                        gap = c.gap;
-                        eff_n = c.eff_n;
+            Staged<R> c{};
+            if (k < n) c = st[k];
+            const bool movable = k < n && c.v.w > R(0);
+            ContactGeometry<R> g{c.p, c.normal, c.gap, c.eff_n};
+            unsigned from = 0;
+            bool moved = pass == 2; // the sphere's centre since `g` was formed
+            for (;;) {
+                ContactTry<R> t{};
+                if (movable && lane >= from) {
+                    auto attempt = [&](auto &m) {
+                        if (pass == 2 && moved) g = contactGeometry<R>(m, c.p - sp.center, cr, c.inm, ism, iin);
+                        t = contactTry<R>(m, S, sp, xyz(c.v), g, c.v.w, c.inm, c.before, ism, iin, pass == 2);
+                    };
+                    if constexpr (std::is_same<R, float>::value) {
+                        QuickMath quick;
+                        attempt(quick);
+                        if (!quick.good) {
+                            PlainMath<R> plain;
+                            attempt(plain);
+                        }
                     } else {
-                        r = c.p - sp.center;
-                        const R distance = length(r);
-                        normal = normalized(r);
-                        const V3<R> rn = cross(r, normal);
-                        eff_n = c.inm + ism + iin * dot(rn, rn);
-                        gap = distance - cr;
-                    }
-                    const int probe = contactProbe(S, sp, xyz(c.v), r, normal, gap, eff_n, pass == 2, vn, ni);
-                    hit = probe == 2;
-                    graze = probe == 1;
-                    pen = -gap;
-                }
-            }
-            const unsigned mask = __ballot_sync(0xffffffffU, hit);
-            const unsigned limit = mask ? static_cast<unsigned>(__ffs(mask) - 1) : 32U;
-            // The grazes before the first hit raise the record as the serial
-            // chain would have, one after another.
-            const bool raises = graze && lane < limit && pen > max_pen;
-            if (__any_sync(0xffffffffU, raises)) {
-                R best = raises ? pen : max_pen;
-                if constexpr (std::is_same<R, float>::value) {
-                    // The record starts at zero and only grows, so a raising
-                    // value is positive and its bits order as its value.
-                    best = __uint_as_float(__reduce_max_sync(0xffffffffU, __float_as_uint(best)));
-                } else {
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const R other = __shfl_xor_sync(0xffffffffU, best, o);
-                        best = other > best ? other : best;
+                        PlainMath<R> plain;
+                        attempt(plain);
                     }
                 }
-                if (best > max_pen) {
-                    max_pen = best;
-                    acc.max_penetration = static_cast<double>(best);
+                const unsigned mask = __ballot_sync(0xffffffffU, t.kind == 2);
+                const unsigned j = mask ? static_cast<unsigned>(__ffs(mask) - 1) : 32U;
+                if (t.kind != 0 && lane <= j && -g.gap > max_pen) max_pen = -g.gap;
+                if (mask == 0) break;
+                const bool mine = lane == j;
+                const bool impulse = __ballot_sync(0xffffffffU, mine && t.impulse) != 0;
+                const int src = static_cast<int>(j);
+                sp.velocity = {__shfl_sync(0xffffffffU, t.sv.x, src), __shfl_sync(0xffffffffU, t.sv.y, src),
+                               __shfl_sync(0xffffffffU, t.sv.z, src)};
+                sp.angular = {__shfl_sync(0xffffffffU, t.sw.x, src), __shfl_sync(0xffffffffU, t.sw.y, src),
+                              __shfl_sync(0xffffffffU, t.sw.z, src)};
+                if (mine) {
+                    if (impulse) st[k].v = Q4<R>{t.nv.x, t.nv.y, t.nv.z, c.v.w};
+                    else t.log.flags = 0;
+                    t.log.flags |= k << 8;
+                    lg[hits] = t.log;
                 }
+                ++hits;
+                impulses += impulse ? 1U : 0U;
+                moved = false;
+                if (pass == 2) {
+                    V3<R> center = sp.center;
+                    const bool deep = mine && g.gap < -S.c_margin;
+                    if (deep) {
+                        Q4<R> uq = c.u;
+                        const R corr = contactCorrect<R>(S, sp, g, c.inm, ism, uq, center);
+                        st[k].u = uq;
+                        if (corr > max_corr) max_corr = corr;
+                    }
+                    moved = __any_sync(0xffffffffU, deep);
+                    if (moved)
+                        sp.center = {__shfl_sync(0xffffffffU, center.x, src), __shfl_sync(0xffffffffU, center.y, src),
+                                     __shfl_sync(0xffffffffU, center.z, src)};
+                }
+                from = j + 1;
+                if (from == 32) break;
             }
-            if (mask == 0) {
-                k0 += 32;
-                continue;
-            }
-            const std::uint32_t j = k0 + limit;
-            Staged<R> c = st[j];
-            // The hit lane's geometry, computed in the scan against the state
-            // the chain is in, to every lane.
-            const int src = static_cast<int>(limit);
-            const V3<R> hr{__shfl_sync(0xffffffffU, r.x, src), __shfl_sync(0xffffffffU, r.y, src),
-                           __shfl_sync(0xffffffffU, r.z, src)};
-            const V3<R> hn{__shfl_sync(0xffffffffU, normal.x, src), __shfl_sync(0xffffffffU, normal.y, src),
-                           __shfl_sync(0xffffffffU, normal.z, src)};
-            const R hgap = __shfl_sync(0xffffffffU, gap, src);
-            const R hni = __shfl_sync(0xffffffffU, ni, src);
-            ContactLog<R> entry;
-            const bool logs = contactChain(S, sp, c, hr, hn, hgap, hni, ism, iin, pass == 2, acc, max_pen, max_corr,
-                                           entry);
-            __syncwarp();
-            if (lane == 0) {
-                st[j] = c;
-                if (logs) lg[hits] = entry;
-            }
-            hits += logs ? 1U : 0U;
-            k0 = j + 1;
         }
+        acc.impulse_contacts += impulses;
         if (lane == 0) logged = hits;
     };
-    // The next slab with candidates after b (L.blocks: none).
-    auto nextSlab = [&](std::uint32_t b) {
-        while (b < L.blocks && L.cand_count[b] == 0) ++b;
-        return b;
-    };
-
-    if (buffers == 2) {
-        std::uint32_t cur = nextSlab(0);
-        if (cur < L.blocks) stageSlab(cur, stage_base, 0, blockDim.x);
+    Chunk cur = chunkAt(0, 0), prev{L.blocks, 0U, 0U};
+    if (cur.b < L.blocks) copyIn(cur, stage_base, 0, blockDim.x);
+    __syncthreads();
+    unsigned cb = 0;
+    while (cur.b < L.blocks) {
+        const Chunk nxt = chunkAt(cur.b, cur.off + cur.count);
+        const unsigned ob = cb ^ 1U;
+        Staged<R> *const other = stage_base + ob * kChunk;
+        ContactLog<R> *const other_log = log_base + ob * kChunk;
+        if (chain) {
+            runChain(cur.count, stage_base + cb * kChunk, log_base + cb * kChunk, log_count[cb]);
+        } else if (threadIdx.x < 64) {
+            if (fold && prev.b < L.blocks) foldLog(other_log, log_count[ob]);
+        } else {
+            if (prev.b < L.blocks) writeBack(prev, other, other_log, log_count[ob], 64, blockDim.x - 64);
+            // The write-back reads the buffer the copy fills.
+            asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x - 64) : "memory");
+            if (nxt.b < L.blocks) copyIn(nxt, other, 64, blockDim.x - 64);
+        }
         __syncthreads();
-        std::uint32_t prev = L.blocks;
-        unsigned cb = 0;
-        while (cur < L.blocks) {
-            const std::uint32_t nxt = nextSlab(cur + 1);
-            const unsigned ob = cb ^ 1U;
-            if (chain) {
-                runChain(L.cand_count[cur], stage_base + cb * kCandidatesPerBlock, log_base + cb * kCandidatesPerBlock,
-                         log_count[cb]);
-            } else if (threadIdx.x < 64) {
-                if (fold && prev < L.blocks) foldLog(log_base + ob * kCandidatesPerBlock, log_count[ob]);
-            } else {
-                Staged<R> *other = stage_base + ob * kCandidatesPerBlock;
-                if (prev < L.blocks) writeBack(prev, other, 64, blockDim.x - 64);
-                if (nxt < L.blocks) stageSlab(nxt, other, 64, blockDim.x - 64);
-            }
-            __syncthreads();
-            prev = cur;
-            cur = nxt;
-            cb = ob;
-        }
-        if (prev < L.blocks) {
-            if (fold) foldLog(log_base + (cb ^ 1U) * kCandidatesPerBlock, log_count[cb ^ 1U]);
-            writeBack(prev, stage_base + (cb ^ 1U) * kCandidatesPerBlock, 0, blockDim.x);
-        }
-    } else {
-        for (std::uint32_t b = nextSlab(0); b < L.blocks; b = nextSlab(b + 1)) {
-            stageSlab(b, stage_base, 0, blockDim.x);
-            __syncthreads();
-            if (chain) runChain(L.cand_count[b], stage_base, log_base, log_count[0]);
-            __syncthreads();
-            if (fold) foldLog(log_base, log_count[0]);
-            writeBack(b, stage_base, 0, blockDim.x);
-            __syncthreads();
-        }
+        prev = cur;
+        cur = nxt;
+        cb = ob;
+    }
+    if (prev.b < L.blocks) {
+        const unsigned ob = cb ^ 1U;
+        if (fold) foldLog(log_base + ob * kChunk, log_count[ob]);
+        writeBack(prev, stage_base + ob * kChunk, log_base + ob * kChunk, log_count[ob], 0, blockDim.x);
     }
     if (fold) folded[lane] = sum;
+    if (chain) {
+        for (int o = 16; o > 0; o >>= 1) {
+            max_pen = maxR(max_pen, __shfl_xor_sync(0xffffffffU, max_pen, o));
+            max_corr = maxR(max_corr, __shfl_xor_sync(0xffffffffU, max_corr, o));
+        }
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
+        // The records only ever hold a widened R.
+        if (max_pen > R(acc.max_penetration)) acc.max_penetration = static_cast<double>(max_pen);
+        if (max_corr > R(acc.max_correction)) acc.max_correction = static_cast<double>(max_corr);
         acc.impulse_x = folded[0];
         acc.impulse_y = folded[1];
         acc.impulse_z = folded[2];
