@@ -2177,6 +2177,7 @@ private:
         c.nc_rebuild = 1; // the pair list is built before its first use
         c.energy_flat_fraction = 1.0e-3;
         c.calm_damage_margin = 0.5;
+        c.damage_floor = 1.0e-6F; // 9.9999999747e-7
         c.step_limit = step_limit;
         c.live_bonds = slots_[k]->live_bonds;
         ctl_host_[k] = c;

@@ -123,6 +123,7 @@ struct Ctl {
     unsigned long long total_steps, first_failure_step, last_failure_step, last_energy_gain_step, last_damage_gain_step;
     unsigned failure_rounds, broken_bonds, rank_deficient, exit_reason;
     double removed_energy, max_damage, plastic_work;
+    float damage_floor; // the largest float not above max_damage + 1e-6
     unsigned max_t, max_c, max_s, max_plastic; // non-negative float bit patterns
     ContactAcc contact;
     LoadLedger ext;
@@ -299,6 +300,15 @@ __device__ __forceinline__ const Dev<R> &descriptorIn(const Grid<R> &g, const Wo
 
 template <class R> __device__ __forceinline__ V3<R> pos(const Dev<R> &L, std::uint32_t i) {
     return xyz(L.x0[i]) + xyz(L.u[i]);
+}
+
+// The node arrays a bond's sample reads.
+template <class R> struct NodeView {
+    const Q4<R> *u, *x0, *strain;
+};
+template <class R> __device__ __forceinline__ NodeView<R> viewOf(const Dev<R> &L) { return {L.u, L.x0, L.strain}; }
+template <class R> __device__ __forceinline__ V3<R> pos(const NodeView<R> &V, std::uint32_t i) {
+    return xyz(V.x0[i]) + xyz(V.u[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -545,36 +555,36 @@ __global__ void __launch_bounds__(kThreads) kRestartStrain(const Grid<R> launch,
 // Bond samples (LatticePhysics.hpp:921-959, 1116-1126).
 // ---------------------------------------------------------------------------
 template <class R, bool Direct>
-__device__ __forceinline__ V3<R> bondVector(const Dev<R> &L, std::uint32_t a, std::uint32_t b, V3<R> edge) {
-    if (Direct) return pos(L, b) - pos(L, a);
-    return edge + (xyz(L.u[b]) - xyz(L.u[a]));
+__device__ __forceinline__ V3<R> bondVector(const NodeView<R> &V, std::uint32_t a, std::uint32_t b, V3<R> edge) {
+    if (Direct) return pos(V, b) - pos(V, a);
+    return edge + (xyz(V.u[b]) - xyz(V.u[a]));
 }
 
-template <class R, bool Direct>
-__device__ void sampleBond(const Dev<R> &L, std::uint32_t a, std::uint32_t b, const BondRec<R> &rec, V3<R> edge,
-                           R len, R &t, R &c, R &s) {
+template <class R, bool Direct, class M>
+__device__ __forceinline__ void sampleBond(M &m, const NodeView<R> &V, std::uint32_t a, std::uint32_t b, const BondRec<R> &rec,
+                                           V3<R> edge, R len, R &t, R &c, R &s) {
     const R rest = rec.rest;
     R stretch;
     if (Direct) {
-        stretch = len / rest - R(1);
+        stretch = m.div(len, rest) - R(1);
     } else {
-        const V3<R> du = xyz(L.u[b]) - xyz(L.u[a]);
+        const V3<R> du = xyz(V.u[b]) - xyz(V.u[a]);
         const R num = rec.rsm + R(2) * dot(edge, du) + dot(du, du);
-        stretch = num / ((len + rest) * rest);
+        stretch = m.div(num, (len + rest) * rest);
     }
     t = stretch;
     c = -stretch;
     s = R(0);
-    const R rl = length(edge);
+    const R rl = m.root(dot(edge, edge));
     if (rl > R(1.0e-9)) {
-        const V3<R> dir = edge * (R(1) / rl);
+        const V3<R> dir = edge * m.div(R(1), rl);
         const std::uint32_t ends[2] = {a, b};
         for (int q = 0; q < 2; ++q) {
-            const Q4<R> s0 = L.strain[2 * ends[q]], s1 = L.strain[2 * ends[q] + 1];
+            const Q4<R> s0 = V.strain[2 * ends[q]], s1 = V.strain[2 * ends[q] + 1];
             if (s1.z == R(0)) continue;
             const R e[6] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y};
             R nn, sh;
-            resolveAlong(e, dir, nn, sh);
+            resolveAlong(m, e, dir, nn, sh);
             t = maxR(t, nn);
             c = maxR(c, -nn);
             s = maxR(s, sh);
@@ -582,19 +592,49 @@ __device__ void sampleBond(const Dev<R> &L, std::uint32_t a, std::uint32_t b, co
     }
 }
 
+// The current length of a bond and its sample, branch-free in the float lane
+// where its operands allow.
+template <class R> struct BondSample {
+    R len, t, c, s;
+};
+template <class R, bool Direct, class M>
+__device__ __forceinline__ BondSample<R> lengthAndSample(M &m, const NodeView<R> &V, std::uint32_t a, std::uint32_t b,
+                                                         const BondRec<R> &rec, V3<R> edge) {
+    BondSample<R> o;
+    const V3<R> now = bondVector<R, Direct>(V, a, b, edge);
+    o.len = m.root(dot(now, now));
+    sampleBond<R, Direct>(m, V, a, b, rec, edge, o.len, o.t, o.c, o.s);
+    return o;
+}
 template <class R, bool Direct>
-__device__ __forceinline__ void startSample(const Dev<R> &L, std::uint32_t j) {
+__device__ __noinline__ BondSample<R> sampleAnywhere(NodeView<R> V, std::uint32_t a, std::uint32_t b, R rsm, R rest,
+                                                     V3<R> edge) {
+    PlainMath<R> plain;
+    return lengthAndSample<R, Direct>(plain, V, a, b, BondRec<R>{a, b, rsm, rest}, edge);
+}
+template <class R, bool Direct>
+__device__ __forceinline__ BondSample<R> sampleOf(const NodeView<R> &V, std::uint32_t a, std::uint32_t b, const BondRec<R> &rec,
+                                                  V3<R> edge) {
+    if constexpr (std::is_same<R, float>::value && !Direct) {
+        QuickMath quick;
+        const BondSample<R> o = lengthAndSample<R, Direct>(quick, V, a, b, rec, edge);
+        return quick.good ? o : sampleAnywhere<R, Direct>(V, a, b, rec.rsm, rec.rest, edge);
+    } else {
+        PlainMath<R> plain;
+        return lengthAndSample<R, Direct>(plain, V, a, b, rec, edge);
+    }
+}
+
+template <class R, bool Direct>
+__device__ __forceinline__ void startSample(const Dev<R> &L, const NodeView<R> &V, std::uint32_t j) {
     const BondRec<R> rec = L.rec[j];
     if (rec.a & kDeadBit) return;
     const Q4<R> g = L.geo[j];
-    R t, c, s;
-    const V3<R> edge{g.x, g.y, g.z};
-    const R len = length(bondVector<R, Direct>(L, endA(rec), endB(rec), edge));
-    sampleBond<R, Direct>(L, endA(rec), endB(rec), rec, edge, len, t, c, s);
+    const BondSample<R> o = sampleOf<R, Direct>(V, endA(rec), endB(rec), rec, V3<R>{g.x, g.y, g.z});
     Q4<R> p = L.prev[j];
-    p.x = maxR(R(0), t);
-    p.y = maxR(R(0), c);
-    p.z = maxR(R(0), s);
+    p.x = maxR(R(0), o.t);
+    p.y = maxR(R(0), o.c);
+    p.z = maxR(R(0), o.s);
     L.prev[j] = p;
 }
 
@@ -608,13 +648,14 @@ template <class R, bool Many, bool Direct>
 __global__ void __launch_bounds__(kThreads) kRestartBonds(const Grid<R> launch, int after_kick) {
     startAfterPrevious();
     const Work w = item<Many>(launch);
-    Dev<R> L = descriptor<R, Many>(launch, w);
-    if (after_kick) L.u = L.up;
+    __shared__ SharedDesc<R> desc;
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     if (L.ctl->stop) return;
+    const NodeView<R> V{after_kick ? L.up : L.u, L.x0, L.strain};
     const std::uint32_t d = w.begin + threadIdx.x;
     if (d >= w.end) return;
     if (L.ctl->full_restart) {
-        startSample<R, Direct>(L, d);
+        startSample<R, Direct>(L, V, d);
         return;
     }
     const std::uint32_t dirty = L.ctl->dirty_count;
@@ -624,7 +665,7 @@ __global__ void __launch_bounds__(kThreads) kRestartBonds(const Grid<R> launch, 
         const std::uint32_t node = L.dirty_list[q - static_cast<std::uint64_t>(k) * dirty];
         if (!inBounds(node, L.N, kSiteDirty)) continue;
         const std::uint32_t bond = L.nbr_bond[static_cast<std::size_t>(k) * L.N + node];
-        if (bond != kNoBond && inBounds(bond, L.B, kSiteDirtyBond)) startSample<R, Direct>(L, bond);
+        if (bond != kNoBond && inBounds(bond, L.B, kSiteDirtyBond)) startSample<R, Direct>(L, V, bond);
     }
 }
 
@@ -1555,12 +1596,12 @@ __device__ __forceinline__ FloatStep floatStep(const Settings<float> &S, V3<floa
     FloatStep s;
     s.dl = quotient(pull, w, recipNearest(w));
     s.dir = {quotient(delta.x, cl, ycl), quotient(delta.y, cl, ycl), quotient(delta.z, cl, ycl)};
-    s.moves = true; // rootOk: the length is above 1e-12
+    s.moves = true; // a square of 2^-78 or more: the length is above 1e-12
     const std::uint32_t least =
         __vimin3_u32(__vimin3_u32(dividendKey(delta.x), dividendKey(delta.y), dividendKey(delta.z)), dividendKey(num),
                      min(dividendKey(pull), dividendKey(compliance)));
     // An infinite or NaN operand leaves a NaN or an infinity in s.dl or w.
-    if (!(rootOk(sq) && divisorOk(den) && divisorOk(w) && least >= kDividendLeast && fabsf(s.dl) < 0x1p100F))
+    if (!(rootOk(sq) && sq >= 0x1p-78F && divisorOk(den) && divisorOk(w) && least >= kDividendLeast && fabsf(s.dl) < 0x1p100F))
         s = floatStepAnywhere<Plastic>(ua, ub, edge, rsm, original, compliance, wa, wb, lambda, plastic, S.dt);
     return s;
 }
@@ -1901,7 +1942,7 @@ __global__ void __launch_bounds__(kThreads) kDamp(const Grid<R> launch, R fracti
         const R ma = va.w, mb = vb.w;
         if (ma <= R(0) || mb <= R(0)) continue;
         const Q4<R> g = L.geo[d];
-        const V3<R> n = normalized(bondVector<R, Direct>(L, a, b, V3<R>{g.x, g.y, g.z}));
+        const V3<R> n = normalized(bondVector<R, Direct>(viewOf(L), a, b, V3<R>{g.x, g.y, g.z}));
         const R rel = dot(xyz(vb) - xyz(va), n);
         const R im = R(1) / ma + R(1) / mb;
         const R impulse = -fraction * rel / im;
@@ -1991,7 +2032,6 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
     __shared__ SharedDesc<R> desc;
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     __shared__ double tile_work[kThreads / 32];
-    __shared__ unsigned peak[4];
     if (L.ctl->stop) return;
     // part 0: every tile; 1: the tiles outside the contact halo; 2: inside it.
     if (part != 0) {
@@ -1999,18 +2039,8 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
         if (late != (part == 2)) return;
     }
     const std::uint32_t j = w.begin + threadIdx.x; // storage index; items start on multiples of 256
-    // A bond can raise the run's damage maximum only if it exceeds the maximum
-    // as the substep began (CpuLatticeBackend.cpp:462-465); the bound is formed
-    // once per CTA.
-    __shared__ double damage_floor;
-    __shared__ int any_work;
-    if (threadIdx.x < 4) peak[threadIdx.x] = 0;
-    if (threadIdx.x == 0) {
-        damage_floor = L.ctl->max_damage + 1.0e-6;
-        any_work = 0;
-    }
-    __syncthreads();
     double plastic_work = 0.0;
+    unsigned peaks[4] = {0, 0, 0, 0};
     if (j < w.end) {
         // Every per-bond array is loaded at once, ahead of the liveness test
         // and of the node gathers that wait on the record: one trip to memory
@@ -2029,7 +2059,8 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
             R pext = R(0);
             // The bond's current length, used by the plastic return, the
             // sample and the stored energy of a failure alike.
-            const R len = length(bondVector<R, Direct>(L, a, b, edge));
+            const BondSample<R> sample = sampleOf<R, Direct>(viewOf(L), a, b, rec, edge);
+            const R len = sample.len, t = sample.t, c = sample.c, s = sample.s;
             if (Plastic) {
                 pext = pl.x;
                 if (S.yield_stretch > R(0)) {
@@ -2043,17 +2074,14 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
                         pl.y = pl.y + inc;
                         L.plastic[j] = pl;
                         pext = pl.x;
-                        const R c = g.w;
-                        if (c > R(0)) {
+                        if (g.w > R(0)) {
                             const R yield_end = yield + h * inc;
-                            plastic_work = static_cast<double>(R(0.5) * (yield + yield_end) * inc / c);
+                            plastic_work = static_cast<double>(R(0.5) * (yield + yield_end) * inc / g.w);
                         }
                     }
                     plastic_stretch = static_cast<float>(absR(pl.x) / rec.rest);
                 }
             }
-            R t, c, s;
-            sampleBond<R, Direct>(L, a, b, rec, edge, len, t, c, s);
             const R pt = maxR(R(0), maxR(pv.x, t));
             const R pc = maxR(R(0), maxR(pv.y, c));
             const R ps = maxR(R(0), maxR(pv.z, s));
@@ -2073,8 +2101,8 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
             }
             L.prev[j] = pv;
             const float dmg = static_cast<float>(pv.w);
-            const std::uint32_t js = L.dev2sched[j];
             if (pv.w >= R(1)) {
+                const std::uint32_t js = L.dev2sched[j];
                 const R cc = g.w;
                 R energy = R(0);
                 if (!(cc <= R(0))) {
@@ -2090,35 +2118,42 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
                 L.ev_ends[js] = make_uint2(a, b);
                 atomicOr(L.ev_bits + (js >> 5), 1U << (js & 31U));
             }
-            if (static_cast<double>(dmg) > damage_floor) {
+            // A bond can raise the run's damage maximum only if it exceeds the
+            // maximum as the substep began (CpuLatticeBackend.cpp:462-465);
+            // the bound is a float (kLedger), so no thread forms an FP64 one.
+            if (dmg > L.ctl->damage_floor) {
+                const std::uint32_t js = L.dev2sched[j];
                 L.ev_damage[js] = dmg;
                 atomicOr(L.dmg_bits + (js >> 5), 1U << (js & 31U));
             }
             // Peaks are non-negative, so their bit patterns order as the values do.
-            atomicMax(&peak[0], floatBits(static_cast<float>(pt)));
-            atomicMax(&peak[1], floatBits(static_cast<float>(pc)));
-            atomicMax(&peak[2], floatBits(static_cast<float>(ps)));
-            if (Plastic && S.yield_stretch > R(0)) atomicMax(&peak[3], floatBits(plastic_stretch));
+            peaks[0] = floatBits(static_cast<float>(pt));
+            peaks[1] = floatBits(static_cast<float>(pc));
+            peaks[2] = floatBits(static_cast<float>(ps));
+            if (Plastic && S.yield_stretch > R(0)) peaks[3] = floatBits(plastic_stretch);
         }
     }
-    // Fixed-order sums of the plastic work; a sum of zeros is +0 whichever
-    // way it is formed, so all-zero warps and tiles skip the FP64 adds.
-    double warp_work = 0.0;
-    if (Plastic && __any_sync(0xffffffffU, plastic_work != 0.0)) {
-        warp_work = warpSumFixed(plastic_work);
-        if ((threadIdx.x & 31) == 0) any_work = 1;
+    // The run's peaks: a warp asks for the atomic only above what it reads
+    // there (they only grow, so a stale read asks once too often at most).
+    unsigned *const records[4] = {&L.ctl->max_t, &L.ctl->max_c, &L.ctl->max_s, &L.ctl->max_plastic};
+    for (int q = 0; q < (Plastic ? 4 : 3); ++q) {
+        const unsigned top = __reduce_max_sync(0xffffffffU, peaks[q]);
+        if ((threadIdx.x & 31) == 0 && top > *records[q]) atomicMax(records[q], top);
     }
+    if (!Plastic) return;
+    // Fixed-order sums of the plastic work; a sum of zeros is +0 whichever
+    // way it is formed, so all-zero tiles skip the FP64 adds.
+    if (!__syncthreads_or(plastic_work != 0.0)) {
+        if (threadIdx.x == 0) L.tile_plastic[w.begin / kThreads] = 0.0;
+        return;
+    }
+    const double warp_work = warpSumFixed(plastic_work);
     if ((threadIdx.x & 31) == 0) tile_work[threadIdx.x / 32] = warp_work;
     __syncthreads();
     if (threadIdx.x == 0) {
         double wsum = 0.0;
-        if (any_work)
-            for (int q = 0; q < kThreads / 32; ++q) wsum += tile_work[q];
+        for (int q = 0; q < kThreads / 32; ++q) wsum += tile_work[q];
         L.tile_plastic[w.begin / kThreads] = wsum;
-        if (peak[0]) atomicMax(&L.ctl->max_t, peak[0]);
-        if (peak[1]) atomicMax(&L.ctl->max_c, peak[1]);
-        if (peak[2]) atomicMax(&L.ctl->max_s, peak[2]);
-        if (peak[3]) atomicMax(&L.ctl->max_plastic, peak[3]);
     }
 }
 
@@ -2622,6 +2657,7 @@ __global__ void __launch_bounds__(32) kLedger(const Grid<R> launch, Settings<R> 
     c.plastic_work += c.plastic_substep;
     if (gained) {
         c.max_damage = record;
+        c.damage_floor = __double2float_rd(record + 1.0e-6);
         c.last_damage_gain_step = step;
     }
     const unsigned broken = c.event_count;

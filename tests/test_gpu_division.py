@@ -34,6 +34,14 @@ __global__ void roots(ull *bad, int exponent) {
     if (!rootOk(s)) atomicAdd(bad + 1, 1ULL);
     note(bad, 1, rootNearest(s), __fsqrt_rn(s));
 }
+// QuickMath::root scales what is below 2^-60: zero, every denormal exponent's
+// mantissas and the normals up to there.
+__global__ void tinyRoots(ull *bad, unsigned first) {
+    const float s = __uint_as_float(first + blockIdx.x * blockDim.x + threadIdx.x);
+    QuickMath m;
+    note(bad, 1, m.root(s), __fsqrt_rn(s));
+    if (!m.good) atomicAdd(bad + 1, 1ULL);
+}
 __global__ void midpoints(ull *bad, ull *tried) {
     const unsigned B = (1U << 23) | (blockIdx.x * blockDim.x + threadIdx.x);
     const float b = __uint_as_float(0x3f800000U | (B & 0x7fffffU)), y = recipNearest(b);
@@ -77,9 +85,10 @@ int main() {
     ull *c;
     cudaMallocManaged(&c, 8 * sizeof(ull));
     for (int k = 0; k < 8; ++k) c[k] = 0;
-    const int divisors[] = {-90, -40, -1, 0, 1, 29}, radicands[] = {-78, -77, -20, -19, 0, 1, 58, 59};
+    const int divisors[] = {-90, -40, -1, 0, 1, 29}, radicands[] = {-100, -99, -78, -77, -20, -19, 0, 1, 58, 59};
     for (int e : divisors) reciprocals<<<(1 << 23) / 256, 256>>>(c, e);
     for (int e : radicands) roots<<<(1 << 23) / 256, 256>>>(c, e);
+    for (unsigned e : {0U, 1U, 2U, 30U, 66U, 67U, 68U}) tinyRoots<<<(1 << 23) / 256, 256>>>(c, e << 23);
     midpoints<<<(1 << 23) / 256, 256>>>(c, c + 4);
     pairs<<<1024, 256>>>(c, 2000);
     const cudaError_t e = cudaDeviceSynchronize();
