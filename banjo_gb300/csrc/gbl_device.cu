@@ -2297,6 +2297,7 @@ private:
         using U = std::uint32_t;
         nodes_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.N; }, kThreads);
         bonds_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.B; }, kThreads);
+        restart_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.B; }, kRestartPer);
         tiles_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.dev.tiles_b; }, kCountTiles);
         static_assert(kCountTiles == kEmitTiles * (kEmitThreads / 32), "one item of tiles for both launches");
         several_blocks_ = false;
@@ -2706,7 +2707,7 @@ private:
                 next(kRestartStrain<R, M, kDirect, false>, nodes_.count, kThreads, 0, st, grid(nodes_), after_kick, plate, yield);
         }
         mark(1);
-        if (bonds_.count) next(kRestartBonds<R, M, kDirect>, bonds_.count, kThreads, 0, st, grid(bonds_), after_kick);
+        if (restart_.count) next(kRestartBonds<R, M, kDirect>, restart_.count, kThreads, 0, st, grid(restart_), after_kick);
         mark(2);
     }
 
@@ -2758,7 +2759,7 @@ private:
     unsigned *running_{}, *running_host_{};
     Dev<R> *table_{};
     Work *work_{};
-    Span nodes_{}, bonds_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, whole_{}, buckets_{},
+    Span nodes_{}, bonds_{}, restart_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, whole_{}, buckets_{},
         wrench_{};
     unsigned staged_threads_{0}; // the staged sweep's CTA size (0: the lattices do not sweep staged)
     std::size_t staged_smem_{0};

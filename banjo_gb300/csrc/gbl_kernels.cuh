@@ -639,11 +639,14 @@ __device__ __forceinline__ void startSample(const Dev<R> &L, const NodeView<R> &
 }
 
 // Every live bond after an upload, or the live bonds at each dirty node after a
-// failure round: items cover the bond storage range, and the lattice's threads
-// share the (slot, dirty node) pairs, consecutive threads on consecutive dirty
-// nodes. A bond with both ends dirty is sampled twice to the same values. (One
+// failure round: items cover the bond storage range, kRestartPer bonds a CTA
+// (most substeps have few dirty nodes, and a CTA per 256 bonds spent 111 us of
+// a 128-trial substep starting CTAs, 88,000 of them; 21 now), and the
+// lattice's threads share the (slot, dirty node) pairs, consecutive threads
+// on consecutive dirty nodes. A bond with both ends dirty is sampled twice to the same values. (One
 // thread per dirty node walking its slots was a chain of 18 or 32 samples: 39
 // us a substep in the 32x8x8 beam, now 8; 100 in the 128x32x32 bar, now 11.)
+constexpr unsigned kRestartPer = 8 * kThreads;
 template <class R, bool Many, bool Direct>
 __global__ void __launch_bounds__(kThreads) kRestartBonds(const Grid<R> launch, int after_kick) {
     startAfterPrevious();
@@ -652,15 +655,14 @@ __global__ void __launch_bounds__(kThreads) kRestartBonds(const Grid<R> launch, 
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     if (L.ctl->stop) return;
     const NodeView<R> V{after_kick ? L.up : L.u, L.x0, L.strain};
-    const std::uint32_t d = w.begin + threadIdx.x;
-    if (d >= w.end) return;
     if (L.ctl->full_restart) {
-        startSample<R, Direct>(L, V, d);
+        for (std::uint32_t d = w.begin + threadIdx.x; d < w.end; d += kThreads) startSample<R, Direct>(L, V, d);
         return;
     }
     const std::uint32_t dirty = L.ctl->dirty_count;
     const std::uint64_t pairs = static_cast<std::uint64_t>(dirty) * L.D;
-    for (std::uint64_t q = d; q < pairs; q += L.B) {
+    const std::uint64_t threads = static_cast<std::uint64_t>((L.B + kRestartPer - 1) / kRestartPer) * kThreads;
+    for (std::uint64_t q = w.begin / kRestartPer * kThreads + threadIdx.x; q < pairs; q += threads) {
         const std::uint32_t k = static_cast<std::uint32_t>(q / dirty);
         const std::uint32_t node = L.dirty_list[q - static_cast<std::uint64_t>(k) * dirty];
         if (!inBounds(node, L.N, kSiteDirty)) continue;
