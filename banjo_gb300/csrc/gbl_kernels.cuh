@@ -753,17 +753,113 @@ __global__ void __launch_bounds__(kThreads) kKick(const Grid<R> launch, Settings
 }
 
 // ---------------------------------------------------------------------------
+// A serial FP64 sum, by one warp: what s = (((s + x[0]) + x[1]) + ...) gives,
+// rounding by rounding, without its chain of dependent adds (38 ns each here).
+//
+// While the running sum stays inside one binade, it is an integer number M of
+// that binade's ulps, and adding x rounds M + x/ulp to the nearest integer:
+// unless x/ulp lies half-way between two integers, that is M + rint(x/ulp),
+// whatever M is. So the roundings are known before the sums, and the running
+// sums are integer prefix sums, which any order forms alike. A run of terms
+// is taken up to the first one that is a tie, is too large for the integers,
+// or takes the sum to the end of its binade (a sum that rounds to a binade's
+// own bound may have rounded in the one below); that term is added by the
+// hardware, and the next run starts from there. Sums of one sign cross few
+// binades. One that keeps crossing goes on term by term, longer each time.
+//
+// All of it is integer arithmetic on the terms' bits (this GPU has two FP64
+// lanes an SM: the same run with FP64 scaling, rint and conversions was slower
+// than the chain). `x` is in shared memory; every lane calls with the same
+// arguments and gets the sum.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double foldSerial(double s, const double *x, unsigned n) {
+    using u64 = unsigned long long;
+    constexpr unsigned kPer = 8; // consecutive terms per lane in a run
+    constexpr u64 kOne = 1ULL << 52;
+    const unsigned lane = threadIdx.x & 31;
+    const u64 *bits = reinterpret_cast<const u64 *>(x);
+    unsigned patience = 16; // terms taken one by one after a run that came to little
+    for (unsigned at = 0; at < n;) {
+        const u64 sb = static_cast<u64>(__double_as_longlong(s));
+        const int exponent = static_cast<int>((sb >> 52) & 0x7ff);
+        unsigned serial = 0;
+        if (exponent == 0 || exponent == 0x7ff) { // zero, subnormal or not finite
+            if ((sb << 1) == 0) {
+                // Zero terms leave a zero sum as it is (it is never -0 here: it
+                // started as +0 or is a cancellation).
+                const bool some = at + lane < n && (bits[at + lane] << 1) != 0;
+                const unsigned mask = __ballot_sync(0xffffffffU, some);
+                if (mask == 0) {
+                    at += 32;
+                    continue;
+                }
+                at += static_cast<unsigned>(__ffs(mask) - 1);
+            }
+            serial = 1;
+        } else {
+            const bool negative = (sb >> 63) != 0;
+            const unsigned first = at + lane * kPer;
+            // The running sums in ulps, signed as the sum is: M positive.
+            long long upto[kPer], sum = 0;
+            unsigned bad = kPer; // the first of the lane's terms that ends a run by itself
+#pragma unroll
+            for (unsigned k = 0; k < kPer; ++k) {
+                const u64 b = first + k < n ? bits[first + k] : 0ULL;
+                const int e = static_cast<int>((b >> 52) & 0x7ff);
+                const u64 mantissa = (b & (kOne - 1)) | (e ? kOne : 0ULL);
+                const int shift = exponent - (e ? e : 1); // x = mantissa / 2^shift ulps
+                const int by = shift < 0 ? 0 : shift > 55 ? 55 : shift;
+                const u64 low = mantissa & ((1ULL << by) - 1), half = (1ULL << by) >> 1;
+                const long long r = static_cast<long long>((mantissa >> by) + (low > half ? 1 : 0));
+                if (bad == kPer && (shift < 0 || (low == half && half != 0) || first + k >= n)) bad = k;
+                sum += ((b >> 63) != 0) != negative ? -r : r;
+                upto[k] = sum;
+            }
+            long long before = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long y = __shfl_up_sync(0xffffffffU, before, o);
+                if (lane >= static_cast<unsigned>(o)) before += y;
+            }
+            before += static_cast<long long>((sb & (kOne - 1)) | kOne) - sum;
+#pragma unroll
+            for (unsigned k = 0; k < kPer; ++k) {
+                const long long total = before + upto[k];
+                if (bad > k && !(total > static_cast<long long>(kOne) && total < static_cast<long long>(2 * kOne))) bad = k;
+            }
+            const unsigned stop = __reduce_min_sync(0xffffffffU, bad < kPer ? lane * kPer + bad : 32 * kPer);
+            if (stop) {
+                const unsigned pick = (stop - 1) % kPer;
+                long long mine = upto[0];
+#pragma unroll
+                for (unsigned k = 1; k < kPer; ++k)
+                    if (pick == k) mine = upto[k];
+                const u64 total = static_cast<u64>(__shfl_sync(0xffffffffU, before + mine, static_cast<int>((stop - 1) / kPer)));
+                s = __longlong_as_double(static_cast<long long>((sb & (0xfffULL << 52)) | (total & (kOne - 1))));
+            }
+            at += stop;
+            if (stop < 32 * kPer) {
+                serial = stop < 16 ? patience : 1;
+                patience = stop < 16 ? 2 * patience : stop >= 64 ? 16 : patience;
+            }
+        }
+        for (; serial && at < n; --serial, ++at) s += x[at];
+    }
+    return s;
+}
+
+// ---------------------------------------------------------------------------
 // External wrenches (ExternalLoads.hpp:171-238): each wrench's force and
 // torque spread over its nodes by mass about their mass centre, from the
 // current positions, before every kick. One CTA per wrench. The region's sums
-// (mass, centre, inertia tensor, the resultant checks) are folded serially in
-// node order as the reference folds them, each sum a chain on its own
-// thread, from chunks the CTA stages in shared memory; the eigen-solve of the
-// tensor is the reference's cyclic Jacobi in double. apply 1 writes the
-// kick's forces (when loads remain); a wrench the current geometry cannot
-// carry then stops the lattice before the kick changes anything, with
-// kErrWrench set (the reference throws there). apply 0 only validates, into
-// *verdict.
+// (mass, centre, inertia tensor, the resultant checks) are the reference's
+// serial folds in node order: the CTA forms a chunk's terms, a node per thread,
+// and a warp folds each sum (foldSerial). (Formed by the folding thread, a
+// node's divisions and norms cost it a microsecond each: 410 us a kick with 81
+// and 18 nodes, 173 now, most of it the eigen-solve.) The eigen-solve of the tensor is the
+// reference's cyclic Jacobi in double. apply 1 writes the kick's forces (when
+// loads remain); a wrench the current geometry cannot carry then stops the
+// lattice before the kick changes anything, with kErrWrench set (the reference
+// throws there). apply 0 only validates, into *verdict.
 // ---------------------------------------------------------------------------
 constexpr unsigned kWrenchThreads = 256;
 
@@ -777,68 +873,75 @@ __device__ __forceinline__ void wrenchSpread(const Dev<R> &L, const WrenchDev *w
     const WrenchDev w = ws[index];
     const std::uint32_t *list = lists + w.begin;
     const std::uint32_t n = w.end - w.begin;
-    const unsigned t = threadIdx.x;
-    __shared__ double sm[kWrenchThreads], sr[3][kWrenchThreads], sf[3][kWrenchThreads];
-    __shared__ double mass, center[3], tensor[9], alpha[3], moment[3], sums[8];
+    const unsigned t = threadIdx.x, warp = t / 32;
+    __shared__ double terms[8][kWrenchThreads]; // a chunk's terms of up to eight sums
+    __shared__ double sums[8], mass, center[3], tensor[9], alpha[3], moment[3];
     __shared__ int bad;
     if (t == 0) bad = 0;
     const std::uint32_t a0 = list[0];
     const V3<R> p0 = xyz(L.x0[a0]) + xyz(L.u[a0]);
     const double anchor[3] = {double(p0.x), double(p0.y), double(p0.z)};
     __syncthreads();
-    // One pass over the region: stage(k, slot) for the chunk's nodes, then
-    // fold(count) over the staged chunk.
-    auto pass = [&](auto &&stage, auto &&fold) {
+    // One pass over the region: form(k, j) writes node k's terms at place j of
+    // the first `count` sums; warp q folds sum q, left in sums[q].
+    auto pass = [&](unsigned count, auto &&form) {
+        double acc = 0.0;
         for (std::uint32_t base = 0; base < n; base += kWrenchThreads) {
-            if (base + t < n) stage(base + t, t);
+            if (base + t < n) form(base + t, t);
             __syncthreads();
-            fold(n - base < kWrenchThreads ? n - base : kWrenchThreads);
+            if (warp < count) acc = foldSerial(acc, terms[warp], n - base < kWrenchThreads ? n - base : kWrenchThreads);
             __syncthreads();
         }
+        if (warp < count && t % 32 == 0) sums[warp] = acc;
+        __syncthreads();
     };
-    // Mass and position relative to the anchor; movable, finite nodes only.
-    auto stageNode = [&](std::uint32_t k, unsigned j) {
+    // Mass, and position relative to the anchor; movable, finite nodes only.
+    auto node = [&](std::uint32_t k, double &m, double r[3]) {
         const std::uint32_t i = list[k];
         const Q4<R> u = L.u[i], v = L.v[i]; // w: inverse mass, mass
         const V3<R> p = xyz(L.x0[i]) + xyz(u);
-        sm[j] = double(v.w);
-        sr[0][j] = double(p.x) - anchor[0];
-        sr[1][j] = double(p.y) - anchor[1];
-        sr[2][j] = double(p.z) - anchor[2];
-        if (!(v.w > R(0)) || !(u.w > R(0)) || !isfinite(v.w) || !isfinite(u.w) || !isfinite(sr[0][j]) ||
-            !isfinite(sr[1][j]) || !isfinite(sr[2][j]))
+        m = double(v.w);
+        r[0] = double(p.x) - anchor[0];
+        r[1] = double(p.y) - anchor[1];
+        r[2] = double(p.z) - anchor[2];
+        if (!(v.w > R(0)) || !(u.w > R(0)) || !isfinite(v.w) || !isfinite(u.w) || !isfinite(r[0]) || !isfinite(r[1]) ||
+            !isfinite(r[2]))
             bad = 1;
     };
-    double acc = 0.0;
-    pass(stageNode, [&](unsigned m) {
-        if (t == 0)
-            for (unsigned j = 0; j < m; ++j) acc += sm[j];
+    pass(1, [&](std::uint32_t k, unsigned j) {
+        double m, r[3];
+        node(k, m, r);
+        terms[0][j] = m;
     });
     if (t == 0) {
-        mass = acc;
-        if (!(acc > 0) || !isfinite(acc)) bad = 1;
+        mass = sums[0];
+        if (!(mass > 0) || !isfinite(mass)) bad = 1;
     }
     __syncthreads();
-    acc = 0.0;
-    pass(stageNode, [&](unsigned m) {
-        if (t < 3)
-            for (unsigned j = 0; j < m; ++j) acc = acc + sr[t][j] * (sm[j] / mass);
+    pass(3, [&](std::uint32_t k, unsigned j) {
+        double m, r[3];
+        node(k, m, r);
+        const double share = m / mass;
+        for (int q = 0; q < 3; ++q) terms[q][j] = r[q] * share;
     });
-    if (t < 3) center[t] = acc;
+    if (t < 3) center[t] = sums[t];
     __syncthreads();
-    acc = 0.0;
-    pass(stageNode, [&](unsigned m) {
-        if (t < 9) {
-            const unsigned a = t / 3, b = t % 3;
-            for (unsigned j = 0; j < m; ++j) {
-                const double r[3] = {sr[0][j] - center[0], sr[1][j] - center[1], sr[2][j] - center[2]};
-                const double share = sm[j] / mass;
-                acc = acc + share * (a == b ? r[(a + 1) % 3] * r[(a + 1) % 3] + r[(a + 2) % 3] * r[(a + 2) % 3]
-                                            : -r[a] * r[b]);
-            }
-        }
+    // The tensor is symmetric: xx, yy, zz, xy, xz, yz.
+    pass(6, [&](std::uint32_t k, unsigned j) {
+        double m, p[3];
+        node(k, m, p);
+        const double r[3] = {p[0] - center[0], p[1] - center[1], p[2] - center[2]};
+        const double share = m / mass;
+        for (int a = 0; a < 3; ++a)
+            terms[a][j] = share * (r[(a + 1) % 3] * r[(a + 1) % 3] + r[(a + 2) % 3] * r[(a + 2) % 3]);
+        terms[3][j] = share * (-r[0] * r[1]);
+        terms[4][j] = share * (-r[0] * r[2]);
+        terms[5][j] = share * (-r[1] * r[2]);
     });
-    if (t < 9) tensor[t] = acc;
+    if (t < 9) {
+        const unsigned a = t / 3, b = t % 3;
+        tensor[t] = sums[a == b ? a : a + b + 2];
+    }
     __syncthreads();
     if (t == 0) {
         const double arm[3] = {((w.point[0] - L.origin[0]) - anchor[0]) - center[0],
@@ -885,20 +988,16 @@ __device__ __forceinline__ void wrenchSpread(const Dev<R> &L, const WrenchDev *w
         }
     }
     __syncthreads();
-    // Node forces, written for the kick, then the resultant checks.
-    double part = 0.0;
-    pass([&](std::uint32_t k, unsigned j) {
-        stageNode(k, j);
-        const double m = sm[j], share = m / mass;
-        const double r[3] = {sr[0][j] - center[0], sr[1][j] - center[1], sr[2][j] - center[2]};
+    // Node forces, written for the kick, and the resultant checks.
+    pass(8, [&](std::uint32_t k, unsigned j) {
+        double m, p[3];
+        node(k, m, p);
+        const double share = m / mass;
+        const double r[3] = {p[0] - center[0], p[1] - center[1], p[2] - center[2]};
         const double cr[3] = {alpha[1] * r[2] - alpha[2] * r[1], alpha[2] * r[0] - alpha[0] * r[2],
                               alpha[0] * r[1] - alpha[1] * r[0]};
         double f[3];
-        for (int q = 0; q < 3; ++q) {
-            f[q] = w.force[q] * share + cr[q] * m;
-            sr[q][j] = r[q];
-            sf[q][j] = f[q];
-        }
+        for (int q = 0; q < 3; ++q) f[q] = w.force[q] * share + cr[q] * m;
         const R fx = R(f[0]), fy = R(f[1]), fz = R(f[2]);
         if (!isfinite(f[0]) || !isfinite(f[1]) || !isfinite(f[2]) || !isfinite(fx) || !isfinite(fy) || !isfinite(fz))
             bad = 1;
@@ -909,19 +1008,14 @@ __device__ __forceinline__ void wrenchSpread(const Dev<R> &L, const WrenchDev *w
             L.ext_req[3 * static_cast<std::size_t>(i) + 1] = f[1];
             L.ext_req[3 * static_cast<std::size_t>(i) + 2] = f[2];
         }
-    }, [&](unsigned m) {
-        if (t >= 8) return;
-        for (unsigned j = 0; j < m; ++j) {
-            const double r[3] = {sr[0][j], sr[1][j], sr[2][j]}, f[3] = {sf[0][j], sf[1][j], sf[2][j]};
-            const double mo[3] = {r[1] * f[2] - r[2] * f[1], r[2] * f[0] - r[0] * f[2], r[0] * f[1] - r[1] * f[0]};
-            if (t < 3) part = part + f[t];
-            else if (t < 6) part = part + mo[t - 3];
-            else if (t == 6) part += normD(f[0], f[1], f[2]);
-            else part += normD(mo[0], mo[1], mo[2]);
+        const double mo[3] = {r[1] * f[2] - r[2] * f[1], r[2] * f[0] - r[0] * f[2], r[0] * f[1] - r[1] * f[0]};
+        for (int q = 0; q < 3; ++q) {
+            terms[q][j] = f[q];
+            terms[3 + q][j] = mo[q];
         }
+        terms[6][j] = normD(f[0], f[1], f[2]);
+        terms[7][j] = normD(mo[0], mo[1], mo[2]);
     });
-    if (t < 8) sums[t] = part;
-    __syncthreads();
     if (t == 0) {
         for (int q = 0; q < 8; ++q)
             if (!isfinite(sums[q])) bad = 1;
@@ -2452,10 +2546,9 @@ __global__ void __launch_bounds__(kEmitThreads) kEmitEvents(const Grid<R> launch
 // kinetic energy, each node's term formed in backend precision and widened,
 // folded serially in node order as the reference folds it, so the audit
 // ledgers match the reference's bit for bit. The CTA forms the next chunk of
-// terms in shared memory while thread 0 folds the current one; the fold is
-// one chain of dependent FP64 adds (N of them), so the kernel is bound by FP64
-// add latency. kAuditMark keeps the energy before a phase; the other modes
-// charge the drop across the phase to the striker or the damping ledger.
+// terms in shared memory while warp 0 folds the current one (foldSerial).
+// kAuditMark keeps the energy before a phase; the other modes charge the drop
+// across the phase to the striker or the damping ledger.
 // ---------------------------------------------------------------------------
 constexpr unsigned kFoldThreads = 1024;
 constexpr int kAuditMark = 0, kAuditStriker = 1, kAuditDamping = 2;
@@ -2470,7 +2563,7 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
     __shared__ double terms[2][kFoldThreads];
     double total = 0.0;
     unsigned buf = 0;
-    // Thread 0 reaches the barrier of chunk k+1 only after folding chunk k,
+    // Warp 0 reaches the barrier of chunk k+1 only after folding chunk k,
     // so chunk k+2 never overwrites a buffer still being read.
     for (std::uint32_t base = 0; base < L.N; base += kFoldThreads, buf ^= 1U) {
         const std::uint32_t i = base + threadIdx.x;
@@ -2480,11 +2573,7 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
             terms[buf][threadIdx.x] = static_cast<double>(R(0.5) * q.w * dot(v, v));
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const std::uint32_t n = L.N - base < kFoldThreads ? L.N - base : kFoldThreads;
-#pragma unroll 8
-            for (std::uint32_t k = 0; k < n; ++k) total += terms[buf][k];
-        }
+        if (threadIdx.x < 32) total = foldSerial(total, terms[buf], L.N - base < kFoldThreads ? L.N - base : kFoldThreads);
     }
     if (threadIdx.x != 0) return;
     if (mode == kAuditMark) c.ke_mark = total;
@@ -2496,23 +2585,18 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
 // The external-load ledger of a substep (ExternalLoads.hpp:126-140): thirteen
 // independent serial folds over the loaded nodes in list order -- impulse,
 // angular impulse, work, requested impulse and requested angular impulse, per
-// component -- then added to the run's ledger. Lane q of warp 0 runs fold q,
-// so the thirteen chains advance together and each keeps the reference's
-// order; the other warps stage the next chunk of node contributions into
-// shared memory meanwhile. The wrench sources' node runs tile the list in
-// source order, so the same pass folds each source's own change and hands it
-// to its ledger when its run ends.
+// component -- then added to the run's ledger. The wrench sources' node runs
+// tile the list in source order, so the same pass folds each source's own
+// change and hands it to its ledger when its run ends.
 //
-// A fold is a chain of dependent FP64 adds, one per loaded node, so its
-// length sets its time (GB300's FP64 add latency is long). Nothing in the
-// substep reads the ledger before the exit rules at its end, so the kernel
-// runs on a stream of its own from the kick, whose contributions it reads,
-// beside the contact passes, the sweep and the end sample.
+// Nothing in the substep reads the ledger before the exit rules at its end, so
+// the kernel runs on a stream of its own from the kick, whose contributions it
+// reads, beside the contact passes, the sweep and the end sample.
 // ---------------------------------------------------------------------------
 constexpr int kLedgerFolds = 13;
-constexpr unsigned kLedgerThreads = 128;                   // one folding lane, three staging warps
+constexpr unsigned kLedgerThreads = 128;                   // one folding warp, three staging ones
 constexpr unsigned kLedgerStagers = kLedgerThreads - 32;
-constexpr unsigned kLedgerChunk = 384;                      // entries staged per round
+constexpr unsigned kLedgerChunk = 768;                      // entries staged per round
 
 // Adds a source's folded change (component q) to its ledger.
 __device__ __forceinline__ void addLoadComponent(LoadLedger &g, int q, double x) {
@@ -2523,12 +2607,10 @@ __device__ __forceinline__ void addLoadComponent(LoadLedger &g, int q, double x)
     else g.req_ang[q - 10] = g.req_ang[q - 10] + x;
 }
 
-// One CTA per (lattice, component): blockIdx.y is the component q. Thread 0
-// folds it; the other warps stage the next chunk of its node contributions.
-// Each fold is one chain of dependent FP64 adds, and GB300 has little FP64
-// issue per SM, so the thirteen chains run on thirteen SMs (measured, 1,984
-// loaded nodes: 246 us with the chains on thirteen warps of one CTA, 182 us
-// on thirteen lanes of one warp).
+// One CTA per (lattice, component): blockIdx.y is the component q. Warp 0
+// folds it (foldSerial; the chain of 1,984 dependent FP64 adds it stands for
+// took 75 us); the other warps stage the next chunk of its node
+// contributions.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> launch, Settings<R> S) {
     startAfterPrevious();
@@ -2541,7 +2623,6 @@ __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> laun
     if (!(c.ext_count && c.loads_remaining > 0)) return;
     __shared__ double stage[2][kLedgerChunk];
     const int q = static_cast<int>(blockIdx.y);
-    const bool folder = threadIdx.x == 0;
     const bool stager = threadIdx.x >= 32;
     const std::uint32_t n = c.ext_count;
     const unsigned sources = c.wrench_count;
@@ -2561,46 +2642,42 @@ __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> laun
     double run = 0.0;
     const auto flush = [&](std::uint32_t at) {
         while (k < sources && L.wrench[k].end == at) {
-            SourceSlot &slot = L.sources[L.wrench[k].slot];
-            addLoadComponent(slot.load, q, run);
-            if (q == 0) {
-                if (slot.load.steps == 0) slot.order = c.source_seq++;
-                slot.load.steps += 1;
-                slot.load.elapsed = slot.load.elapsed + static_cast<double>(S.dt);
+            if (threadIdx.x == 0) {
+                SourceSlot &slot = L.sources[L.wrench[k].slot];
+                addLoadComponent(slot.load, q, run);
+                if (q == 0) {
+                    if (slot.load.steps == 0) slot.order = c.source_seq++;
+                    slot.load.steps += 1;
+                    slot.load.elapsed = slot.load.elapsed + static_cast<double>(S.dt);
+                }
             }
             run = 0.0;
             ++k;
         }
     };
     if (stager) fill(0, 0);
-    if (folder) flush(0);
+    else flush(0);
     __syncthreads();
     double total = 0.0;
     unsigned buf = 0;
     for (std::uint32_t base = 0; base < n; base += kLedgerChunk, buf ^= 1U) {
         if (stager) {
             if (base + kLedgerChunk < n) fill(base + kLedgerChunk, buf ^ 1U);
-        } else if (folder) {
+        } else {
             const std::uint32_t cnt = n - base < kLedgerChunk ? n - base : kLedgerChunk;
             const double *col = stage[buf];
-            if (sources == 0) {
-                // Unrolled so the shared-memory loads run ahead of the
-                // dependent adds.
-#pragma unroll 8
-                for (std::uint32_t e = 0; e < cnt; ++e) total += col[e];
-            } else {
-                for (std::uint32_t e = 0; e < cnt; ++e) {
-                    const double x = col[e];
-                    total += x;
-                    run += x;
-                    flush(base + e + 1);
-                }
+            total = foldSerial(total, col, cnt);
+            for (std::uint32_t e = 0; k < sources && e < cnt;) {
+                const std::uint32_t end = L.wrench[k].end - base;
+                const std::uint32_t upto = end < cnt ? end : cnt;
+                run = foldSerial(run, col + e, upto - e);
+                e = upto;
+                flush(base + e);
             }
         }
         __syncthreads();
     }
-    if (folder) {
-        flush(n); // only sources with empty runs past the list's end remain
+    if (threadIdx.x == 0) {
         LoadLedger &g = c.ext;
         addLoadComponent(g, q, total);
         if (q == 0) {
