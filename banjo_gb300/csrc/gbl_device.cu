@@ -21,6 +21,7 @@
 #include <cstring>
 #include <deque>
 #include <functional>
+#include <iterator>
 #include <limits>
 #include <map>
 #include <memory>
@@ -461,6 +462,49 @@ template <class F> void parallelFor(std::size_t n, F &&f, std::size_t grain = st
     f(std::size_t(0), n / T);
     for (auto &th : pool) th.join();
     returnHelpers(T - 1);
+}
+
+// Whether a download of `bytes` has the device write the caller's arrays in
+// place (where it reaches pageable memory) rather than through a device buffer,
+// the pinned slices and host threads: the slices' stream, events and threads
+// cost more than a small lattice's bytes (0.1 MB: 27 us in place, 167 through
+// the slices; 11 MB: 138 and 525; 109 MB: 1,130 and 2,119), and from 268 MB on
+// the slices are as fast (3.9 and 4.1 ms).
+constexpr std::size_t kInPlaceOutMaxBytes = std::size_t(128) << 20;
+bool downloadInPlace(std::size_t bytes) {
+    static const bool chosen = std::getenv("GBL_HOST_COPY") != nullptr; // the copies' way is fixed: they are made
+    return !chosen && deviceReadsPageable() && bytes < kInPlaceOutMaxBytes;
+}
+
+// Makes the pages of a download's arrays present and writable from the host, a
+// byte a page rewritten with itself: a page the device touched first would
+// cost a fault across the link. Pages that turn out to be new (a fault each)
+// are shared over host threads, which present ones are not worth starting.
+void touchPages(const std::pair<void *, std::size_t> *arrays, std::size_t count) {
+    constexpr std::size_t kPage = 4096, kBlock = 64;
+    auto touch = [](char *p, std::size_t bytes, std::size_t first, std::size_t last) {
+        for (std::size_t k = first; k < last; ++k) {
+            volatile char *at = p + std::min(k * kPage, bytes - 1);
+            *at = *at;
+        }
+    };
+    bool fresh = false;
+    for (std::size_t a = 0; a < count; ++a) {
+        char *p = static_cast<char *>(arrays[a].first);
+        const std::size_t bytes = arrays[a].second;
+        if (!bytes) continue;
+        const std::size_t pages = (bytes - 1) / kPage + 2; // the last byte's page included
+        std::size_t done = 0;
+        while (done < pages && !fresh) {
+            const std::size_t upto = std::min(pages, done + kBlock);
+            const auto t0 = std::chrono::steady_clock::now();
+            touch(p, bytes, done, upto);
+            fresh = std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(15);
+            done = upto;
+        }
+        if (done < pages)
+            parallelFor(pages - done, [&](std::size_t lo, std::size_t hi) { touch(p, bytes, done + lo, done + hi); }, 4 * kBlock);
+    }
 }
 
 } // namespace
@@ -1422,16 +1466,39 @@ template <class R> struct Resident {
         return out;
     }
 
+    // The caller's arrays written by the device in place.
+    void writeInPlace(gbl_state_view &st, cudaStream_t stream) const {
+        const std::size_t n3 = 3 * static_cast<std::size_t>(N) * sizeof(double), b = B;
+        const std::pair<void *, std::size_t> arrays[] = {
+            {st.u, n3}, {st.u_prev, n3}, {st.v, n3}, {st.alive, b}, {st.failure_mode, b}, {st.damage, 8 * b},
+            {st.prev_tensile, 8 * b}, {st.prev_compressive, 8 * b}, {st.prev_shear, 8 * b},
+            {st.plastic_extension, 8 * b}, {st.plastic_strain, 8 * b}};
+        touchPages(arrays, std::size(arrays));
+        if (N) kNodesOut<R><<<reorderGrid(N), kThreads, 0, stream>>>(st.u, st.u_prev, st.v, dev.u, dev.up, dev.v, N);
+        if (B)
+            kBondsOut<R><<<reorderGrid(B), kThreads, 0, stream>>>(
+                BondsOut{st.alive, st.failure_mode, st.damage, st.prev_tensile, st.prev_compressive, st.prev_shear,
+                         st.plastic_extension, st.plastic_strain},
+                bonds(), dev.dev2sched, B);
+        check(cudaGetLastError(), "kernel launch");
+        check(cudaStreamSynchronize(stream), "download");
+    }
+
     // download (WorkingLattice::toState, LatticeWorking.hpp:126-142): the
-    // device writes the state's layout, copied straight into the caller's
-    // arrays (which the caller has already touched).
+    // device writes the state's layout into the caller's arrays, in place or
+    // through a buffer of its own.
     void download(gbl_state_view &st, gbl_sphere *sphere, cudaStream_t stream) {
         if (st.node_count != N || st.bond_count != B) invalid("download state does not match the lattice");
-        const StateOut out = stateOut(stream);
-        check(cudaStreamSynchronize(stream), "download");
-        out.copyTo(st);
-        check(cudaFreeAsync(out.base, stream), "device free");
-        check(cudaStreamSynchronize(stream), "download");
+        const std::size_t bytes = static_cast<std::size_t>(N) * 72 + static_cast<std::size_t>(B) * 50;
+        if (downloadInPlace(bytes)) {
+            writeInPlace(st, stream);
+        } else {
+            const StateOut out = stateOut(stream);
+            check(cudaStreamSynchronize(stream), "download");
+            out.copyTo(st);
+            check(cudaFreeAsync(out.base, stream), "device free");
+            check(cudaStreamSynchronize(stream), "download");
+        }
         if (sphere) *sphere = fetchSphere();
     }
 
