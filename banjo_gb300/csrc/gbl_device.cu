@@ -2372,6 +2372,7 @@ private:
         blocks_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.dev.tiles_b / kScanBlock + 1; }, 1);
         each_ = span([](const Res &, U &b, U &e) { b = 0; e = 1; }, 1);
         slabs_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.sched.block_count; }, 1);
+        owners_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.nc_mem ? l.N : 0U; }, kGatherOwners);
         buckets_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.nc_mem ? l.dev.nc_mask + 1U : 0U; }, kThreads);
         // The lattices swept staged, or whole in one CTA each where the shape
         // says so, largest first; the level launches and the isolated-node
@@ -2754,9 +2755,9 @@ private:
         if (buckets_.count) next(kContactBuckets<R, M>, buckets_.count, kThreads, 0, st, grid(buckets_));
         if (nodes_.count) next(kContactScatter<R, M>, nodes_.count, kThreads, 0, st, grid(nodes_));
         if (buckets_.count) next(kContactSort<R, M>, buckets_.count, kThreads, 0, st, grid(buckets_));
-        if (nodes_.count) next(kContactGather<R, M, false>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
+        if (owners_.count) next(kContactGather<R, M, false>, owners_.count, kThreads, 0, st, grid(owners_), S);
         next(kContactTiles<R, M>, each_.count, kContactScanThreads, 0, st, grid(each_));
-        if (nodes_.count) next(kContactGather<R, M, true>, nodes_.count, kThreads, 0, st, grid(nodes_), S);
+        if (owners_.count) next(kContactGather<R, M, true>, owners_.count, kThreads, 0, st, grid(owners_), S);
         mark(14);
         next(kContactNarrow<R, M>, each_.count, 32, 0, st, grid(each_), S);
         mark(15);
@@ -2826,7 +2827,7 @@ private:
     unsigned *running_{}, *running_host_{};
     Dev<R> *table_{};
     Work *work_{};
-    Span nodes_{}, bonds_{}, restart_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, whole_{}, buckets_{},
+    Span nodes_{}, bonds_{}, restart_{}, tiles_{}, blocks_{}, each_{}, slabs_{}, whole_{}, owners_{}, buckets_{},
         wrench_{};
     unsigned staged_threads_{0}; // the staged sweep's CTA size (0: the lattices do not sweep staged)
     std::size_t staged_smem_{0};

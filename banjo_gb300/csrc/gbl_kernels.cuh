@@ -2849,6 +2849,7 @@ __global__ void __launch_bounds__(kThreads) kContactCells(const Grid<R> launch, 
     const std::uint32_t b = cellBucket(x, y, z, L.nc_mask);
     L.nc_cell[i] = make_int4(x, y, z, static_cast<int>(b));
     L.nc_built[i] = L.u[i];
+    if (i % kThreads == 0) L.nc_tile[i / kThreads] = 0U; // the gather adds to it
     if (!(L.v[i].w <= R(0))) atomicAdd(&L.nc_count[b], 1U);
 }
 
@@ -2909,78 +2910,119 @@ __global__ void __launch_bounds__(kThreads) kContactSort(const Grid<R> launch) {
     }
 }
 
-// Rebuild, step 5 (nodeContactGather, node items; tile = the item's 256
-// nodes). Count pass: each owner's pairs and the tile's total, and the pairs
-// that did not fit. Write pass: the pairs at the owner's place in the list.
+// Rebuild, step 5 (nodeContactGather; a tile is 256 nodes). Count pass: each
+// owner's pairs and the tile's total, and the pairs that did not fit. Write
+// pass: the pairs at the owner's place in the list. One warp per owner, a lane
+// per cell: the 27 cells' chains of loads (bucket, members, cell, position,
+// the owner's bonds) run side by side, and a scan over the lanes puts the
+// pairs in cell order. (One thread walked them all: the broad phase of the
+// 24x10x18 cracking box took 220 us a substep, 40 now.)
+constexpr unsigned kGatherOwners = kThreads / 32; // per CTA
+constexpr unsigned kGatherSlots = 32;             // an owner's bonds kept in shared memory
 template <class R, bool Many, bool Write>
 __global__ void __launch_bounds__(kThreads) kContactGather(const Grid<R> launch, Settings<R> S) {
     startAfterPrevious();
-    __shared__ unsigned buf[kThreads];
     const Work w = item<Many>(launch);
-    const Dev<R> L = descriptor<R, Many>(launch, w);
+    __shared__ SharedDesc<R> desc;
+    __shared__ std::uint32_t others[kGatherOwners][kGatherSlots], bonds[kGatherOwners][kGatherSlots];
+    __shared__ bool lives[kGatherOwners][kGatherSlots];
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     Ctl &c = *L.ctl;
     if (c.stop || !c.nc_rebuild) return;
-    const std::uint32_t i = w.begin + threadIdx.x;
-    const bool in = i < w.end;
-    const std::uint32_t tile = w.begin / kThreads;
-    std::uint32_t at = 0;
-    if (Write) {
-        unsigned total = 0;
-        at = L.nc_tile[tile] + blockExclusiveScanU(in ? L.nc_fill[i] : 0U, buf, total);
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    const std::uint32_t i = w.begin + warp; // items: up to kGatherOwners nodes of one tile
+    if (i >= w.end) return;
+    const std::uint32_t tile = i / kThreads;
+    if (L.v[i].w <= R(0)) { // not movable: no pairs of its own
+        if (!Write && lane == 0) L.nc_fill[i] = 0U;
+        return;
     }
-    std::uint32_t fill = 0, overflow = 0;
-    if (in && !(L.v[i].w <= R(0))) {
-        const std::size_t N = L.N;
-        const R cutoff = contactCutoff(S);
-        const R cutoff_sq = cutoff * cutoff;
-        const V3<R> p = pos(L, i);
-        const int4 home = L.nc_cell[i];
-        for (int dz = -1; dz <= 1; ++dz)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int gx = home.x + dx, gy = home.y + dy, gz = home.z + dz;
-                    const std::uint32_t b = cellBucket(gx, gy, gz, L.nc_mask);
-                    const std::uint32_t first = L.nc_start[b], n = L.nc_count[b];
-                    for (std::uint32_t k = 0; k < n; ++k) {
-                        const std::uint32_t j = L.nc_members[first + k];
-                        if (j <= i) continue;
-                        const int4 cj = L.nc_cell[j];
-                        if (cj.x != gx || cj.y != gy || cj.z != gz) continue;
-                        const V3<R> r = pos(L, j) - p;
-                        if (dot(r, r) > cutoff_sq) continue;
-                        // The pair's bond, if the owner lists one to j; a live one holds the pair.
-                        std::uint32_t bond = kNoBond;
-                        bool held = false;
-                        for (std::uint32_t s = 0; s < L.D; ++s) {
-                            const std::size_t slot = s * N + i;
-                            const std::uint32_t bs = L.nbr_bond[slot];
-                            if (bs == kNoBond) break;
-                            if (L.nbr_other[slot] != j) continue;
-                            bond = bs;
-                            held = !signbit(L.nbr[slot].w);
-                            break;
-                        }
-                        if (held) continue;
-                        if (fill == kPairsPerNode) {
-                            ++overflow;
-                            continue;
-                        }
-                        if (Write) {
-                            L.nc_pa[at + fill] = i;
-                            L.nc_pb[at + fill] = j;
-                            L.nc_pbond[at + fill] = bond;
-                        }
-                        ++fill;
-                    }
-                }
+    const std::size_t N = L.N;
+    // The owner's bonds, in slot order up to the first padded slot.
+    const std::uint32_t kept = L.D < kGatherSlots ? L.D : kGatherSlots;
+    std::uint32_t bs = kNoBond;
+    if (lane < kept) {
+        const std::size_t slot = lane * N + i;
+        bs = L.nbr_bond[slot];
+        others[warp][lane] = L.nbr_other[slot];
+        bonds[warp][lane] = bs;
+        lives[warp][lane] = !signbit(L.nbr[slot].w);
     }
+    const unsigned padded = __ballot_sync(0xffffffffU, bs == kNoBond);
+    const std::uint32_t listed = padded ? static_cast<std::uint32_t>(__ffs(padded) - 1) : 32U;
+    __syncwarp();
+    // The owner's bond to j, if it lists one; whether that bond is alive.
+    auto bondTo = [&](std::uint32_t j, std::uint32_t &bond) {
+        for (std::uint32_t s = 0; s < listed; ++s)
+            if (others[warp][s] == j) {
+                bond = bonds[warp][s];
+                return lives[warp][s];
+            }
+        for (std::uint32_t s = kGatherSlots; listed == kGatherSlots && s < L.D; ++s) {
+            const std::size_t slot = s * N + i;
+            const std::uint32_t far = L.nbr_bond[slot];
+            if (far == kNoBond) break;
+            if (L.nbr_other[slot] != j) continue;
+            bond = far;
+            return !signbit(L.nbr[slot].w);
+        }
+        return false;
+    };
+    const R cutoff = contactCutoff(S);
+    const R cutoff_sq = cutoff * cutoff;
+    const V3<R> p = pos(L, i);
+    const int4 home = L.nc_cell[i];
+    const int gx = home.x + static_cast<int>(lane % 3) - 1, gy = home.y + static_cast<int>(lane / 3 % 3) - 1,
+              gz = home.z + static_cast<int>(lane / 9) - 1;
+    std::uint32_t first = 0, members = 0;
+    if (lane < 27) {
+        const std::uint32_t b = cellBucket(gx, gy, gz, L.nc_mask);
+        first = L.nc_start[b];
+        members = L.nc_count[b];
+    }
+    // The cell's pairs in member order: take(j, bond).
+    auto pairs = [&](auto &&take) {
+        for (std::uint32_t k = 0; k < members; ++k) {
+            const std::uint32_t j = L.nc_members[first + k];
+            if (j <= i) continue;
+            const int4 cj = L.nc_cell[j];
+            if (cj.x != gx || cj.y != gy || cj.z != gz) continue;
+            const V3<R> r = pos(L, j) - p;
+            if (dot(r, r) > cutoff_sq) continue;
+            std::uint32_t bond = kNoBond;
+            if (bondTo(j, bond)) continue; // a live bond holds the pair
+            take(j, bond);
+        }
+    };
+    std::uint32_t mine = 0;
+    pairs([&](std::uint32_t, std::uint32_t) { ++mine; });
+    const std::uint32_t upto = warpInclusive(mine);
+    const std::uint32_t total = __shfl_sync(0xffffffffU, upto, 31);
+    const std::uint32_t fill = total < kPairsPerNode ? total : kPairsPerNode;
     if (!Write) {
-        if (in) L.nc_fill[i] = fill;
-        unsigned total = 0;
-        blockExclusiveScanU(fill, buf, total);
-        if (threadIdx.x == 0) L.nc_tile[tile] = total;
-        if (overflow) atomicAdd(&c.node.pair_overflow, static_cast<unsigned long long>(overflow));
+        if (lane == 0) {
+            L.nc_fill[i] = fill;
+            if (fill) atomicAdd(&L.nc_tile[tile], fill);
+            if (total > fill) atomicAdd(&c.node.pair_overflow, static_cast<unsigned long long>(total - fill));
+        }
+        return;
     }
+    if (total == 0) return;
+    // The owner's place: its tile's first pair and the pairs of the tile's
+    // nodes before it.
+    std::uint32_t before = 0;
+    for (std::uint32_t q = tile * kThreads + lane; q < i; q += 32) before += L.nc_fill[q];
+    before = __reduce_add_sync(0xffffffffU, before);
+    std::uint32_t rank = upto - mine;
+    const std::uint32_t at = L.nc_tile[tile] + before;
+    pairs([&](std::uint32_t j, std::uint32_t bond) {
+        if (rank < kPairsPerNode) {
+            L.nc_pa[at + rank] = i;
+            L.nc_pb[at + rank] = j;
+            L.nc_pbond[at + rank] = bond;
+        }
+        ++rank;
+    });
 }
 
 // Rebuild, step 6 (one CTA per lattice): the tiles' first pairs in node order,
@@ -3008,6 +3050,62 @@ __global__ void __launch_bounds__(kContactScanThreads) kContactTiles(const Grid<
     }
 }
 
+// One pair against the current state (nodeContactPair, LatticePhysics.hpp:
+// 1441-1647): its gap, whether it responds, and the velocities after it.
+template <class R> struct PairResponse {
+    bool tested, acts, impulse_on;
+    R gap, ia, ib; // 1 / mass of the two nodes, once past the contact gate
+    V3<R> n, va, vb;
+    R lost;            // kinetic energy before minus after
+    V3<R> momentum;    // what rounding left of the pair's momentum change
+};
+template <class R, class M>
+__device__ __forceinline__ PairResponse<R> pairResponse(M &m, const Settings<R> &S, bool respond, V3<R> r, const Q4<R> &qa,
+                                                        const Q4<R> &qb) {
+    PairResponse<R> o{};
+    const R ma = qa.w, mb = qb.w;
+    const R distance = m.root(dot(r, r));
+    o.n = distance > R(1.0e-12) ? m.div(r, distance) : mk<R>(1, 0, 0); // normalized(r)
+    o.gap = distance - R(2) * S.nc_radius;
+    o.va = xyz(qa);
+    o.vb = xyz(qb);
+    if (!respond) return o;
+    const R vn = dot(o.vb - o.va, o.n);
+    if (o.gap > maxR(S.nc_margin, -vn * S.dt)) return o;
+    o.ia = m.div(R(1), ma);
+    o.ib = m.div(R(1), mb);
+    const R pair_inverse = o.ia + o.ib;
+    const R restitution = -vn > S.nc_threshold ? S.nc_restitution : R(0);
+    const R desired = o.gap > S.nc_margin ? m.div(-o.gap, S.dt) : -restitution * minR(vn, R(0));
+    const R impulse = maxR(R(0), m.div(desired - vn, pair_inverse));
+    o.impulse_on = impulse > R(0);
+    o.acts = o.impulse_on || o.gap < -S.nc_margin;
+    if (!o.impulse_on) return o;
+    const V3<R> va0 = o.va, vb0 = o.vb;
+    const R before = R(0.5) * ma * dot(va0, va0) + R(0.5) * mb * dot(vb0, vb0);
+    const V3<R> j = impulse * o.n;
+    o.vb = o.vb + o.ib * j;
+    o.va = o.va - o.ia * j;
+    const V3<R> rel = o.vb - o.va;
+    const V3<R> t = rel - dot(rel, o.n) * o.n;
+    const R sq = dot(t, t);
+    if (!(sq < R(0x1p-80))) { // below, the speed is under 1e-12 whatever its root's rounding
+        const R speed = m.root(sq);
+        if (speed > R(1.0e-12)) {
+            const V3<R> dir = m.div(t, speed);
+            const R stick = m.div(speed, pair_inverse);
+            const R friction = stick <= S.nc_static * impulse ? stick : minR(stick, S.nc_dynamic * impulse);
+            const V3<R> f = -friction * dir;
+            o.vb = o.vb + o.ib * f;
+            o.va = o.va - o.ia * f;
+        }
+    }
+    o.lost = before - (R(0.5) * ma * dot(o.va, o.va) + R(0.5) * mb * dot(o.vb, o.vb));
+    o.momentum = {ma * (o.va.x - va0.x) + mb * (o.vb.x - vb0.x), ma * (o.va.y - va0.y) + mb * (o.vb.y - vb0.y),
+                  ma * (o.va.z - va0.z) + mb * (o.vb.z - vb0.z)};
+    return o;
+}
+
 // The narrow phase (nodeContactPass and nodeContactPair), one warp per lattice.
 // The lanes evaluate the next 32 pairs of the list against the current state
 // at once; the first pair whose response changes a velocity or a position is
@@ -3031,105 +3129,81 @@ __global__ void __launch_bounds__(32) kContactNarrow(const Grid<R> launch, Setti
     const std::uint32_t count = c.nc_pairs;
     NodeAcc acc = c.node;
     const bool respond = S.nc_mode == 2U;
+    // The records only ever hold a widened R; the four FP64 sums are lanes 0
+    // to 3's, one each.
+    R deepest = R(0), largest = R(0);
+    double sum = lane == 0 ? acc.dissipated : lane < 4 ? acc.momentum[lane - 1] : 0.0;
     for (std::uint32_t at = 0; at < count;) {
         const std::uint32_t q = at + lane;
-        bool tested = false, acts = false, impulse_on = false;
+        PairResponse<R> o{};
         std::uint32_t a = 0, b = 0;
-        R gap = R(0), ma = R(0), mb = R(0), impulse = R(0), pair_inverse = R(0), ia = R(0), ib = R(0);
-        V3<R> n{}, va{}, vb{};
+        Q4<R> qa{}, qb{};
         if (q < count) {
             a = L.nc_pa[q];
             b = L.nc_pb[q];
             const std::uint32_t bond = L.nc_pbond[q];
-            const Q4<R> qa = L.v[a], qb = L.v[b];
-            ma = qa.w;
-            mb = qb.w;
+            qa = L.v[a];
+            qb = L.v[b];
             const bool held = bond != kNoBond && !(L.rec[bond].a & kDeadBit);
-            if (!held && !(ma <= R(0) || mb <= R(0))) {
-                tested = true;
+            if (!held && !(qa.w <= R(0) || qb.w <= R(0))) {
                 const V3<R> r = pos(L, b) - pos(L, a);
-                const R distance = length(r);
-                n = normalized(r);
-                gap = distance - R(2) * S.nc_radius;
-                if (respond) {
-                    va = xyz(qa);
-                    vb = xyz(qb);
-                    const R vn = dot(vb - va, n);
-                    if (!(gap > maxR(S.nc_margin, -vn * S.dt))) {
-                        ia = R(1) / ma;
-                        ib = R(1) / mb;
-                        pair_inverse = ia + ib;
-                        const R restitution = -vn > S.nc_threshold ? S.nc_restitution : R(0);
-                        const R desired = gap > S.nc_margin ? -gap / S.dt : -restitution * minR(vn, R(0));
-                        impulse = maxR(R(0), (desired - vn) / pair_inverse);
-                        impulse_on = impulse > R(0);
-                        acts = impulse_on || gap < -S.nc_margin;
+                if constexpr (std::is_same<R, float>::value) {
+                    QuickMath quick;
+                    o = pairResponse<R>(quick, S, respond, r, qa, qb);
+                    if (!quick.good) {
+                        PlainMath<R> plain;
+                        o = pairResponse<R>(plain, S, respond, r, qa, qb);
                     }
+                } else {
+                    PlainMath<R> plain;
+                    o = pairResponse<R>(plain, S, respond, r, qa, qb);
                 }
+                o.tested = true;
             }
         }
-        const unsigned acting = __ballot_sync(kAll, acts);
+        const unsigned acting = __ballot_sync(kAll, o.acts);
         const unsigned first = acting ? static_cast<unsigned>(__ffs(acting)) - 1U : 32U;
-        const bool counted = tested && lane <= first;
+        const bool counted = o.tested && lane <= first;
         acc.pair_tests += static_cast<unsigned long long>(__popc(__ballot_sync(kAll, counted)));
-        // The deepest overlap among the counted pairs (a running maximum of
-        // the same values, so the order of the lanes does not matter).
-        R deepest = counted && gap < R(0) ? -gap : R(0);
-        for (int o = 16; o > 0; o >>= 1) deepest = maxR(deepest, __shfl_xor_sync(kAll, deepest, o));
-        if (deepest > static_cast<R>(acc.max_overlap)) acc.max_overlap = static_cast<double>(deepest);
+        if (counted && -o.gap > deepest) deepest = -o.gap;
         if (first == 32U) {
             at += 32;
             continue;
         }
-        double dissipated = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
-        R correction = R(0);
         if (lane == first) {
-            if (impulse_on) {
-                const V3<R> va0 = va, vb0 = vb;
-                const R before = R(0.5) * ma * dot(va, va) + R(0.5) * mb * dot(vb, vb);
-                const V3<R> j = impulse * n;
-                vb = vb + ib * j;
-                va = va - ia * j;
-                const V3<R> rel = vb - va;
-                const V3<R> t = rel - dot(rel, n) * n;
-                const R speed = length(t);
-                if (speed > R(1.0e-12)) {
-                    const V3<R> dir = t / speed;
-                    const R stick = speed / pair_inverse;
-                    const R friction = stick <= S.nc_static * impulse ? stick : minR(stick, S.nc_dynamic * impulse);
-                    const V3<R> f = -friction * dir;
-                    vb = vb + ib * f;
-                    va = va - ia * f;
-                }
-                L.v[a] = Q4<R>{va.x, va.y, va.z, ma};
-                L.v[b] = Q4<R>{vb.x, vb.y, vb.z, mb};
-                dissipated = static_cast<double>(before - (R(0.5) * ma * dot(va, va) + R(0.5) * mb * dot(vb, vb)));
-                mx = static_cast<double>(ma * (va.x - va0.x) + mb * (vb.x - vb0.x));
-                my = static_cast<double>(ma * (va.y - va0.y) + mb * (vb.y - vb0.y));
-                mz = static_cast<double>(ma * (va.z - va0.z) + mb * (vb.z - vb0.z));
+            if (o.impulse_on) {
+                L.v[a] = Q4<R>{o.va.x, o.va.y, o.va.z, qa.w};
+                L.v[b] = Q4<R>{o.vb.x, o.vb.y, o.vb.z, qb.w};
             }
-            if (gap < -S.nc_margin) {
-                correction = minR(-gap - S.nc_margin, R(0.2) * S.nc_radius);
-                const V3<R> shift = (correction / pair_inverse) * n;
+            if (o.gap < -S.nc_margin) {
+                const R correction = minR(-o.gap - S.nc_margin, R(0.2) * S.nc_radius);
+                const V3<R> shift = (correction / (o.ia + o.ib)) * o.n;
                 const Q4<R> ua = L.u[a], ub = L.u[b];
-                const V3<R> na = xyz(ua) - ia * shift, nb = xyz(ub) + ib * shift;
+                const V3<R> na = xyz(ua) - o.ia * shift, nb = xyz(ub) + o.ib * shift;
                 L.u[a] = Q4<R>{na.x, na.y, na.z, ua.w};
                 L.u[b] = Q4<R>{nb.x, nb.y, nb.z, ub.w};
+                if (correction > largest) largest = correction;
             }
         }
-        // The applied pair's sums, folded in list order on every lane.
-        if (__shfl_sync(kAll, impulse_on, first)) {
-            acc.dissipated += __shfl_sync(kAll, dissipated, first);
-            acc.momentum[0] += __shfl_sync(kAll, mx, first);
-            acc.momentum[1] += __shfl_sync(kAll, my, first);
-            acc.momentum[2] += __shfl_sync(kAll, mz, first);
+        // The applied pair's sums, folded in list order.
+        const int src = static_cast<int>(first);
+        if (__ballot_sync(kAll, lane == first && o.impulse_on)) {
+            const R x0 = __shfl_sync(kAll, o.lost, src), x1 = __shfl_sync(kAll, o.momentum.x, src);
+            const R x2 = __shfl_sync(kAll, o.momentum.y, src), x3 = __shfl_sync(kAll, o.momentum.z, src);
+            if (lane < 4) sum += static_cast<double>(lane == 0 ? x0 : lane == 1 ? x1 : lane == 2 ? x2 : x3);
             ++acc.contacts;
         }
-        correction = __shfl_sync(kAll, correction, first);
-        if (correction > static_cast<R>(acc.max_correction)) acc.max_correction = static_cast<double>(correction);
         __syncwarp(); // the applied pair's writes, before the next window reads
         at += first + 1U;
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        deepest = maxR(deepest, __shfl_xor_sync(kAll, deepest, o));
+        largest = maxR(largest, __shfl_xor_sync(kAll, largest, o));
+    }
+    if (deepest > static_cast<R>(acc.max_overlap)) acc.max_overlap = static_cast<double>(deepest);
+    if (largest > static_cast<R>(acc.max_correction)) acc.max_correction = static_cast<double>(largest);
+    acc.dissipated = __shfl_sync(kAll, sum, 0);
+    for (int q = 0; q < 3; ++q) acc.momentum[q] = __shfl_sync(kAll, sum, q + 1);
     if (lane == 0) c.node = acc;
 }
 
