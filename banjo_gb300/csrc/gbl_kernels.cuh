@@ -445,20 +445,24 @@ __device__ __noinline__ void plateBending(const Dev<R> &L, std::uint32_t i, V3<R
                 b12 * (u1[rows[q]] * u2[cols[q]] + u2[rows[q]] * u1[cols[q]]);
 }
 
-template <class R, bool Direct, bool Plate = false>
+template <class R, bool Direct, bool Plate = false, int Ahead = 2>
 __device__ void nodeStrain(const Dev<R> &L, std::uint32_t i, R plate_half_thickness = R(0), R plate_yield = R(0)) {
     const std::size_t N = L.N;
     if (L.dirty[i]) {
         R cov[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         std::uint32_t live = 0;
+        // A slot that is dead, padded or a degenerate rest edge has no weight
+        // and adds zeros, which change nothing: no branch, so the slots' loads
+        // are in flight together.
+#pragma unroll 6
         for (std::uint32_t k = 0; k < L.D; ++k) {
             const Q4<R> q = L.nbr[k * N + i];
             const R w = liveWeight(q.w);
-            if (w <= R(0)) continue; // dead, padded, or a degenerate rest edge
-            const R rr[3] = {q.x, q.y, q.z};
+            const bool counts = !(w <= R(0));
+            const R rr[3] = {counts ? q.x : R(0), counts ? q.y : R(0), counts ? q.z : R(0)};
             for (int r = 0; r < 3; ++r)
                 for (int c = 0; c < 3; ++c) cov[r * 3 + c] += w * rr[r] * rr[c];
-            ++live;
+            live += counts ? 1U : 0U;
         }
         R valid = R(0);
         if (live >= 1U) {
@@ -479,7 +483,7 @@ __device__ void nodeStrain(const Dev<R> &L, std::uint32_t i, R plate_half_thickn
     }
     R acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     const V3<R> xi = Direct ? pos(L, i) : xyz(L.u[i]);
-#pragma unroll 2
+#pragma unroll Ahead
     for (std::uint32_t k = 0; k < L.D; ++k) {
         const std::size_t slot = k * N + i;
         const Q4<R> q = L.nbr[slot];
@@ -534,6 +538,12 @@ __global__ void __launch_bounds__(kThreads) kStrainAll(const Grid<R> launch, int
 // src/fastlattice/ParallelCpuLatticeBackend.cpp:1718-1757 relies on the same fact).
 // It reads the substep's starting positions: before the kick from u, or after
 // it (beside the first contact pass) from u_prev, where the kick copied them.
+// After an upload every node is dirty, and what bounds the kernel is one
+// thread's chain: covariance loads, 12 Jacobi sweeps, moment loads. Six slots'
+// loads in flight and an eigen-solve in registers: 32x8x8 33 -> 27 us,
+// 128x32x32 62 -> 54 us, 128 mixed lattices 89 -> 70 us. (The end sample, which
+// solves no eigensystem for most nodes, is bound by memory: 3, 6 or 9 slots
+// ahead there measured the same as 2.)
 template <class R, bool Many, bool Direct, bool Plate>
 __global__ void __launch_bounds__(kThreads) kRestartStrain(const Grid<R> launch, int after_kick, R plate, R yield) {
     startAfterPrevious();
@@ -544,10 +554,10 @@ __global__ void __launch_bounds__(kThreads) kRestartStrain(const Grid<R> launch,
     // Items cover the node index range; a dirty list is never longer.
     const std::uint32_t t = w.begin + threadIdx.x;
     if (t >= w.end) return;
-    if (L.ctl->full_restart) nodeStrain<R, Direct, Plate>(L, t, plate, yield);
+    if (L.ctl->full_restart) nodeStrain<R, Direct, Plate, 6>(L, t, plate, yield);
     else if (t < L.ctl->dirty_count) {
         const std::uint32_t node = L.dirty_list[t];
-        if (inBounds(node, L.N, kSiteDirty)) nodeStrain<R, Direct, Plate>(L, node, plate, yield);
+        if (inBounds(node, L.N, kSiteDirty)) nodeStrain<R, Direct, Plate, 6>(L, node, plate, yield);
     }
 }
 
@@ -968,6 +978,7 @@ __device__ __forceinline__ void wrenchSpread(const Dev<R> &L, const WrenchDev *w
             largest = largest < fabs(eig[1]) ? fabs(eig[1]) : largest;
             largest = largest < fabs(eig[2]) ? fabs(eig[2]) : largest;
             double un[3] = {moment[0], moment[1], moment[2]};
+#pragma unroll
             for (int axis = 0; axis < 3; ++axis) {
                 if (!(eig[axis] > 1e-10 * largest)) continue;
                 const double dir[3] = {axes[axis], axes[3 + axis], axes[6 + axis]};
