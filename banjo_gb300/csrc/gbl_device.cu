@@ -2444,7 +2444,7 @@ private:
                     g.levels.push_back(over([&](const Res &l, U &b, U &e) {
                         b = d < l.levels.size() ? l.levels[d].begin : 0;
                         e = d < l.levels.size() ? l.levels[d].end : 0;
-                    }, kThreads * kSolvePer));
+                    }, kSolveThreads<R>));
                 g.isolated = over([](const Res &l, U &b, U &e) { b = 0; e = static_cast<U>(l.isolated.size()); },
                                   kThreads);
                 groups_.push_back(std::move(g));
@@ -2465,9 +2465,9 @@ private:
                     const U b = d < l.levels.size() ? l.levels[d].begin : 0;
                     const U e = d < l.levels.size() ? l.levels[d].end : 0;
                     if (lead) { b0 = b; e0 = e; lead = false; }
-                    ranges(k, b, e, kThreads * kSolvePer);
+                    ranges(k, b, e, kThreads);
                 }
-                damp_.push_back(Span{first, static_cast<U>(all.size()) - first, b0, e0, kThreads * kSolvePer});
+                damp_.push_back(Span{first, static_cast<U>(all.size()) - first, b0, e0, kThreads});
             }
         }
         if (all.size() > work_cap_) {
@@ -2805,7 +2805,7 @@ private:
     case K:                                                                                                         \
         launchOverlapped(overlap,                                                                                   \
                          kSolve<R, M, kDirect, ((K) & 8) != 0, ((K) & 4) != 0, ((K) & 2) != 0, ((K) & 1) != 0>,     \
-                         lv.count, kThreads, grid(lv), S_);                                                         \
+                         lv.count, lv.per, grid(lv), S_);                                                           \
         break;
         switch (key) {
             GBL_SOLVE(0) GBL_SOLVE(1) GBL_SOLVE(2) GBL_SOLVE(3) GBL_SOLVE(4) GBL_SOLVE(5) GBL_SOLVE(6) GBL_SOLVE(7)

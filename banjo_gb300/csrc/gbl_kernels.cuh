@@ -1624,31 +1624,32 @@ __device__ __forceinline__ bool supportProject(const Dev<R> &L, const Settings<R
     return projected;
 }
 
-// Bonds per thread of the sweep and the sweep CTAs an SM keeps resident: a
-// thread issues the record loads of all its bonds, then all their gathers,
-// then solves them. A level's bonds share no node, so the order among them is
-// free. Measured on GB300 (impact 256x128x128, sweep ms per substep): one bond
-// per thread with six 256-thread CTAs per SM 2.50; two bonds, four CTAs 2.66;
-// one bond, eight CTAs (spilling at 32 registers) 2.76; two bonds, five CTAs
-// 2.93.
-#ifndef GBL_SOLVE_PER
-#define GBL_SOLVE_PER 1
-#endif
-#ifndef GBL_SOLVE_MIN_BLOCKS
-#define GBL_SOLVE_MIN_BLOCKS 6
-#endif
-constexpr int kSolvePer = GBL_SOLVE_PER;
+// One bond per thread. Float: 256-thread CTAs, six to an SM (sweep of
+// 256x128x128, ms per substep: six 2.47, four or five 2.58, eight, spilling at
+// 32 registers, 3.02; two bonds a thread 2.81. A level too small for all the
+// SMs waits for latency, not for work: 128, 64 and 32 threads measured the same
+// there, and 64 and 32 slower on large levels). Double: an SM has two FP64
+// lanes, so what bounds a level is its busiest SM's bonds, and a level is dealt
+// out in single warps; no spilling at up to 80 registers. Sweep of 48x24x40 in
+// 27 levels of 59 CTAs of 256 threads, us per substep: 1,302 at the 40
+// registers of the float lane's six CTAs, 1,176 without spills, 1,010, 916 and
+// 864 in 128, 64 and 32 threads, 818 with the rest positions and the compliance
+// term fetched ahead (bondAhead). 128x64x64: 3,880 in 256 threads, 3,627 in 32.
+template <class R> constexpr unsigned kSolveThreads = sizeof(R) == 8 ? 32U : static_cast<unsigned>(kThreads);
+template <class R> constexpr unsigned kSolveBlocks = sizeof(R) == 8 ? 24U : 6U;
 
 // A sweep level (programmatic dependent launch, startAfterPrevious) loads what
 // no earlier kernel of the substep writes -- records, geometry, multipliers,
-// plastic extension, the stop flag -- before it waits for the previous grid;
-// at most two levels overlap.
+// plastic extension, the double lane's rest positions, the stop flag -- before
+// it waits for the previous grid; at most two levels overlap.
+
 // The projection of one live bond (LatticePhysics.hpp:1132-1168): its unit
-// direction and the multiplier's change, with the reference's expressions.
-// Returns whether the nodes move (a degenerate bond leaves them).
+// direction and the multiplier's change, with the reference's expressions;
+// alpha is the compliance over dt^2. Returns whether the nodes move (a
+// degenerate bond leaves them).
 template <class R, bool Direct, bool Plastic>
 __device__ __forceinline__ bool bondStep(V3<R> x0a, V3<R> x0b, V3<R> ua, V3<R> ub, V3<R> edge, R rsm, R original,
-                                         R compliance, R wa, R wb, R lambda, R plastic, R dt, V3<R> &dir, R &dl) {
+                                         R alpha, R wa, R wb, R lambda, R plastic, V3<R> &dir, R &dl) {
     const V3<R> delta = Direct ? (x0b + ub) - (x0a + ua) : edge + (ub - ua);
     const R cl = length(delta);
     if (!(cl > R(1.0e-12))) return false;
@@ -1662,7 +1663,6 @@ __device__ __forceinline__ bool bondStep(V3<R> x0a, V3<R> x0b, V3<R> ua, V3<R> u
         constraint = (Plastic ? num - plastic * (rest + original) : num) / (cl + rest);
     }
     dir = delta / cl;
-    const R alpha = compliance / (dt * dt);
     dl = (-constraint - alpha * lambda) / (wa + wb + alpha);
     return true;
 }
@@ -1677,8 +1677,8 @@ __device__ __noinline__ FloatStep floatStepAnywhere(V3<float> ua, V3<float> ub, 
                                                     float original, float compliance, float wa, float wb, float lambda,
                                                     float plastic, float dt) {
     FloatStep s{};
-    s.moves = bondStep<float, false, Plastic>(V3<float>{}, V3<float>{}, ua, ub, edge, rsm, original, compliance, wa, wb,
-                                              lambda, plastic, dt, s.dir, s.dl);
+    s.moves = bondStep<float, false, Plastic>(V3<float>{}, V3<float>{}, ua, ub, edge, rsm, original,
+                                              compliance / (dt * dt), wa, wb, lambda, plastic, s.dir, s.dl);
     return s;
 }
 // The float lane's step. The same values from the branch-free quotients: the
@@ -1713,6 +1713,26 @@ __device__ __forceinline__ FloatStep floatStep(const Settings<float> &S, V3<floa
     return s;
 }
 
+// What the double lane's step needs and no kernel of the sweep writes, for a
+// level to fetch and form before it waits for the level ahead of it: the rest
+// positions and the compliance over dt^2 (the float lane works on differences
+// and divides branch-free, and takes neither).
+template <class R> struct BondAhead {
+    V3<R> x0a, x0b;
+    R alpha;
+};
+template <class R, bool Direct>
+__device__ __forceinline__ BondAhead<R> bondAhead(const Dev<R> &L, const Settings<R> &S, const BondRec<R> &rec,
+                                                  R compliance) {
+    BondAhead<R> h{};
+    if (Direct && !(rec.a & kDeadBit)) {
+        h.x0a = xyz(L.x0[endA(rec)]);
+        h.x0b = xyz(L.x0[endB(rec)]);
+        h.alpha = compliance / (S.dt * S.dt);
+    }
+    return h;
+}
+
 // Where a sweep keeps its nodes' positions: the lattice's array in global
 // memory (through L2, which every SM shares), or a CTA's shared memory
 // (StagedNodes, below).
@@ -1742,7 +1762,7 @@ __device__ __forceinline__ void supportLast(const Dev<R> &L, const Settings<R> &
 template <class R, bool Direct, bool Plastic, bool Support, class Nodes>
 __device__ __forceinline__ void solveBond(const Dev<R> &L, const Settings<R> &S, const Nodes &nodes, R *lambdas,
                                           std::uint32_t d, const BondRec<R> &rec, const Q4<R> &g, R lambda, R plastic,
-                                          bool last) {
+                                          bool last, const BondAhead<R> &ahead) {
     const std::uint32_t a = endA(rec), b = endB(rec);
     const bool live = !(rec.a & kDeadBit);
     bool write_a = false, write_b = false;
@@ -1761,9 +1781,8 @@ __device__ __forceinline__ void solveBond(const Dev<R> &L, const Settings<R> &S,
             dl = s.dl;
             moves = s.moves;
         } else {
-            const V3<R> x0a = Direct ? xyz(L.x0[a]) : V3<R>{}, x0b = Direct ? xyz(L.x0[b]) : V3<R>{};
-            moves = bondStep<R, Direct, Plastic>(x0a, x0b, ua, ub, edge, rec.rsm, rec.rest, g.w, wa, wb, lambda, plastic,
-                                                 S.dt, dir, dl);
+            moves = bondStep<R, Direct, Plastic>(ahead.x0a, ahead.x0b, ua, ub, edge, rec.rsm, rec.rest, ahead.alpha, wa,
+                                                 wb, lambda, plastic, dir, dl);
         }
         if (moves) {
             if (!last) __stcs(lambdas + d, lambda + dl);
@@ -1783,33 +1802,29 @@ __device__ __forceinline__ void solveBond(const Dev<R> &L, const Settings<R> &S,
 }
 
 template <class R, bool Many, bool Direct, bool First, bool Last, bool Plastic, bool Support>
-__global__ void __launch_bounds__(kThreads, GBL_SOLVE_MIN_BLOCKS) kSolve(const Grid<R> launch, Settings<R> S) {
+__global__ void __launch_bounds__(kSolveThreads<R>, kSolveBlocks<R>) kSolve(const Grid<R> launch, Settings<R> S) {
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
-    BondRec<R> rec[kSolvePer];
-    Q4<R> geo[kSolvePer];
-    R lam[kSolvePer], pl[kSolvePer];
-    std::uint32_t at[kSolvePer];
+    const std::uint32_t at = w.begin + threadIdx.x;
+    BondRec<R> rec{};
+    Q4<R> geo{};
+    R lam = R(0), pl = R(0);
     // Everything that no kernel since the last end sample has written.
-#pragma unroll
-    for (int k = 0; k < kSolvePer; ++k) {
-        at[k] = w.begin + threadIdx.x + static_cast<std::uint32_t>(k) * kThreads;
-        if (at[k] < w.end) {
-            rec[k] = ldStream(L.rec + at[k]);
-            geo[k] = ldStream(L.geo + at[k]);
-            lam[k] = First ? R(0) : __ldcs(L.lambda + at[k]);
-            pl[k] = Plastic ? L.plastic[at[k]].x : R(0);
-        }
+    if (at < w.end) {
+        rec = ldStream(L.rec + at);
+        geo = ldStream(L.geo + at);
+        if (!First) lam = __ldcs(L.lambda + at);
+        if (Plastic) pl = L.plastic[at].x;
     }
+    const bool solve = at < w.end && endsInBounds(rec, L.N, kSiteSolve);
+    BondAhead<R> ahead{};
+    if (solve) ahead = bondAhead<R, Direct>(L, S, rec, geo.w);
     const unsigned stop = L.ctl->stop;
     waitPreviousGrid();
     allowNextGrid();
     if (stop) return;
     const GlobalNodes<R> nodes{L.u};
-#pragma unroll
-    for (int k = 0; k < kSolvePer; ++k)
-        if (at[k] < w.end && endsInBounds(rec[k], L.N, kSiteSolve))
-            solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, at[k], rec[k], geo[k], lam[k], pl[k], Last);
+    if (solve) solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, at, rec, geo, lam, pl, Last, ahead);
 }
 
 // The whole sweep of one lattice in one CTA: every iteration, every level in
@@ -1903,7 +1918,7 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 2) kSweepLattice(const Grid
         if (d < end && endsInBounds(now.rec, L.N, kSiteSolve)) {
             if (self_next && cur.it != 0) now.lam = __ldcs(L.lambda + d);
             solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, d, now.rec, now.geo, now.lam, now.pl,
-                                                   cur.it + 1 == I);
+                                                   cur.it + 1 == I, bondAhead<R, Direct>(L, S, now.rec, now.geo.w));
         }
         if (!more) {
             supportIsolatedInCta<R, Support>(L, S);
@@ -2008,7 +2023,8 @@ kSweepStaged(const __grid_constant__ Grid<float> launch, const __grid_constant__
         fetch(next_it, next_lv, next);
         if (now.d != kNoBond && endsInBounds(now.rec, N, kSiteSolve)) {
             if (late_lambda && it != 0) now.lam = __ldcs(lambdas + now.d);
-            solveBond<float, false, Plastic, Support>(L, S, nodes, lambdas, now.d, now.rec, now.geo, now.lam, now.pl, last);
+            solveBond<float, false, Plastic, Support>(L, S, nodes, lambdas, now.d, now.rec, now.geo, now.lam, now.pl, last,
+                                                           BondAhead<float>{});
         }
         if (Support && next_it != it) {
             // Nodes without bonds, each iteration by the same thread; no
