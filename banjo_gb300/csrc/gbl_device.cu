@@ -2792,9 +2792,33 @@ private:
         }
         mark(11);
         if (bonds_.count) {
-            if (plastic_) next(kEndSample<R, M, kDirect, true>, bonds_.count, kThreads, 0, st, grid(bonds_), S_, part);
-            else next(kEndSample<R, M, kDirect, false>, bonds_.count, kThreads, 0, st, grid(bonds_), S_, part);
+            if (part == 2) {
+                // Up to four rounds of CTAs on the chip before one looks at several tiles.
+                const unsigned blocks = std::max((bonds_.count + kLateTiles - 1) / kLateTiles,
+                                                 std::min(bonds_.count, 24U * static_cast<unsigned>(sms_)));
+                if (plastic_)
+                    next(kEndSampleLate<R, M, kDirect, true>, blocks, kThreads, 0, st, grid(bonds_), S_, bonds_.count);
+                else
+                    next(kEndSampleLate<R, M, kDirect, false>, blocks, kThreads, 0, st, grid(bonds_), S_, bonds_.count);
+                return;
+            }
+            const std::uint32_t stripes = M ? 1U : sampleStripes(), tiles = bonds_.count;
+            const std::uint32_t each = tiles / stripes, extra = tiles % stripes;
+            const dim3 blocks = M ? dim3(tiles) : dim3(stripes, each + (extra ? 1U : 0U));
+            if (plastic_)
+                next(kEndSample<R, M, kDirect, true>, blocks, kThreads, 0, st, grid(bonds_), S_, part, each, extra);
+            else
+                next(kEndSample<R, M, kDirect, false>, blocks, kThreads, 0, st, grid(bonds_), S_, part, each, extra);
         }
+    }
+    // The stripes of tiles the end sample goes through side by side: the number
+    // of levels of the widest's size, at most the tiles, and no fewer than keep
+    // a stripe within a grid column.
+    std::uint32_t sampleStripes() const {
+        const Resident<R> &l = *slots_[one_];
+        const std::uint32_t widest = std::max(1U, widestLevel(l)), bonds = static_cast<std::uint32_t>(l.B);
+        const std::uint32_t levels = bonds / widest + (bonds % widest > widest / 2 ? 1U : 0U);
+        return std::max({1U, (bonds_.count + 65533U) / 65534U, std::min(bonds_.count, levels)});
     }
 
     template <bool M> void launchSolve(const Span &lv, bool first, bool last, bool overlap) {

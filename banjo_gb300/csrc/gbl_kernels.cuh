@@ -2148,19 +2148,9 @@ __device__ __forceinline__ double warpSumFixed(double x) {
     return x;
 }
 
-template <class R, bool Many, bool Direct, bool Plastic>
-__global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Settings<R> S, int part) {
-    startAfterPrevious();
-    const Work w = item<Many>(launch);
-    __shared__ SharedDesc<R> desc;
-    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
-    __shared__ double tile_work[kThreads / 32];
-    if (L.ctl->stop) return;
-    // part 0: every tile; 1: the tiles outside the contact halo; 2: inside it.
-    if (part != 0) {
-        const bool late = L.late_tile_stamp[w.begin / kThreads] == substepStamp(L);
-        if (late != (part == 2)) return;
-    }
+// One tile, by the whole CTA.
+template <class R, bool Direct, bool Plastic>
+__device__ __forceinline__ void endSampleTile(const Dev<R> &L, const Settings<R> &S, const Work &w, double *tile_work) {
     const std::uint32_t j = w.begin + threadIdx.x; // storage index; items start on multiples of 256
     double plastic_work = 0.0;
     unsigned peaks[4] = {0, 0, 0, 0};
@@ -2277,6 +2267,74 @@ __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Set
         double wsum = 0.0;
         for (int q = 0; q < kThreads / 32; ++q) wsum += tile_work[q];
         L.tile_plastic[w.begin / kThreads] = wsum;
+    }
+}
+
+// Whether a tile of the bonds touches the contact halo of this substep.
+template <class R> __device__ __forceinline__ bool lateTile(const Dev<R> &L, const Work &w) {
+    return L.late_tile_stamp[w.begin / kThreads] == substepStamp(L);
+}
+
+// Every tile (outside_halo 0), or those outside the contact halo (1). Bonds lie
+// level after level, and every level covers the whole lattice, so tiles in
+// storage order read each node's arrays again once per level, from HBM where
+// the lattice's do not fit in L2 (256x128x128: 134 MB). The CTAs therefore
+// start in stripes of the tiles in turn -- as many as the lattice has levels of
+// the widest's size -- so that those running together sample one region of
+// every level. 256x128x128: 1,107 us in storage order, 896 us in stripes. A batch's lattices, listed one after another, are each small.
+template <class R, bool Many, bool Direct, bool Plastic>
+__global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Settings<R> S, int outside_halo,
+                                                       std::uint32_t each, std::uint32_t extra) {
+    startAfterPrevious();
+    Work w;
+    if (Many) {
+        w = launch.list[blockIdx.x];
+    } else {
+        // Stripe p (a column of the grid) holds `each` tiles, the first `extra`
+        // stripes one more.
+        const std::uint32_t p = blockIdx.x, q = blockIdx.y;
+        if (q == each && p >= extra) return;
+        const std::uint32_t b = launch.base + (p * each + (p < extra ? p : extra) + q) * kThreads;
+        w = Work{0U, b, b + kThreads < launch.end ? b + kThreads : launch.end};
+    }
+    __shared__ SharedDesc<R> desc;
+    const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
+    __shared__ double tile_work[kThreads / 32];
+    if (L.ctl->stop || (outside_halo && lateTile(L, w))) return;
+    endSampleTile<R, Direct, Plastic>(L, S, w, tile_work);
+}
+
+// The tiles inside the contact halo, few among many: a CTA looks at the stamps
+// of up to kLateTiles of them, a lane a tile, and samples those that are. They
+// lie together, so a CTA's are gridDim.x apart. One tile a CTA, 145,860 CTAs of
+// 256x128x128 that mostly return took 153 us, this 28 us.
+constexpr unsigned kLateTiles = 16;
+template <class R, bool Many, bool Direct, bool Plastic>
+__global__ void __launch_bounds__(kThreads) kEndSampleLate(const Grid<R> launch, Settings<R> S, std::uint32_t tiles) {
+    startAfterPrevious();
+    __shared__ SharedDesc<R> desc;
+    __shared__ double tile_work[kThreads / 32];
+    auto tileAt = [&](std::uint32_t k) {
+        if (Many) return launch.list[k];
+        const std::uint32_t b = launch.base + k * kThreads;
+        return Work{0U, b, b + kThreads < launch.end ? b + kThreads : launch.end};
+    };
+    bool late = false;
+    const std::uint32_t mine = blockIdx.x + (threadIdx.x & 31U) * gridDim.x;
+    if ((threadIdx.x & 31U) < kLateTiles && mine < tiles) {
+        const Work w = tileAt(mine);
+        if (Many) {
+            const Dev<R> &L = launch.table[w.lattice];
+            late = !L.ctl->stop && lateTile(L, w);
+        } else {
+            late = !launch.one.ctl->stop && lateTile(launch.one, w);
+        }
+    }
+    // The same in every warp: nothing that runs beside this writes stamps or stops.
+    for (unsigned left = __ballot_sync(0xffffffffU, late); left; left &= left - 1) {
+        const Work w = tileAt(blockIdx.x + static_cast<std::uint32_t>(__ffs(left) - 1) * gridDim.x);
+        if (Many) __syncthreads(); // the descriptor of the tile before is read no more
+        endSampleTile<R, Direct, Plastic>(descriptorIn<R, Many>(launch, w, desc), S, w, tile_work);
     }
 }
 
