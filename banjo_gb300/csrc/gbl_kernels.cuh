@@ -2281,7 +2281,8 @@ template <class R> __device__ __forceinline__ bool lateTile(const Dev<R> &L, con
 // the lattice's do not fit in L2 (256x128x128: 134 MB). The CTAs therefore
 // start in stripes of the tiles in turn -- as many as the lattice has levels of
 // the widest's size -- so that those running together sample one region of
-// every level. 256x128x128: 1,107 us in storage order, 896 us in stripes. A batch's lattices, listed one after another, are each small.
+// every level. 256x128x128: 1,107 us in storage order, 896 us in stripes. A
+// batch's lattices, listed one after another, are each small.
 template <class R, bool Many, bool Direct, bool Plastic>
 __global__ void __launch_bounds__(kThreads) kEndSample(const Grid<R> launch, Settings<R> S, int outside_halo,
                                                        std::uint32_t each, std::uint32_t extra) {
