@@ -390,9 +390,6 @@ void copySegments(const std::vector<Segment> &segments, cudaMemcpyKind kind, Cre
     returnHelpers(T - 1);
     check(static_cast<cudaError_t>(failed.load()), "copy");
 }
-void copyParallel(void *dst, const void *src, std::size_t bytes, cudaMemcpyKind kind) {
-    copySegments({{dst, src, bytes}}, kind);
-}
 
 // Whether the device reads pageable host memory coherently through the host's
 // page tables (as over a Grace CPU's chip-to-chip link).

@@ -3250,7 +3250,7 @@ template <class R> __device__ __forceinline__ V3<R> shfl3(const V3<R> &v, int sr
 // a later pair shares a node, one evaluation; the next 32 pairs' nodes are
 // loaded meanwhile and take the same updates. Reading every pair's nodes again
 // from memory after each response, the window moved up to the next pair, took
-// 305 us where this takes 173 (24x10x18 box, some 500 responses), and the first
+// 305 us where this takes 173 (24x10x18 box), and the first
 // 20 substeps of cracking 53.1 ms against 30.9.
 template <class R, bool Many>
 __global__ void __launch_bounds__(32) kContactNarrow(const Grid<R> launch, Settings<R> S) {

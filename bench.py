@@ -685,7 +685,7 @@ def batched_leg(args, lattice) -> dict:
             "speedup_vs_plain": value / plain, "e2e_speedup_vs_plain": batch_e2e / plain_e2e,
             "roofline": {"bound": "hbm", "achieved": algo / (sweep_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": algo / (sweep_ms * 1e-3) / 1e9 / peak, "peak_kind": peak_kind,
-                         "kernel": "kSweepLattice + kSolve (the batch's projection sweep)",
+                         "kernel": "kSolve (the batch's projection sweep; kSweepLattice where the tuned shape sweeps lattices whole)",
                          "sweep_ms_per_substep": sweep_ms, "algorithmic_bytes_per_substep_sweep": algo},
             "parity": {"ok": all(v["ok"] for v in parity.values()), "members": parity,
                        "substeps": w + k, "largest_member_bonds": counts[largest][1],
