@@ -1068,7 +1068,9 @@ private:
     }
 
     void loop(unsigned index) {
-        std::uint64_t seen = seq_.load(std::memory_order_acquire);
+        // From zero, not from the value as the thread starts: a run too short to
+        // split may have published the stop flag by then.
+        std::uint64_t seen = 0;
         for (;;) {
             std::uint64_t now = seq_.load(std::memory_order_acquire);
             unsigned spins = 0;
