@@ -461,16 +461,24 @@ template <class F> void parallelFor(std::size_t n, F &&f, std::size_t grain = st
     returnHelpers(T - 1);
 }
 
+// Whether an array of T starts on a multiple of its element, which a device
+// access of one needs and a host copy does not.
+template <class T> bool startsOnElement(const T *p) { return reinterpret_cast<std::uintptr_t>(p) % sizeof(T) == 0; }
+
 // Whether a download of `bytes` has the device write the caller's arrays in
 // place (where it reaches pageable memory) rather than through a device buffer,
 // the pinned slices and host threads: the slices' stream, events and threads
 // cost more than a small lattice's bytes (0.1 MB: 27 us in place, 167 through
 // the slices; 11 MB: 138 and 525; 109 MB: 1,130 and 2,119), and from 268 MB on
-// the slices are as fast (3.9 and 4.1 ms).
+// the slices are as fast (3.9 and 4.1 ms). The device stores whole doubles, so
+// an array of them that starts on no multiple of eight bytes is copied to.
 constexpr std::size_t kInPlaceOutMaxBytes = std::size_t(128) << 20;
-bool downloadInPlace(std::size_t bytes) {
+bool downloadInPlace(std::size_t bytes, const gbl_state_view &st) {
     static const bool chosen = std::getenv("GBL_HOST_COPY") != nullptr; // the copies' way is fixed: they are made
-    return !chosen && deviceReadsPageable() && bytes < kInPlaceOutMaxBytes;
+    if (chosen || !deviceReadsPageable() || bytes >= kInPlaceOutMaxBytes) return false;
+    const double *const written[] = {st.u, st.u_prev, st.v, st.damage, st.prev_tensile, st.prev_compressive,
+                                     st.prev_shear, st.plastic_extension, st.plastic_strain};
+    return std::all_of(std::begin(written), std::end(written), startsOnElement<double>);
 }
 
 // Makes the pages of a download's arrays present and writable from the host, a
@@ -1487,7 +1495,7 @@ template <class R> struct Resident {
     void download(gbl_state_view &st, gbl_sphere *sphere, cudaStream_t stream) {
         if (st.node_count != N || st.bond_count != B) invalid("download state does not match the lattice");
         const std::size_t bytes = static_cast<std::size_t>(N) * 72 + static_cast<std::size_t>(B) * 50;
-        if (downloadInPlace(bytes)) {
+        if (downloadInPlace(bytes, st)) {
             writeInPlace(st, stream);
         } else {
             const StateOut out = stateOut(stream);
