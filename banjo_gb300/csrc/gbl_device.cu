@@ -405,6 +405,10 @@ bool deviceReadsPageable() {
     return yes;
 }
 
+// Whether an array of T starts on a multiple of its element, which a device
+// access of one needs and a host copy does not.
+template <class T> bool startsOnElement(const T *p) { return reinterpret_cast<std::uintptr_t>(p) % sizeof(T) == 0; }
+
 // Whether an upload of `bytes` of caller arrays has its conversion kernels
 // read them in place (where the device reads pageable memory) rather than
 // staged: copied in chunks into device buffers (through the pinned slices, or
@@ -416,9 +420,19 @@ bool deviceReadsPageable() {
 // 0.43-1.35 s on first reads and 0.16-1.17 s again (it varies from process to
 // process: the device's translations of the host's pages), staged through the
 // pinned slices 0.21-0.30 s, staged through the driver's copies 1.36-1.45 s.
+// Arrays of which any starts on no multiple of its element are staged.
 constexpr std::size_t kInPlaceMaxBytes = std::size_t(1) << 30;
-bool uploadInPlace(std::size_t bytes) {
+bool uploadInPlace(std::size_t bytes, const gbl_state_view &st) {
     if (!deviceReadsPageable()) return false;
+    const double *const doubles[] = {st.u, st.u_prev, st.v, st.x0, st.mass, st.inv_mass, st.nbr_rest, st.nbr_weight,
+                                     st.rest_length_sq_minus, st.rest_length, st.rest_edge, st.compliance,
+                                     st.prev_tensile, st.prev_compressive, st.prev_shear, st.damage, st.threshold,
+                                     st.plastic_extension, st.plastic_strain};
+    const std::uint32_t *const indices[] = {st.nbr_other, st.nbr_bond, st.bond_a, st.bond_b, st.bond_slot_a,
+                                            st.bond_slot_b};
+    if (!std::all_of(std::begin(doubles), std::end(doubles), startsOnElement<double>) ||
+        !std::all_of(std::begin(indices), std::end(indices), startsOnElement<std::uint32_t>))
+        return false;
     static const int choice = [] {
         const char *env = std::getenv("GBL_UPLOAD");
         if (env && std::strcmp(env, "in_place") == 0) return 1;
@@ -460,10 +474,6 @@ template <class F> void parallelFor(std::size_t n, F &&f, std::size_t grain = st
     for (auto &th : pool) th.join();
     returnHelpers(T - 1);
 }
-
-// Whether an array of T starts on a multiple of its element, which a device
-// access of one needs and a host copy does not.
-template <class T> bool startsOnElement(const T *p) { return reinterpret_cast<std::uintptr_t>(p) % sizeof(T) == 0; }
 
 // Whether a download of `bytes` has the device write the caller's arrays in
 // place (where it reaches pageable memory) rather than through a device buffer,
@@ -1045,7 +1055,7 @@ template <class R> struct Resident {
         if (B) check(cudaMallocAsync(&staged, hi - lo, stream), "device allocation");
         // Host-side copies on other streams need the allocation made; the
         // in-place path keeps all its work on `stream`.
-        in_place_ = !image_ && uploadInPlace(hostBytes());
+        in_place_ = !image_ && uploadInPlace(hostBytes(), view_);
         if (!in_place_) check(cudaStreamSynchronize(stream), "device allocation");
         if (image_) {
             const unsigned char *img = image_.get();

@@ -15,6 +15,10 @@ pytestmark = pytest.mark.gpu
 OUT_DOUBLES = ("u", "u_prev", "v", "damage", "prev_tensile", "prev_compressive", "prev_shear", "plastic_extension",
                "plastic_strain")
 OUT_BYTES = ("alive", "failure_mode")
+IN_DOUBLES = ("x0", "u", "u_prev", "v", "inv_mass", "mass", "nbr_rest", "nbr_weight", "rest_edge", "rest_length",
+              "rest_length_sq_minus", "compliance", "threshold", "damage", "prev_tensile", "prev_compressive",
+              "prev_shear", "plastic_extension", "plastic_strain")
+IN_INDICES = ("nbr_bond", "nbr_other", "bond_slot_a", "bond_slot_b", "bond_a", "bond_b")
 
 
 def _shifted(array, by):
@@ -74,3 +78,26 @@ def test_download_into_unaligned_arrays(device, precision):
         for raw, (k, part) in zip(held, parts.items()):  # and nothing around it
             at = part.ctypes.data - raw.ctypes.data
             assert not raw[:at].any() and not raw[at + part.size:].any(), (k, some)
+
+
+def test_upload_from_unaligned_arrays(device):
+    case, sched, state = _scene(device)
+    settings, sphere = device.step_settings(case["settings"]), device.sphere_state(case["sphere"])
+    backend = device.make_gb300_lattice_backend(sched)
+
+    def result(view):
+        device._call(device.library().gbl_upload, backend._h, C.byref(view), C.byref(settings), C.byref(sphere))
+        backend.run(device.RunControl(max_steps=12))
+        out = device.build_lattice_state(case, sched)
+        backend.download(out)
+        return {k: out.arrays[k].copy() for k in OUT_DOUBLES + OUT_BYTES}
+
+    expected = result(state.view)
+    assert np.any(expected["u"] != 0)
+    shifts = [{name: 4} for name in IN_DOUBLES] + [{name: 2} for name in IN_INDICES]
+    shifts += [{name: by for name in IN_DOUBLES + IN_INDICES + OUT_BYTES + ("nbr_alive",)} for by in (1, 6)]
+    for some in shifts:
+        view, held, _ = _view(device, state, some)
+        got = result(view)
+        for k, want in expected.items():
+            assert np.array_equal(got[k].view(np.uint8), want.view(np.uint8)), (k, some)
