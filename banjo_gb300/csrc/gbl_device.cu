@@ -40,7 +40,9 @@ namespace gbl {
 namespace {
 
 void check(cudaError_t e, const char *what) {
-    if (e != cudaSuccess) runtime(std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    cudaGetLastError(); // reported here: a later launch does not report it again
+    runtime(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 // One allocation per lattice, carved into aligned arrays. The layout is
@@ -1721,23 +1723,26 @@ public:
     }
 
     // The device half of add: a prepared lattice takes the first free slot.
-    std::size_t place(std::unique_ptr<Resident<R>> r, std::uint64_t step_limit = 0) {
+    // Every allocation is made before it does: one that is refused leaves the
+    // engine as it was, and the prepared lattice with the caller.
+    std::size_t place(std::unique_ptr<Resident<R>> &&r, std::uint64_t step_limit = 0) {
         std::lock_guard<std::mutex> lock(place_mutex_);
-        r->commit(stream_);
         std::size_t k = 0;
         while (k < slots_.size() && slots_[k]) ++k;
+        if (ready_) {
+            growControl(k + 1);
+            ensureScratch(*r, S_);
+        }
+        r->commit(stream_);
         if (k == slots_.size()) slots_.emplace_back();
         slots_[k] = std::move(r);
         listActive();
         dirty_ = true;
         if (ready_) {
-            growControl(slots_.size());
             if (slots_[k]->plastic_state && !plastic_) {
                 plastic_ = true;
                 dropGraph();
             }
-            if (S_.nc_mode != 0) slots_[k]->ensureContact();
-            if (S_.sphere_enabled) slots_[k]->ensureSphere();
             initControl(k, step_limit);
             pushDescriptor(k);
             check(cudaStreamSynchronize(stream_), "admit");
@@ -1760,15 +1765,15 @@ public:
     void settle(const gbl_step_settings &set) {
         validate(set);
         if (active_.empty()) invalid("the batch holds no lattice");
+        // The settings are taken once what they need is there: an allocation
+        // that is refused leaves the ones before them in force.
+        const Settings<R> S = convertSettings(set);
+        for (auto k : active_) ensureScratch(*slots_[k], S);
+        growControl(slots_.size());
         dropGraph();
-        S_ = convertSettings(set);
+        S_ = S;
         plastic_ = S_.yield_stretch > R(0);
         for (auto k : active_) plastic_ = plastic_ || slots_[k]->plastic_state;
-        if (S_.nc_mode != 0)
-            for (auto k : active_) slots_[k]->ensureContact();
-        if (S_.sphere_enabled)
-            for (auto k : active_) slots_[k]->ensureSphere();
-        growControl(slots_.size());
         for (auto k : active_) initControl(k, 0);
         for (auto k : active_) pushDescriptor(k);
         check(cudaStreamSynchronize(stream_), "settle");
@@ -1779,16 +1784,14 @@ public:
     // A settle() without lattices: the settings of a server that admits later.
     void configure(const gbl_step_settings &set) {
         validate(set);
+        const Settings<R> S = convertSettings(set);
+        for (auto k : active_) ensureScratch(*slots_[k], S);
         dropGraph();
-        S_ = convertSettings(set);
+        S_ = S;
         plastic_ = S_.yield_stretch > R(0);
         for (auto k : active_) plastic_ = plastic_ || slots_[k]->plastic_state;
         if (S_.nc_mode != 0 || S_.sphere_enabled) {
-            for (auto k : active_) {
-                if (S_.nc_mode != 0) slots_[k]->ensureContact();
-                if (S_.sphere_enabled) slots_[k]->ensureSphere();
-                pushDescriptor(k);
-            }
+            for (auto k : active_) pushDescriptor(k);
             check(cudaStreamSynchronize(stream_), "descriptors");
         }
         ready_ = true;
@@ -2215,6 +2218,12 @@ private:
             }
         }
         return o;
+    }
+
+    // A lattice's contact scratch under these settings.
+    static void ensureScratch(Resident<R> &l, const Settings<R> &S) {
+        if (S.nc_mode != 0) l.ensureContact();
+        if (S.sphere_enabled) l.ensureSphere();
     }
 
     void listActive() {
