@@ -643,12 +643,18 @@ template <class R> struct Resident {
         for (auto b : contactParts(n)) total += b;
         return total;
     }
-    // The sphere contact's candidate records (with a sphere in the settings).
+    // The sphere contact's candidate records (with a sphere in the settings),
+    // stream-ordered from the pool as the arena is: a request that enters or
+    // leaves a server does not wait for the device.
     static std::size_t sphereBytes(std::uint32_t blocks) {
         return static_cast<std::size_t>(blocks) * kCandidatesPerBlock * sizeof(Staged<R>);
     }
-    void ensureSphere() {
-        if (!dev.cand_stage) check(cudaMalloc(&dev.cand_stage, sphereBytes(sched.block_count)), "device allocation");
+    Arena sphere_records;
+    void ensureSphere(cudaStream_t stream) {
+        if (sphere_records.base()) return;
+        if (!sphere_records.bytes())
+            sphere_records.reserve(dev.cand_stage, static_cast<std::size_t>(sched.block_count) * kCandidatesPerBlock);
+        sphere_records.allocate(stream);
     }
     void ensureContact() {
         if (nc_mem) return;
@@ -681,7 +687,6 @@ template <class R> struct Resident {
         }
         if (flowed_dev_) cudaFree(flowed_dev_);
         if (nc_mem) cudaFree(nc_mem);
-        if (dev.cand_stage) cudaFree(dev.cand_stage);
         if (ext_force) cudaFree(ext_force);
         if (ext_req) cudaFree(ext_req);
         if (ext_contrib) cudaFree(ext_contrib);
@@ -2221,9 +2226,9 @@ private:
     }
 
     // A lattice's contact scratch under these settings.
-    static void ensureScratch(Resident<R> &l, const Settings<R> &S) {
+    void ensureScratch(Resident<R> &l, const Settings<R> &S) {
         if (S.nc_mode != 0) l.ensureContact();
-        if (S.sphere_enabled) l.ensureSphere();
+        if (S.sphere_enabled) l.ensureSphere(stream_);
     }
 
     void listActive() {
