@@ -2401,7 +2401,13 @@ private:
         blocks_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.dev.tiles_b / kScanBlock + 1; }, 1);
         each_ = span([](const Res &, U &b, U &e) { b = 0; e = 1; }, 1);
         slabs_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.sched.block_count; }, 1);
-        owners_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.nc_mem ? l.N : 0U; }, kGatherOwners);
+        {
+            std::uint64_t owners = 0;
+            for (auto k : active_) owners += slots_[k]->nc_mem ? slots_[k]->N : 0U;
+            const std::uint64_t once = static_cast<std::uint64_t>(kGatherOwners) * kGatherPerSm * sms_;
+            owners_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.nc_mem ? l.N : 0U; },
+                           kGatherOwners * std::max(1U, static_cast<U>((owners + once - 1) / once)));
+        }
         buckets_ = span([](const Res &l, U &b, U &e) { b = 0; e = l.nc_mem ? l.dev.nc_mask + 1U : 0U; }, kThreads);
         // The lattices swept staged, or whole in one CTA each where the shape
         // says so, largest first; the level launches and the isolated-node

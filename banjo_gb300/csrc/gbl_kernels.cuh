@@ -3001,9 +3001,18 @@ __global__ void __launch_bounds__(kThreads) kContactSort(const Grid<R> launch) {
 // pass: the pairs at the owner's place in the list. One warp per owner, a lane
 // per cell: the 27 cells' chains of loads (bucket, members, cell, position,
 // the owner's bonds) run side by side, and a scan over the lanes puts the
-// pairs in cell order. (One thread walked them all: the broad phase of the
-// 24x10x18 cracking box took 220 us a substep, 40 now.)
-constexpr unsigned kGatherOwners = kThreads / 32; // per CTA
+// pairs in cell order; owners without pairs, most of a lattice whose bonds hold,
+// are passed over by the write pass.
+//
+// Both passes are launched every substep and mostly return at once, so what
+// bounds them then is starting CTAs: at most kGatherPerSm of them an SM, each
+// over a run of owners, whose lists lie together. Broad phase without a rebuild
+// and with one, us: 640,000 nodes 59 and 1,086 (a CTA per 8 owners 211 and
+// 1,190; a thread per owner 57 and 1,313), 163,840 nodes 31 and 255 (64 and
+// 280; 41 and 413), 4,320 nodes 14 and 37 (14 and 37; 39 and 197); at 16, 64 an
+// SM 54 and 1,114, 67 and 1,068 with 640,000.
+constexpr unsigned kGatherOwners = kThreads / 32; // a CTA's at a time
+constexpr unsigned kGatherPerSm = 32;
 constexpr unsigned kGatherSlots = 32;             // an owner's bonds kept in shared memory
 template <class R, bool Many, bool Write>
 __global__ void __launch_bounds__(kThreads) kContactGather(const Grid<R> launch, Settings<R> S) {
@@ -3012,103 +3021,108 @@ __global__ void __launch_bounds__(kThreads) kContactGather(const Grid<R> launch,
     __shared__ SharedDesc<R> desc;
     __shared__ std::uint32_t others[kGatherOwners][kGatherSlots], bonds[kGatherOwners][kGatherSlots];
     __shared__ bool lives[kGatherOwners][kGatherSlots];
+    {
+        const Ctl *ctl = Many ? launch.table[w.lattice].ctl : launch.one.ctl;
+        if (ctl->stop || !ctl->nc_rebuild) return;
+    }
     const Dev<R> &L = descriptorIn<R, Many>(launch, w, desc);
     Ctl &c = *L.ctl;
-    if (c.stop || !c.nc_rebuild) return;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x / 32;
-    const std::uint32_t i = w.begin + warp; // items: up to kGatherOwners nodes of one tile
-    if (i >= w.end) return;
-    const std::uint32_t tile = i / kThreads;
-    if (L.v[i].w <= R(0)) { // not movable: no pairs of its own
-        if (!Write && lane == 0) L.nc_fill[i] = 0U;
-        return;
-    }
     const std::size_t N = L.N;
-    // The owner's bonds, in slot order up to the first padded slot.
-    const std::uint32_t kept = L.D < kGatherSlots ? L.D : kGatherSlots;
-    std::uint32_t bs = kNoBond;
-    if (lane < kept) {
-        const std::size_t slot = lane * N + i;
-        bs = L.nbr_bond[slot];
-        others[warp][lane] = L.nbr_other[slot];
-        bonds[warp][lane] = bs;
-        lives[warp][lane] = !signbit(L.nbr[slot].w);
-    }
-    const unsigned padded = __ballot_sync(0xffffffffU, bs == kNoBond);
-    const std::uint32_t listed = padded ? static_cast<std::uint32_t>(__ffs(padded) - 1) : 32U;
-    __syncwarp();
-    // The owner's bond to j, if it lists one; whether that bond is alive.
-    auto bondTo = [&](std::uint32_t j, std::uint32_t &bond) {
-        for (std::uint32_t s = 0; s < listed; ++s)
-            if (others[warp][s] == j) {
-                bond = bonds[warp][s];
-                return lives[warp][s];
-            }
-        for (std::uint32_t s = kGatherSlots; listed == kGatherSlots && s < L.D; ++s) {
-            const std::size_t slot = s * N + i;
-            const std::uint32_t far = L.nbr_bond[slot];
-            if (far == kNoBond) break;
-            if (L.nbr_other[slot] != j) continue;
-            bond = far;
-            return !signbit(L.nbr[slot].w);
-        }
-        return false;
-    };
     const R cutoff = contactCutoff(S);
     const R cutoff_sq = cutoff * cutoff;
-    const V3<R> p = pos(L, i);
-    const int4 home = L.nc_cell[i];
-    const int gx = home.x + static_cast<int>(lane % 3) - 1, gy = home.y + static_cast<int>(lane / 3 % 3) - 1,
-              gz = home.z + static_cast<int>(lane / 9) - 1;
-    std::uint32_t first = 0, members = 0;
-    if (lane < 27) {
-        const std::uint32_t b = cellBucket(gx, gy, gz, L.nc_mask);
-        first = L.nc_start[b];
-        members = L.nc_count[b];
+    for (std::uint32_t i = w.begin + warp; i < w.end; i += kGatherOwners) {
+        __syncwarp(); // the bonds of the owner before are read no more
+        const std::uint32_t tile = i / kThreads;
+        if (Write) {
+            if (L.nc_fill[i] == 0U) continue;
+        } else if (L.v[i].w <= R(0)) { // not movable: no pairs of its own
+            if (lane == 0) L.nc_fill[i] = 0U;
+            continue;
+        }
+        // The owner's bonds, in slot order up to the first padded slot.
+        const std::uint32_t kept = L.D < kGatherSlots ? L.D : kGatherSlots;
+        std::uint32_t bs = kNoBond;
+        if (lane < kept) {
+            const std::size_t slot = lane * N + i;
+            bs = L.nbr_bond[slot];
+            others[warp][lane] = L.nbr_other[slot];
+            bonds[warp][lane] = bs;
+            lives[warp][lane] = !signbit(L.nbr[slot].w);
+        }
+        const unsigned padded = __ballot_sync(0xffffffffU, bs == kNoBond);
+        const std::uint32_t listed = padded ? static_cast<std::uint32_t>(__ffs(padded) - 1) : 32U;
+        __syncwarp();
+        // The owner's bond to j, if it lists one; whether that bond is alive.
+        auto bondTo = [&](std::uint32_t j, std::uint32_t &bond) {
+            for (std::uint32_t s = 0; s < listed; ++s)
+                if (others[warp][s] == j) {
+                    bond = bonds[warp][s];
+                    return lives[warp][s];
+                }
+            for (std::uint32_t s = kGatherSlots; listed == kGatherSlots && s < L.D; ++s) {
+                const std::size_t slot = s * N + i;
+                const std::uint32_t far = L.nbr_bond[slot];
+                if (far == kNoBond) break;
+                if (L.nbr_other[slot] != j) continue;
+                bond = far;
+                return !signbit(L.nbr[slot].w);
+            }
+            return false;
+        };
+        const V3<R> p = pos(L, i);
+        const int4 home = L.nc_cell[i];
+        const int gx = home.x + static_cast<int>(lane % 3) - 1, gy = home.y + static_cast<int>(lane / 3 % 3) - 1,
+                  gz = home.z + static_cast<int>(lane / 9) - 1;
+        std::uint32_t first = 0, members = 0;
+        if (lane < 27) {
+            const std::uint32_t b = cellBucket(gx, gy, gz, L.nc_mask);
+            first = L.nc_start[b];
+            members = L.nc_count[b];
+        }
+        // The cell's pairs in member order: take(j, bond).
+        auto pairs = [&](auto &&take) {
+            for (std::uint32_t k = 0; k < members; ++k) {
+                const std::uint32_t j = L.nc_members[first + k];
+                if (j <= i) continue;
+                const int4 cj = L.nc_cell[j];
+                if (cj.x != gx || cj.y != gy || cj.z != gz) continue;
+                const V3<R> r = pos(L, j) - p;
+                if (dot(r, r) > cutoff_sq) continue;
+                std::uint32_t bond = kNoBond;
+                if (bondTo(j, bond)) continue; // a live bond holds the pair
+                take(j, bond);
+            }
+        };
+        std::uint32_t mine = 0;
+        pairs([&](std::uint32_t, std::uint32_t) { ++mine; });
+        const std::uint32_t upto = warpInclusive(mine);
+        const std::uint32_t total = __shfl_sync(0xffffffffU, upto, 31);
+        const std::uint32_t fill = total < kPairsPerNode ? total : kPairsPerNode;
+        if (!Write) {
+            if (lane == 0) {
+                L.nc_fill[i] = fill;
+                if (fill) atomicAdd(&L.nc_tile[tile], fill);
+                if (total > fill) atomicAdd(&c.node.pair_overflow, static_cast<unsigned long long>(total - fill));
+            }
+            continue;
+        }
+        // The owner's place: its tile's first pair and the pairs of the tile's
+        // nodes before it.
+        std::uint32_t before = 0;
+        for (std::uint32_t q = tile * kThreads + lane; q < i; q += 32) before += L.nc_fill[q];
+        before = __reduce_add_sync(0xffffffffU, before);
+        std::uint32_t rank = upto - mine;
+        const std::uint32_t at = L.nc_tile[tile] + before;
+        pairs([&](std::uint32_t j, std::uint32_t bond) {
+            if (rank < kPairsPerNode) {
+                L.nc_pa[at + rank] = i;
+                L.nc_pb[at + rank] = j;
+                L.nc_pbond[at + rank] = bond;
+            }
+            ++rank;
+        });
     }
-    // The cell's pairs in member order: take(j, bond).
-    auto pairs = [&](auto &&take) {
-        for (std::uint32_t k = 0; k < members; ++k) {
-            const std::uint32_t j = L.nc_members[first + k];
-            if (j <= i) continue;
-            const int4 cj = L.nc_cell[j];
-            if (cj.x != gx || cj.y != gy || cj.z != gz) continue;
-            const V3<R> r = pos(L, j) - p;
-            if (dot(r, r) > cutoff_sq) continue;
-            std::uint32_t bond = kNoBond;
-            if (bondTo(j, bond)) continue; // a live bond holds the pair
-            take(j, bond);
-        }
-    };
-    std::uint32_t mine = 0;
-    pairs([&](std::uint32_t, std::uint32_t) { ++mine; });
-    const std::uint32_t upto = warpInclusive(mine);
-    const std::uint32_t total = __shfl_sync(0xffffffffU, upto, 31);
-    const std::uint32_t fill = total < kPairsPerNode ? total : kPairsPerNode;
-    if (!Write) {
-        if (lane == 0) {
-            L.nc_fill[i] = fill;
-            if (fill) atomicAdd(&L.nc_tile[tile], fill);
-            if (total > fill) atomicAdd(&c.node.pair_overflow, static_cast<unsigned long long>(total - fill));
-        }
-        return;
-    }
-    if (total == 0) return;
-    // The owner's place: its tile's first pair and the pairs of the tile's
-    // nodes before it.
-    std::uint32_t before = 0;
-    for (std::uint32_t q = tile * kThreads + lane; q < i; q += 32) before += L.nc_fill[q];
-    before = __reduce_add_sync(0xffffffffU, before);
-    std::uint32_t rank = upto - mine;
-    const std::uint32_t at = L.nc_tile[tile] + before;
-    pairs([&](std::uint32_t j, std::uint32_t bond) {
-        if (rank < kPairsPerNode) {
-            L.nc_pa[at + rank] = i;
-            L.nc_pb[at + rank] = j;
-            L.nc_pbond[at + rank] = bond;
-        }
-        ++rank;
-    });
 }
 
 // Rebuild, step 6 (one CTA per lattice): the tiles' first pairs in node order,
