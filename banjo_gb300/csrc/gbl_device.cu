@@ -2126,7 +2126,7 @@ public:
         out.sweep_threads = best.sweep_threads;
         out.whole_max_bonds = best.whole_max_bonds;
         out.group_bytes = best.group_bytes;
-        out.staged_max_nodes = best.staged_max_nodes;
+        out.staged_max_nodes = best.staged_max_nodes ? best.staged_max_nodes : ~0U; // as setShape takes it
         out.sweep_ms = best_ms;
         return out;
     }
@@ -2339,7 +2339,7 @@ private:
     // A lattice of a batch swept by one CTA (kSweepLattice): small enough to
     // keep its nodes in L2 across its levels, with levels that fit the table.
     bool sweptWhole(const Resident<R> &l) const {
-        return l.B > 0 && l.B <= shape_.whole_max_bonds && l.dev.level_count == l.levels.size();
+        return l.B > kNoneWhole && l.B <= shape_.whole_max_bonds && l.dev.level_count == l.levels.size();
     }
 
     // Whether the lattices sweep staged, one CTA each (kSweepStaged): when
@@ -2879,9 +2879,11 @@ private:
     // one-CTA sweep's CTA size, the largest lattice it takes, and the node
     // bytes of a level-launched group. Defaults measured on the trial
     // workload; tune() times candidates on the lattices present.
+    // (A shape's values are none of them the 0 with which setShape keeps one.)
+    static constexpr std::uint32_t kNoneWhole = 1; // a reach of one bond: no lattice is swept by one CTA
     struct Shape {
         unsigned sweep_threads = kSweepThreads;
-        std::uint32_t whole_max_bonds = 0; // none: every shape that used it was slower than level launches
+        std::uint32_t whole_max_bonds = kNoneWhole;
         std::size_t group_bytes = std::size_t(48) << 20;
         std::uint32_t staged_max_nodes = kStagedMaxNodes; // nodes of a lattice swept staged, at most (0: none)
     };

@@ -881,8 +881,9 @@ class Batch:
 
     def set_tuning(self, sweep_threads: int = 0, whole_max_bonds: int = 0, group_bytes: int = 0,
                    staged_max_nodes: int = 0) -> None:
-        """Launch shapes (0 keeps a value; staged_max_nodes 0xFFFFFFFF turns
-        the shared-memory staged sweep off)."""
+        """Launch shapes (0 keeps a value; whole_max_bonds 1 is none,
+        staged_max_nodes 0xFFFFFFFF turns the shared-memory staged sweep off).
+        The fields of the same names in tune()'s result give its shape."""
         t = Tuning(sweep_threads, whole_max_bonds, group_bytes, 0.0, 0.0, 0, staged_max_nodes)
         _call(library().gbl_batch_set_tuning, self._h, C.byref(t))
 

@@ -385,20 +385,20 @@ gbl_result gbl_batch_first_failure_bonds(gbl_batch *batch, uint32_t index, uint3
  * projection sweep of the lattices present under each candidate shape --
  * positions are saved before and restored after, so the lattices' state is
  * unchanged -- and keeps the fastest; gbl_batch_set_tuning applies a known
- * shape without timing (zero fields keep the current value). */
+ * shape without timing (zero fields keep the current value; tune reports none,
+ * so that what it reports is the shape another batch then runs). */
 typedef struct gbl_tuning {
     uint32_t sweep_threads;   /* CTA size of the one-CTA sweep of a small lattice: 256, 512 or 1024 */
     uint32_t whole_max_bonds; /* the largest lattice (bonds) swept by one CTA; larger ones are level-launched
-                                 (0 in tune's output: none, the default) */
+                                 (at most 2^24; 1: none, the default) */
     uint64_t group_bytes;     /* node bytes of a group of level-launched lattices swept together */
     double sweep_ms;          /* the kept shape's sweep, per substep (tune only) */
     double default_ms;        /* the default shape's sweep, per substep (tune only) */
     uint32_t candidates;      /* shapes timed (tune only) */
     uint32_t staged_max_nodes; /* lattices of up to this many nodes may be swept by one CTA each with their positions
-                                  in shared memory (float lane; at most 14,336, the default; done when every lattice
-                                  present is that small with at most 1,024 bonds to a sweep level, and no more of
-                                  them than the device has SMs; 0 off in tune's output; in set_tuning 0 keeps the
-                                  current value and 0xFFFFFFFF turns staging off) */
+                                  in shared memory (float lane; at most 14,336, the default, of which 14,080 fit;
+                                  done when every lattice present is that small with at most 1,024 bonds to a sweep
+                                  level, and no more of them than the device has SMs; 0xFFFFFFFF: off) */
 } gbl_tuning;
 gbl_result gbl_batch_tune(gbl_batch *batch, gbl_tuning *chosen);
 gbl_result gbl_batch_set_tuning(gbl_batch *batch, const gbl_tuning *shape);
