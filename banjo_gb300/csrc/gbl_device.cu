@@ -2032,28 +2032,28 @@ public:
 
     // The batch autotuner: times the projection sweep of the lattices present
     // under candidate launch shapes and keeps the fastest. The sweep writes
-    // positions (saved here and restored after), multipliers (rewritten by
-    // the first iteration of every sweep) and support contact flags (cleared
-    // by every kick), so the lattices' state is unchanged.
+    // positions and multipliers (saved here and restored after) and support
+    // contact flags (cleared by every kick), so the lattices' state is unchanged.
     gbl_tuning tune() {
         requireReady();
         if (active_.empty()) invalid("the batch holds no lattice");
         dropGraph();
         std::size_t total = 0;
-        for (auto k : active_) total += sizeof(Q4<R>) * slots_[k]->N;
+        for (auto k : active_) total += sizeof(Q4<R>) * slots_[k]->N + sizeof(R) * slots_[k]->B;
         void *saved = nullptr;
         check(cudaMallocAsync(&saved, total ? total : 256, stream_), "device allocation");
-        auto positions = [&](bool save) {
-            std::size_t off = 0;
+        auto swept = [&](bool save) {
+            char *keep = static_cast<char *>(saved);
+            auto part = [&](void *p, std::size_t n) {
+                if (n) check(cudaMemcpyAsync(save ? keep : p, save ? p : keep, n, cudaMemcpyDeviceToDevice, stream_), "copy");
+                keep += n;
+            };
             for (auto k : active_) {
-                const std::size_t n = sizeof(Q4<R>) * slots_[k]->N;
-                char *keep = static_cast<char *>(saved) + off;
-                void *u = slots_[k]->dev.u;
-                if (n) check(cudaMemcpyAsync(save ? keep : u, save ? u : keep, n, cudaMemcpyDeviceToDevice, stream_), "copy");
-                off += n;
+                part(slots_[k]->dev.u, sizeof(Q4<R>) * slots_[k]->N);
+                part(slots_[k]->dev.lambda, sizeof(R) * slots_[k]->B);
             }
         };
-        positions(true);
+        swept(true);
         cudaEvent_t t0 = nullptr, t1 = nullptr;
         check(cudaEventCreate(&t0), "event");
         check(cudaEventCreate(&t1), "event");
@@ -2116,7 +2116,7 @@ public:
                 attempt(sh);
             }
         }
-        positions(false);
+        swept(false);
         check(cudaFreeAsync(saved, stream_), "device free");
         check(cudaStreamSynchronize(stream_), "tune");
         cudaEventDestroy(t0);
@@ -2649,8 +2649,7 @@ private:
         const unsigned I = S.iterations;
         for (const Group &g : groups_)
             for (unsigned it = 0; it < I; ++it) {
-                const bool first = it == 0, last = it + 1 == I;
-                for (const Span &lv : g.levels) launchSolve<M>(lv, first, last, g.levels.size() >= 2);
+                for (const Span &lv : g.levels) launchSolve<M>(lv, it == 0, g.levels.size() >= 2);
                 mark(5);
                 if (S.plane_count && g.isolated.count)
                     next(kSupportIsolated<R, M>, g.isolated.count, kThreads, 0, st, grid(g.isolated), S);
@@ -2830,20 +2829,17 @@ private:
         return std::max({1U, (bonds_.count + 65533U) / 65534U, std::min(bonds_.count, levels)});
     }
 
-    template <bool M> void launchSolve(const Span &lv, bool first, bool last, bool overlap) {
+    template <bool M> void launchSolve(const Span &lv, bool first, bool overlap) {
         if (!lv.count) return;
         const bool support = S_.plane_count != 0;
-        const int key = (first ? 8 : 0) | (last ? 4 : 0) | (plastic_ ? 2 : 0) | (support ? 1 : 0);
+        const int key = (first ? 4 : 0) | (plastic_ ? 2 : 0) | (support ? 1 : 0);
 #define GBL_SOLVE(K)                                                                                                \
     case K:                                                                                                         \
-        launchOverlapped(overlap,                                                                                   \
-                         kSolve<R, M, kDirect, ((K) & 8) != 0, ((K) & 4) != 0, ((K) & 2) != 0, ((K) & 1) != 0>,     \
-                         lv.count, lv.per, grid(lv), S_);                                                           \
+        launchOverlapped(overlap, kSolve<R, M, kDirect, ((K) & 4) != 0, ((K) & 2) != 0, ((K) & 1) != 0>, lv.count,  \
+                         lv.per, grid(lv), S_);                                                                     \
         break;
         switch (key) {
             GBL_SOLVE(0) GBL_SOLVE(1) GBL_SOLVE(2) GBL_SOLVE(3) GBL_SOLVE(4) GBL_SOLVE(5) GBL_SOLVE(6) GBL_SOLVE(7)
-            GBL_SOLVE(8) GBL_SOLVE(9) GBL_SOLVE(10) GBL_SOLVE(11) GBL_SOLVE(12) GBL_SOLVE(13) GBL_SOLVE(14)
-            GBL_SOLVE(15)
         }
 #undef GBL_SOLVE
     }

@@ -1756,13 +1756,15 @@ __device__ __forceinline__ void supportLast(const Dev<R> &L, const Settings<R> &
 // A bond from its record, geometry, multiplier and plastic extension: its nodes
 // gathered, the projection, then the support projection of the nodes whose
 // last bond of the sweep it is, then the write-back of what moved. The
-// multiplier is stored unless this is the last iteration. A degenerate bond
-// leaves its nodes; a broken or degenerate last bond still carries their
-// support projection.
+// multiplier is stored in every iteration: a bond that is degenerate in a
+// substep's first one, which would start it from zero, goes on from the
+// substep before (LatticePhysics.hpp:1133-1168). A degenerate bond leaves its
+// nodes; a broken or degenerate last bond still carries their support
+// projection.
 template <class R, bool Direct, bool Plastic, bool Support, class Nodes>
 __device__ __forceinline__ void solveBond(const Dev<R> &L, const Settings<R> &S, const Nodes &nodes, R *lambdas,
                                           std::uint32_t d, const BondRec<R> &rec, const Q4<R> &g, R lambda, R plastic,
-                                          bool last, const BondAhead<R> &ahead) {
+                                          const BondAhead<R> &ahead) {
     const std::uint32_t a = endA(rec), b = endB(rec);
     const bool live = !(rec.a & kDeadBit);
     bool write_a = false, write_b = false;
@@ -1785,7 +1787,7 @@ __device__ __forceinline__ void solveBond(const Dev<R> &L, const Settings<R> &S,
                                                  wb, lambda, plastic, dir, dl);
         }
         if (moves) {
-            if (!last) __stcs(lambdas + d, lambda + dl);
+            __stcs(lambdas + d, lambda + dl);
             const V3<R> na = ua - (wa * dl) * dir;
             const V3<R> nb = ub + (wb * dl) * dir;
             qa = Q4<R>{na.x, na.y, na.z, wa};
@@ -1801,7 +1803,7 @@ __device__ __forceinline__ void solveBond(const Dev<R> &L, const Settings<R> &S,
     if (write_b) nodes.store(b, qb);
 }
 
-template <class R, bool Many, bool Direct, bool First, bool Last, bool Plastic, bool Support>
+template <class R, bool Many, bool Direct, bool First, bool Plastic, bool Support>
 __global__ void __launch_bounds__(kSolveThreads<R>, kSolveBlocks<R>) kSolve(const Grid<R> launch, Settings<R> S) {
     const Work w = item<Many>(launch);
     const Dev<R> L = descriptor<R, Many>(launch, w);
@@ -1824,7 +1826,7 @@ __global__ void __launch_bounds__(kSolveThreads<R>, kSolveBlocks<R>) kSolve(cons
     allowNextGrid();
     if (stop) return;
     const GlobalNodes<R> nodes{L.u};
-    if (solve) solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, at, rec, geo, lam, pl, Last, ahead);
+    if (solve) solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, at, rec, geo, lam, pl, ahead);
 }
 
 // The whole sweep of one lattice in one CTA: every iteration, every level in
@@ -1918,7 +1920,7 @@ __global__ void __launch_bounds__(T, T >= 1024 ? 1 : 2) kSweepLattice(const Grid
         if (d < end && endsInBounds(now.rec, L.N, kSiteSolve)) {
             if (self_next && cur.it != 0) now.lam = __ldcs(L.lambda + d);
             solveBond<R, Direct, Plastic, Support>(L, S, nodes, L.lambda, d, now.rec, now.geo, now.lam, now.pl,
-                                                   cur.it + 1 == I, bondAhead<R, Direct>(L, S, now.rec, now.geo.w));
+                                                   bondAhead<R, Direct>(L, S, now.rec, now.geo.w));
         }
         if (!more) {
             supportIsolatedInCta<R, Support>(L, S);
@@ -2014,7 +2016,6 @@ kSweepStaged(const __grid_constant__ Grid<float> launch, const __grid_constant__
     std::uint32_t it = 0, lv = 0;
     // One level; false after the last one of the sweep.
     auto level = [&](Streamed &now, Streamed &next) {
-        const bool last = it + 1 == I;
         std::uint32_t next_it = it, next_lv = lv + 1;
         if (next_lv == levels) {
             next_lv = 0;
@@ -2023,8 +2024,8 @@ kSweepStaged(const __grid_constant__ Grid<float> launch, const __grid_constant__
         fetch(next_it, next_lv, next);
         if (now.d != kNoBond && endsInBounds(now.rec, N, kSiteSolve)) {
             if (late_lambda && it != 0) now.lam = __ldcs(lambdas + now.d);
-            solveBond<float, false, Plastic, Support>(L, S, nodes, lambdas, now.d, now.rec, now.geo, now.lam, now.pl, last,
-                                                           BondAhead<float>{});
+            solveBond<float, false, Plastic, Support>(L, S, nodes, lambdas, now.d, now.rec, now.geo, now.lam, now.pl,
+                                                      BondAhead<float>{});
         }
         if (Support && next_it != it) {
             // Nodes without bonds, each iteration by the same thread; no
