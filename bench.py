@@ -44,6 +44,10 @@ Legs (each with its own parity, FP64 error and CPU baseline where it applies):
             request run alone.
   cascade   the 128x32x32 notched bar under its ramped end load.
 
+Standard output gets one JSON line, the main line whole and each leg's figures
+(headline); the whole of it, a table per member checked included, goes to
+standard error behind "detail: ".
+
 --impl reference times the reference's CPU lane on the same workload, metric
 and window (the substeps of the same K steps after the same W warm-up steps).
 The reference tree does not travel to the GPU machine, so there it runs as the CPU
@@ -58,6 +62,7 @@ from __future__ import annotations
 import argparse
 import gc
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -399,7 +404,8 @@ def run_gb300(args) -> None:
             else:
                 line[name] = fn(args, lattice)
     if rank == 0:
-        print(json.dumps(line))
+        print("detail: " + json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)))
     if dist is not None:
         dist.destroy_process_group()
 
@@ -1038,6 +1044,34 @@ def sum_over_ranks(x: float, dist, torch) -> float:
     t = torch.tensor([x], dtype=torch.float64, device=_reduce_device(dist))
     dist.all_reduce(t, op=dist.ReduceOp.SUM)
     return float(t.item())
+
+
+# What the printed line keeps of a leg's tables; its own figures it keeps, its
+# prose it does not.
+LEG_TABLES = {"e2e": ("value", "unit", "wall_s"), "plain": ("value", "e2e"), "parity": ("ok",),
+              "cpu_baseline": ("value", "unit", "cores"), "roofline": ("achieved", "unit", "frac"),
+              "fp64_error": ("max_position_error_over_extent", "broken_state_differs"),
+              "stress": ("value", "unit", "requests", "p50_latency_s", "p99_latency_s")}
+LEGS = ("cantilever", "batched", "served", "cascade")
+
+
+def headline(line: dict) -> dict:
+    """The printed line: the headline workload whole, each leg's figures,
+    measured values to seven digits. A few KB, so that whatever keeps the end
+    of the output keeps all of it; the whole line goes to stderr."""
+    def short(v):
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items()}
+        return float(f"{v:.7g}") if isinstance(v, float) and math.isfinite(v) else v
+
+    def leg(figures):
+        out = {k: v for k, v in figures.items() if isinstance(v, (bool, int, float)) or k == "unit"}
+        for table, keys in LEG_TABLES.items():
+            if table in figures:
+                out[table] = {k: figures[table][k] for k in keys if k in figures[table]}
+        return out
+
+    return {k: v if not isinstance(v, dict) else short(leg(v) if k in LEGS else v) for k, v in line.items()}
 
 
 def run_reference(args) -> None:
