@@ -1459,8 +1459,6 @@ template <class R> struct Resident {
         return out;
     }
 
-    // The device arrays a download needs, raw, into `raw` (its buffers reused
-    // when large enough).
     // The state's layout of this lattice's arrays, written by the device into
     // a new buffer on `stream` (the caller synchronises and frees it).
     StateOut stateOut(cudaStream_t stream) const {
@@ -2336,8 +2334,9 @@ private:
     // A launch's items: [first, first + count) of the work array; for a
     // single lattice, the same items as (base, end, per).
     struct Span { std::uint32_t first, count, base, end, per; };
-    // A lattice of a batch swept by one CTA (kSweepLattice): small enough to
-    // keep its nodes in L2 across its levels, with levels that fit the table.
+
+    // A lattice of a batch swept by one CTA (kSweepLattice): within the shape's
+    // reach, with levels that fit the table.
     bool sweptWhole(const Resident<R> &l) const {
         return l.B > kNoneWhole && l.B <= shape_.whole_max_bonds && l.dev.level_count == l.levels.size();
     }
@@ -2869,14 +2868,14 @@ private:
     };
     std::vector<Group> groups_;
     std::vector<Span> damp_; // the damping sweep's levels, every lattice
-    // Node bytes a group may hold: its node arrays stay in the 129 MB L2
-    // beside the streamed bond records of a level.
     // Launch shapes of a batch's sweep (results do not depend on them): the
-    // one-CTA sweep's CTA size, the largest lattice it takes, and the node
-    // bytes of a level-launched group. Defaults measured on the trial
-    // workload; tune() times candidates on the lattices present.
-    // (A shape's values are none of them the 0 with which setShape keeps one.)
-    static constexpr std::uint32_t kNoneWhole = 1; // a reach of one bond: no lattice is swept by one CTA
+    // one-CTA sweep's CTA size and the largest lattice it takes, the node
+    // bytes of a level-launched group (whose node arrays stay in the 129 MB L2
+    // beside the streamed bond records of a level), and the largest lattice
+    // swept staged. The default sweeps none whole in one CTA: that gains 3 to
+    // 5 % in large batches and loses as much as 2.7x in small ones
+    // (kSweepLattice); tune() times candidates on the lattices present.
+    static constexpr std::uint32_t kNoneWhole = 1; // a reach of one bond, which is never swept whole
     struct Shape {
         unsigned sweep_threads = kSweepThreads;
         std::uint32_t whole_max_bonds = kNoneWhole;

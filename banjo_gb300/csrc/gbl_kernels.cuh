@@ -1830,13 +1830,18 @@ __global__ void __launch_bounds__(kSolveThreads<R>, kSolveBlocks<R>) kSolve(cons
 }
 
 // The whole sweep of one lattice in one CTA: every iteration, every level in
-// order with a barrier between levels, then the isolated nodes' support. A
-// lattice of a batch small enough for one CTA runs here, so its nodes stay in
-// L2 (and the SM's L1) across all its levels instead of being streamed from
-// HBM again at every level launch; the arithmetic and the per-node order are
-// those of the level launches.
-// The CTA size (256, 512 or 1024 threads) is a launch shape the batch's
-// autotuner picks; two CTAs per SM below 1024 threads.
+// order with a barrier between levels, then the isolated nodes' support. Its
+// nodes stay in L2 (and the SM's L1) across all its levels instead of being
+// streamed from HBM again at every level launch; the arithmetic and the
+// per-node order are those of the level launches.
+//
+// What bounds it is one CTA's chain of L2 round trips, so it is for batches
+// whose lattices outnumber the SMs several times, and only the autotuner
+// chooses it (CTA size and reach). Sweep per substep, level launches and this
+// (ms): 600 lattices of 8 to 48 a side 6.62 and 6.32, 2,000 22.6 and 21.9,
+// 4,096 47.5 and 46.0 (1,024 threads, up to 2^18 bonds); 1,000 of 16 to 24 a
+// side 4.24 and 4.02; of 8 to 12 a side, 300 0.24 and 0.26, 4,000 2.26 and 2.32
+// (512 threads); 128 of 8 to 48 1.46 and 4.01.
 constexpr unsigned kSweepThreads = 512; // the default shape
 constexpr std::uint32_t kMaxFusedLevels = 1024;
 
@@ -2467,7 +2472,8 @@ __global__ void __launch_bounds__(kThreads) kTileCounts(const Grid<R> launch) {
 
 // One CTA per scan block, a thread per tile: the tiles' exclusive offsets
 // inside the block, and the block's totals with its plastic work. A lattice
-// of one block (up to 262,143 bonds) is done; kTopScan follows for the others.
+// of one block (up to 1,023 tiles, 261,888 bonds) is done; kTopScan follows for
+// the others.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kScanBlock) kEventScan(const Grid<R> launch, int plastic) {
     startAfterPrevious();
