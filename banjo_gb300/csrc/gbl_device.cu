@@ -2672,7 +2672,12 @@ private:
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = st == side_ ? 0 : 1; // the second stream's wait for the whole of what it forks from
+        // The other streams' kernels wait for the whole of what they fork from:
+        // the second stream's would fill every SM before the contact chain had
+        // one, and the load ledger's CTAs, placed between those of a kernel that
+        // still runs, would share SMs and their two FP64 lanes (54,720 nodes
+        // loaded by forces of any sign: 2.5 ms a substep, 1.95 so).
+        cfg.numAttrs = st == side_ || st == loads_ ? 0 : 1;
         check(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...), "kernel launch");
     }
 

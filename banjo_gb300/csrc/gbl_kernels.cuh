@@ -775,25 +775,38 @@ __global__ void __launch_bounds__(kThreads) kKick(const Grid<R> launch, Settings
 // or takes the sum to the end of its binade (a sum that rounds to a binade's
 // own bound may have rounded in the one below); that term is added by the
 // hardware, and the next run starts from there. Sums of one sign cross few
-// binades. One that keeps crossing goes on term by term, longer each time.
+// binades. One that keeps crossing goes on term by term, longer each time
+// (FoldPace): then it is the chain, by one lane. Cantilevers loaded by forces of
+// any sign, ms a substep, this and a chain alone: 48x12x12 0.27 and 0.27,
+// 64x16x16 0.60 and 0.60, 96x24x24 1.96 and 1.97; under their weight, which goes
+// by runs, 0.22-0.26 and 0.32, 0.38-0.44 and 0.66, 0.91-0.99 and 2.05.
 //
-// All of it is integer arithmetic on the terms' bits (this GPU has two FP64
+// All of a run is integer arithmetic on the terms' bits (this GPU has two FP64
 // lanes an SM: the same run with FP64 scaling, rint and conversions was slower
 // than the chain). `x` is in shared memory; every lane calls with the same
 // arguments and gets the sum.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double foldSerial(double s, const double *x, unsigned n) {
+// How a sum goes on, kept from chunk to chunk: the terms still to be added one
+// by one, and how many that are after the next run that comes to little (a run
+// costs about as much as 30 adds, whatever it comes to). At most 1,024: at 256,
+// 512 and 2,048 the 64x16x16 cantilever takes 0.63, 0.61 and 0.59 ms a substep
+// with forces of any sign, 0.37, 0.37 and 0.42 under its weight.
+constexpr unsigned kFoldWorth = 32, kFoldMost = 1024;
+struct FoldPace {
+    unsigned owed = kFoldWorth, patience = kFoldWorth;
+};
+__device__ __forceinline__ double foldSerial(double s, const double *x, unsigned n, FoldPace &pace) {
     using u64 = unsigned long long;
     constexpr unsigned kPer = 8; // consecutive terms per lane in a run
     constexpr u64 kOne = 1ULL << 52;
     const unsigned lane = threadIdx.x & 31;
     const u64 *bits = reinterpret_cast<const u64 *>(x);
-    unsigned patience = 16; // terms taken one by one after a run that came to little
     for (unsigned at = 0; at < n;) {
         const u64 sb = static_cast<u64>(__double_as_longlong(s));
         const int exponent = static_cast<int>((sb >> 52) & 0x7ff);
-        unsigned serial = 0;
-        if (exponent == 0 || exponent == 0x7ff) { // zero, subnormal or not finite
+        if (pace.owed) {
+            // Terms one by one, below.
+        } else if (exponent == 0 || exponent == 0x7ff) { // zero, subnormal or not finite
             if ((sb << 1) == 0) {
                 // Zero terms leave a zero sum as it is (it is never -0 here: it
                 // started as +0 or is a cancellation).
@@ -805,7 +818,7 @@ __device__ __forceinline__ double foldSerial(double s, const double *x, unsigned
                 }
                 at += static_cast<unsigned>(__ffs(mask) - 1);
             }
-            serial = 1;
+            pace.owed = 1;
         } else {
             const bool negative = (sb >> 63) != 0;
             const unsigned first = at + lane * kPer;
@@ -847,12 +860,30 @@ __device__ __forceinline__ double foldSerial(double s, const double *x, unsigned
                 s = __longlong_as_double(static_cast<long long>((sb & (0xfffULL << 52)) | (total & (kOne - 1))));
             }
             at += stop;
-            if (stop < 32 * kPer) {
-                serial = stop < 16 ? patience : 1;
-                patience = stop < 16 ? 2 * patience : stop >= 64 ? 16 : patience;
+            if (at < n && stop < 32 * kPer) { // the term it ended at is added by the hardware
+                pace.owed = stop >= kFoldWorth ? 1 : pace.patience;
+                if (stop < kFoldWorth) pace.patience = pace.patience < kFoldMost ? 2 * pace.patience : kFoldMost;
+                else if (stop >= 2 * kFoldWorth) pace.patience = kFoldWorth;
             }
         }
-        for (; serial && at < n; --serial, ++at) s += x[at];
+        if (pace.owed && at < n) {
+            const unsigned upto = n - at < pace.owed ? n : at + pace.owed;
+            pace.owed -= upto - at;
+            if (lane == 0) {
+                // Two terms a load: a load between dependent adds costs them 8 cycles of 72.
+                unsigned k = at;
+                if (__cvta_generic_to_shared(x + k) & 8U) s += x[k++];
+#pragma unroll 8
+                for (; k + 2 <= upto; k += 2) {
+                    const double2 t = *reinterpret_cast<const double2 *>(x + k);
+                    s += t.x;
+                    s += t.y;
+                }
+                if (k < upto) s += x[k];
+            }
+            s = __shfl_sync(0xffffffffU, s, 0);
+            at = upto;
+        }
     }
     return s;
 }
@@ -896,10 +927,12 @@ __device__ __forceinline__ void wrenchSpread(const Dev<R> &L, const WrenchDev *w
     // the first `count` sums; warp q folds sum q, left in sums[q].
     auto pass = [&](unsigned count, auto &&form) {
         double acc = 0.0;
+        FoldPace pace;
         for (std::uint32_t base = 0; base < n; base += kWrenchThreads) {
             if (base + t < n) form(base + t, t);
             __syncthreads();
-            if (warp < count) acc = foldSerial(acc, terms[warp], n - base < kWrenchThreads ? n - base : kWrenchThreads);
+            if (warp < count)
+                acc = foldSerial(acc, terms[warp], n - base < kWrenchThreads ? n - base : kWrenchThreads, pace);
             __syncthreads();
         }
         if (warp < count && t % 32 == 0) sums[warp] = acc;
@@ -2656,6 +2689,7 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
     __shared__ double terms[2][kFoldThreads];
     double total = 0.0;
     unsigned buf = 0;
+    FoldPace pace;
     // Warp 0 reaches the barrier of chunk k+1 only after folding chunk k,
     // so chunk k+2 never overwrites a buffer still being read.
     for (std::uint32_t base = 0; base < L.N; base += kFoldThreads, buf ^= 1U) {
@@ -2666,7 +2700,8 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
             terms[buf][threadIdx.x] = static_cast<double>(R(0.5) * q.w * dot(v, v));
         }
         __syncthreads();
-        if (threadIdx.x < 32) total = foldSerial(total, terms[buf], L.N - base < kFoldThreads ? L.N - base : kFoldThreads);
+        if (threadIdx.x < 32)
+            total = foldSerial(total, terms[buf], L.N - base < kFoldThreads ? L.N - base : kFoldThreads, pace);
     }
     if (threadIdx.x != 0) return;
     if (mode == kAuditMark) c.ke_mark = total;
@@ -2687,8 +2722,8 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
 // reads, beside the contact passes, the sweep and the end sample.
 // ---------------------------------------------------------------------------
 constexpr int kLedgerFolds = 13;
-constexpr unsigned kLedgerThreads = 128;                   // one folding warp, three staging ones
-constexpr unsigned kLedgerStagers = kLedgerThreads - 32;
+constexpr unsigned kLedgerThreads = 160;                   // a warp for the total, one for the sources, three staging ones
+constexpr unsigned kLedgerStagers = kLedgerThreads - 64;
 constexpr unsigned kLedgerChunk = 768;                      // entries staged per round
 
 // Adds a source's folded change (component q) to its ledger.
@@ -2701,9 +2736,8 @@ __device__ __forceinline__ void addLoadComponent(LoadLedger &g, int q, double x)
 }
 
 // One CTA per (lattice, component): blockIdx.y is the component q. Warp 0
-// folds it (foldSerial; the chain of 1,984 dependent FP64 adds it stands for
-// took 75 us); the other warps stage the next chunk of its node
-// contributions.
+// folds its total and warp 1 its sources' runs, beside one another (foldSerial);
+// the other warps stage the next chunk of its node contributions.
 template <class R, bool Many>
 __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> launch, Settings<R> S) {
     startAfterPrevious();
@@ -2716,13 +2750,14 @@ __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> laun
     if (!(c.ext_count && c.loads_remaining > 0)) return;
     __shared__ double stage[2][kLedgerChunk];
     const int q = static_cast<int>(blockIdx.y);
-    const bool stager = threadIdx.x >= 32;
+    const unsigned warp = threadIdx.x / 32;
+    const bool stager = warp >= 2;
     const std::uint32_t n = c.ext_count;
     const unsigned sources = c.wrench_count;
     const auto fill = [&](std::uint32_t base, unsigned buf) {
         const std::uint32_t cnt = n - base < kLedgerChunk ? n - base : kLedgerChunk;
 #pragma unroll 4
-        for (unsigned e = threadIdx.x - 32; e < cnt; e += kLedgerStagers) {
+        for (unsigned e = threadIdx.x - 64; e < cnt; e += kLedgerStagers) {
             const std::uint32_t node = L.ext_nodes[base + e];
             stage[buf][e] = inBounds(node, L.N, kSiteLoad)
                 ? L.ext_contrib[kLedgerFolds * static_cast<std::size_t>(node) + q] : 0.0;
@@ -2735,7 +2770,7 @@ __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> laun
     double run = 0.0;
     const auto flush = [&](std::uint32_t at) {
         while (k < sources && L.wrench[k].end == at) {
-            if (threadIdx.x == 0) {
+            if (threadIdx.x == 32) {
                 SourceSlot &slot = L.sources[L.wrench[k].slot];
                 addLoadComponent(slot.load, q, run);
                 if (q == 0) {
@@ -2749,21 +2784,22 @@ __global__ void __launch_bounds__(kLedgerThreads) kLoadLedger(const Grid<R> laun
         }
     };
     if (stager) fill(0, 0);
-    else flush(0);
+    else if (warp == 1) flush(0);
     __syncthreads();
     double total = 0.0;
     unsigned buf = 0;
+    FoldPace pace;
     for (std::uint32_t base = 0; base < n; base += kLedgerChunk, buf ^= 1U) {
         if (stager) {
             if (base + kLedgerChunk < n) fill(base + kLedgerChunk, buf ^ 1U);
         } else {
             const std::uint32_t cnt = n - base < kLedgerChunk ? n - base : kLedgerChunk;
             const double *col = stage[buf];
-            total = foldSerial(total, col, cnt);
-            for (std::uint32_t e = 0; k < sources && e < cnt;) {
+            if (warp == 0) total = foldSerial(total, col, cnt, pace);
+            for (std::uint32_t e = 0; warp == 1 && k < sources && e < cnt;) {
                 const std::uint32_t end = L.wrench[k].end - base;
                 const std::uint32_t upto = end < cnt ? end : cnt;
-                run = foldSerial(run, col + e, upto - e);
+                run = foldSerial(run, col + e, upto - e, pace);
                 e = upto;
                 flush(base + e);
             }
