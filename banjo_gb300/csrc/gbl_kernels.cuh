@@ -795,81 +795,100 @@ constexpr unsigned kFoldWorth = 32, kFoldMost = 1024;
 struct FoldPace {
     unsigned owed = kFoldWorth, patience = kFoldWorth;
 };
-__device__ __forceinline__ double foldSerial(double s, const double *x, unsigned n, FoldPace &pace) {
+
+// Whether a sum goes by runs from here: not when it is zero, subnormal or not
+// finite. Zero terms leave a zero sum as it is (it is never -0 here: it started
+// as +0 or is a cancellation) and are passed over, `at` moved up.
+__device__ __forceinline__ bool foldRuns(double s, const double *x, unsigned &at, unsigned n) {
     using u64 = unsigned long long;
-    constexpr unsigned kPer = 8; // consecutive terms per lane in a run
+    const u64 sb = static_cast<u64>(__double_as_longlong(s));
+    const int exponent = static_cast<int>((sb >> 52) & 0x7ff);
+    if (exponent != 0 && exponent != 0x7ff) return true;
+    if ((sb << 1) != 0) return false;
+    const u64 *bits = reinterpret_cast<const u64 *>(x);
+    const unsigned lane = threadIdx.x & 31;
+    for (; at < n; at += 32) {
+        const bool some = at + lane < n && (bits[at + lane] << 1) != 0;
+        const unsigned mask = __ballot_sync(0xffffffffU, some);
+        if (mask == 0) continue;
+        at += static_cast<unsigned>(__ffs(mask) - 1);
+        break;
+    }
+    return false;
+}
+
+// One run from term `at`: the terms it took, at most kFoldRun, `s` with them.
+constexpr unsigned kFoldPer = 8; // consecutive terms per lane
+constexpr unsigned kFoldRun = 32 * kFoldPer;
+__device__ __forceinline__ unsigned foldRun(double &s, const double *x, unsigned at, unsigned n) {
+    using u64 = unsigned long long;
+    constexpr unsigned kPer = kFoldPer;
     constexpr u64 kOne = 1ULL << 52;
     const unsigned lane = threadIdx.x & 31;
     const u64 *bits = reinterpret_cast<const u64 *>(x);
+    const u64 sb = static_cast<u64>(__double_as_longlong(s));
+    const int exponent = static_cast<int>((sb >> 52) & 0x7ff);
+    const bool negative = (sb >> 63) != 0;
+    const unsigned first = at + lane * kPer;
+    // The running sums in ulps, signed as the sum is: M positive.
+    long long upto[kPer], sum = 0;
+    unsigned bad = kPer; // the first of the lane's terms that ends a run by itself
+#pragma unroll
+    for (unsigned k = 0; k < kPer; ++k) {
+        const u64 b = first + k < n ? bits[first + k] : 0ULL;
+        const int e = static_cast<int>((b >> 52) & 0x7ff);
+        const u64 mantissa = (b & (kOne - 1)) | (e ? kOne : 0ULL);
+        const int shift = exponent - (e ? e : 1); // x = mantissa / 2^shift ulps
+        const int by = shift < 0 ? 0 : shift > 55 ? 55 : shift;
+        const u64 low = mantissa & ((1ULL << by) - 1), half = (1ULL << by) >> 1;
+        const long long r = static_cast<long long>((mantissa >> by) + (low > half ? 1 : 0));
+        if (bad == kPer && (shift < 0 || (low == half && half != 0) || first + k >= n)) bad = k;
+        sum += ((b >> 63) != 0) != negative ? -r : r;
+        upto[k] = sum;
+    }
+    long long before = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffU, before, o);
+        if (lane >= static_cast<unsigned>(o)) before += y;
+    }
+    before += static_cast<long long>((sb & (kOne - 1)) | kOne) - sum;
+#pragma unroll
+    for (unsigned k = 0; k < kPer; ++k) {
+        const long long total = before + upto[k];
+        if (bad > k && !(total > static_cast<long long>(kOne) && total < static_cast<long long>(2 * kOne))) bad = k;
+    }
+    const unsigned stop = __reduce_min_sync(0xffffffffU, bad < kPer ? lane * kPer + bad : 32 * kPer);
+    if (stop) {
+        const unsigned pick = (stop - 1) % kPer;
+        long long mine = upto[0];
+#pragma unroll
+        for (unsigned k = 1; k < kPer; ++k)
+            if (pick == k) mine = upto[k];
+        const u64 total = static_cast<u64>(__shfl_sync(0xffffffffU, before + mine, static_cast<int>((stop - 1) / kPer)));
+        s = __longlong_as_double(static_cast<long long>((sb & (0xfffULL << 52)) | (total & (kOne - 1))));
+    }
+    return stop;
+}
+
+__device__ __forceinline__ double foldSerial(double s, const double *x, unsigned n, FoldPace &pace) {
     for (unsigned at = 0; at < n;) {
-        const u64 sb = static_cast<u64>(__double_as_longlong(s));
-        const int exponent = static_cast<int>((sb >> 52) & 0x7ff);
-        if (pace.owed) {
-            // Terms one by one, below.
-        } else if (exponent == 0 || exponent == 0x7ff) { // zero, subnormal or not finite
-            if ((sb << 1) == 0) {
-                // Zero terms leave a zero sum as it is (it is never -0 here: it
-                // started as +0 or is a cancellation).
-                const bool some = at + lane < n && (bits[at + lane] << 1) != 0;
-                const unsigned mask = __ballot_sync(0xffffffffU, some);
-                if (mask == 0) {
-                    at += 32;
-                    continue;
+        if (pace.owed == 0) {
+            if (foldRuns(s, x, at, n)) {
+                const unsigned stop = foldRun(s, x, at, n);
+                at += stop;
+                if (at < n && stop < kFoldRun) { // the term it ended at is added by the hardware
+                    pace.owed = stop >= kFoldWorth ? 1 : pace.patience;
+                    if (stop < kFoldWorth) pace.patience = pace.patience < kFoldMost ? 2 * pace.patience : kFoldMost;
+                    else if (stop >= 2 * kFoldWorth) pace.patience = kFoldWorth;
                 }
-                at += static_cast<unsigned>(__ffs(mask) - 1);
-            }
-            pace.owed = 1;
-        } else {
-            const bool negative = (sb >> 63) != 0;
-            const unsigned first = at + lane * kPer;
-            // The running sums in ulps, signed as the sum is: M positive.
-            long long upto[kPer], sum = 0;
-            unsigned bad = kPer; // the first of the lane's terms that ends a run by itself
-#pragma unroll
-            for (unsigned k = 0; k < kPer; ++k) {
-                const u64 b = first + k < n ? bits[first + k] : 0ULL;
-                const int e = static_cast<int>((b >> 52) & 0x7ff);
-                const u64 mantissa = (b & (kOne - 1)) | (e ? kOne : 0ULL);
-                const int shift = exponent - (e ? e : 1); // x = mantissa / 2^shift ulps
-                const int by = shift < 0 ? 0 : shift > 55 ? 55 : shift;
-                const u64 low = mantissa & ((1ULL << by) - 1), half = (1ULL << by) >> 1;
-                const long long r = static_cast<long long>((mantissa >> by) + (low > half ? 1 : 0));
-                if (bad == kPer && (shift < 0 || (low == half && half != 0) || first + k >= n)) bad = k;
-                sum += ((b >> 63) != 0) != negative ? -r : r;
-                upto[k] = sum;
-            }
-            long long before = sum;
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long y = __shfl_up_sync(0xffffffffU, before, o);
-                if (lane >= static_cast<unsigned>(o)) before += y;
-            }
-            before += static_cast<long long>((sb & (kOne - 1)) | kOne) - sum;
-#pragma unroll
-            for (unsigned k = 0; k < kPer; ++k) {
-                const long long total = before + upto[k];
-                if (bad > k && !(total > static_cast<long long>(kOne) && total < static_cast<long long>(2 * kOne))) bad = k;
-            }
-            const unsigned stop = __reduce_min_sync(0xffffffffU, bad < kPer ? lane * kPer + bad : 32 * kPer);
-            if (stop) {
-                const unsigned pick = (stop - 1) % kPer;
-                long long mine = upto[0];
-#pragma unroll
-                for (unsigned k = 1; k < kPer; ++k)
-                    if (pick == k) mine = upto[k];
-                const u64 total = static_cast<u64>(__shfl_sync(0xffffffffU, before + mine, static_cast<int>((stop - 1) / kPer)));
-                s = __longlong_as_double(static_cast<long long>((sb & (0xfffULL << 52)) | (total & (kOne - 1))));
-            }
-            at += stop;
-            if (at < n && stop < 32 * kPer) { // the term it ended at is added by the hardware
-                pace.owed = stop >= kFoldWorth ? 1 : pace.patience;
-                if (stop < kFoldWorth) pace.patience = pace.patience < kFoldMost ? 2 * pace.patience : kFoldMost;
-                else if (stop >= 2 * kFoldWorth) pace.patience = kFoldWorth;
+            } else {
+                pace.owed = 1;
             }
         }
         if (pace.owed && at < n) {
             const unsigned upto = n - at < pace.owed ? n : at + pace.owed;
             pace.owed -= upto - at;
-            if (lane == 0) {
+            if ((threadIdx.x & 31) == 0) {
                 // Two terms a load: a load between dependent adds costs them 8 cycles of 72.
                 unsigned k = at;
                 if (__cvta_generic_to_shared(x + k) & 8U) s += x[k++];
@@ -884,6 +903,23 @@ __device__ __forceinline__ double foldSerial(double s, const double *x, unsigned
             s = __shfl_sync(0xffffffffU, s, 0);
             at = upto;
         }
+    }
+    return s;
+}
+
+// The same for terms of one sign: their sum crosses a binade once, so the next
+// run soon pays.
+__device__ __forceinline__ double foldOneSign(double s, const double *x, unsigned n) {
+    unsigned patience = 16;
+    for (unsigned at = 0; at < n;) {
+        unsigned owed = 1;
+        if (foldRuns(s, x, at, n)) {
+            const unsigned stop = foldRun(s, x, at, n);
+            at += stop;
+            owed = stop == kFoldRun ? 0 : stop < 16 ? patience : 1;
+            patience = stop < 16 ? 2 * patience : stop >= 64 ? 16 : patience;
+        }
+        for (; owed && at < n; --owed, ++at) s += x[at];
     }
     return s;
 }
@@ -2689,7 +2725,6 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
     __shared__ double terms[2][kFoldThreads];
     double total = 0.0;
     unsigned buf = 0;
-    FoldPace pace;
     // Warp 0 reaches the barrier of chunk k+1 only after folding chunk k,
     // so chunk k+2 never overwrites a buffer still being read.
     for (std::uint32_t base = 0; base < L.N; base += kFoldThreads, buf ^= 1U) {
@@ -2701,7 +2736,7 @@ __global__ void __launch_bounds__(kFoldThreads) kKineticFold(const Grid<R> launc
         }
         __syncthreads();
         if (threadIdx.x < 32)
-            total = foldSerial(total, terms[buf], L.N - base < kFoldThreads ? L.N - base : kFoldThreads, pace);
+            total = foldOneSign(total, terms[buf], L.N - base < kFoldThreads ? L.N - base : kFoldThreads);
     }
     if (threadIdx.x != 0) return;
     if (mode == kAuditMark) c.ke_mark = total;
