@@ -1122,7 +1122,7 @@ def main() -> None:
     p.add_argument("--impl", default="gb300", choices=["gb300", "reference"])
     p.add_argument("--workload", default="impact", choices=["impact", "impact_mid", "cantilever"])
     p.add_argument("--profile-substeps", type=int, default=3)
-    p.add_argument("--sweep-traffic-per-bond", type=float, default=759.26e6 / 4616704.0,
+    p.add_argument("--sweep-traffic-per-bond", type=float, default=806.03e6 / 4616704.0,
                    help="ncu DRAM bytes of one substep's sweep per bond (impact 128x64x64)")
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--parity-steps", type=int, default=5, help="impact: steps of the parity prefix (0: skip)")
