@@ -932,7 +932,7 @@ __device__ __forceinline__ double foldOneSign(double s, const double *x, unsigne
 // serial folds in node order: the CTA forms a chunk's terms, a node per thread,
 // and a warp folds each sum (foldSerial). (Formed by the folding thread, a
 // node's divisions and norms cost it a microsecond each: 410 us a kick with 81
-// and 18 nodes, 173 now, most of it the eigen-solve.) The eigen-solve of the tensor is the
+// and 18 nodes, 160 now, most of it the eigen-solve.) The eigen-solve of the tensor is the
 // reference's cyclic Jacobi in double. apply 1 writes the kick's forces (when
 // loads remain); a wrench the current geometry cannot carry then stops the
 // lattice before the kick changes anything, with kErrWrench set (the reference
